@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <numeric>
+#include <type_traits>
 
 namespace wrapd {
 
@@ -136,9 +137,9 @@ __device__ __forceinline__ void cp_async16(double* s, const double* g, int src_b
     const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(s));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(g), "r"(src_bytes));
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // Element (i, t), i < rows, t < K, of a source with (TMAJOR) i contiguous:
 // base[i + t * ld], or t contiguous: base[i * ld + t]; zeros up to K4.
@@ -611,405 +612,478 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_wgemm(const double* __restrict
 }
 
 // ---- solve -----------------------------------------------------------------------
-// Per level, one launch per direction.  Forward: a CTA owns a band of 64 rows of
-// the front's M = [Y; W] ((k + r) x k, leading dimension ldy) and a chunk of its
-// columns (Y rows only up to the diagonal): rows < k give z_s = Y t_s, rows >= k
-// give u_s = v_s - W t_s.  Backward: a CTA owns a band of 64 columns and a chunk
-// of the rows below the diagonal and of the W rows: y_s = Y^T z_s - W^T y_rows.  The right-hand side is
-// read from B (a copy of the input), z from Zb, and y written to x, so no CTA
-// reads what another CTA of the same launch writes.
-
-// t_s(i) for i < k, or v_s(i) for i >= k: own b entry plus the children's update
-// entries landing on front row i, in child order (inv: offsets in U, or -1).
-__device__ __forceinline__ void front_rhs(const double* __restrict__ B, const double* __restrict__ U,
-                                          const int64_t* __restrict__ inv, const FrontDesc& d, int i,
-                                          double& v0, double& v1, double& v2) {
-    if (i < d.k) {
-        const double* b = B + 3 * ((int64_t)d.first + i);
-        v0 = b[0]; v1 = b[1]; v2 = b[2];
-    } else {
-        v0 = v1 = v2 = 0.0;
-    }
-    const int64_t* iv = inv + d.inv_off + 2 * (int64_t)i;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int64_t o = iv[q];
-        if (o >= 0) { v0 += __ldcg(U + o); v1 += __ldcg(U + o + 1); v2 += __ldcg(U + o + 2); }
-    }
-}
-
-// Each CTA takes one item: a 64-wide band (rows forward, columns backward) times
-// a chunk of the other dimension (at most SCH).  The CTAs of one band write
-// partial sums; the last one to arrive adds them in chunk order (deterministic)
-// and writes the band's result, then resets the band counter.
-constexpr int SCH = 256;
-constexpr int FWD_WARPS = 4;          // warps of a forward solve CTA (eight CTAs per SM)
+// One launch per direction walks every level of the tree.  The work of a
+// direction is one list of items, forward leaves first and backward root first.
+// Forward: an item is a band of 64 rows of a front's M = [Y; W] ((k + r) x k,
+// leading dimension ldy) times a chunk of its columns (Y rows only up to the
+// diagonal): rows < k give z_s = Y t_s, rows >= k give u_s = v_s - W t_s.
+// Backward: a band of 64 columns times a chunk of the rows below the diagonal
+// and of the W rows: y_s = Y^T z_s - W^T y_rows.
+//
+// Persistent CTAs take items in list order through an atomic head.  What an
+// item reads of other fronts -- forward the children's update entries U,
+// backward the ancestors' solution -- it waits for entry by entry: those
+// buffers hold the pattern kUnset in every entry not yet written, and a reader
+// polls the entry itself until it holds a value.  A value thus crosses from
+// its writer to its reader in one store and one load, with no fence, counter
+// or flag between them, which is what bounds a system of this kind: a tree
+// of ten levels is a chain of ten such hand-overs, each way.  The partial sums
+// of a band's chunks are handed to the band's last item the same way and added
+// in chunk order, so results do not depend on which CTA takes which item.
+// kUnset is a signalling NaN, which no arithmetic operation returns, and every
+// value stored in these buffers is the result of one.
+//
+// Everything waited for comes from items earlier in the list, which were taken
+// by running CTAs, so the earliest unfinished item never waits and the list
+// always drains.  Every wait is bounded (kWaitNs, kWaitPolls): one that gives
+// up sets *status to WRAPD_E_TIMEOUT and its item is skipped, and waits that
+// find *status set return at once.
+//
+// The buffers are unset again on the way: the forward pass unsets the solution
+// buffer, the backward pass U, and a band's last item the partial sums it has
+// read; after a failed launch the host refills them (CholGPU::reset_solve).
+//
+// Measured, us per solve, forward + backward (before: register-staged loads,
+// per-front counters raised behind a fence and read by one thread, an arrival
+// counter per band, a copy of the right-hand side and a memset per solve):
+//   bar          levels  [Y; W]    before          now
+//   8x8x32            6    2 MB   25.5 +   21.6   13.8 +   12.0
+//   13x11x37          8    7 MB   39.0 +   36.2   23.6 +   22.0
+//   16x16x64          9   30 MB   57.4 +   59.2   35.9 +   36.0
+//   24x24x48         10   66 MB   92.9 +   84.9   46.8 +   69.4
+//   32x32x128        12  490 MB  199.9 +  195.9    133 +    164
+//   64x64x160        14  4.5 GB    958 +   1436    957 +   1070   (4.7, 4.2 TB/s)
+// The order of every sum is the earlier kernels', so the results are the same
+// bit for bit: in mixed precision the rounding of the local step turns a last
+// bit here into 1e-8 of the positions within twenty iterations.
+constexpr int SCH = 256;              // longest chunk of the streamed dimension
 constexpr int SCH_MIN = 64;
-constexpr int kSolveCtas = 2 * 148;   // two 256-thread CTAs per SM of a B200
+constexpr int kSolveItems = 2 * 148;   // items wanted per level (see build and build_queues)
+constexpr int kBwdSub = 4;            // narrow backward bands per 64 columns
+constexpr size_t kBwdDeepBytes = (size_t)3 << 29;     // largest [Y; W] of the deep backward ring (see k_bwd_queue)
+constexpr size_t kGateBytes = (size_t)256 << 20;      // largest [Y; W] whose items poll their inputs directly (see k_fwd_queue)
+constexpr unsigned long long kUnset = 0x7ff45a5a5a5a5a5aull;
 
-__device__ __forceinline__ bool band_arrive(unsigned* counter, int nchunk) {
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned old = atomicAdd(counter, 1u);
-        last = old == (unsigned)nchunk - 1;
-        if (last) *counter = 0u;
-    }
-    __syncthreads();
-    if (last) __threadfence();
-    return last;
+__device__ __forceinline__ bool unset(double v) {
+    return static_cast<unsigned long long>(__double_as_longlong(v)) == kUnset;
+}
+__device__ __forceinline__ double ld_relaxed(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed(double* p, double v) {
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_unset3(double* p) {
+    const double u = __longlong_as_double(static_cast<long long>(kUnset));
+    st_relaxed(p, u);
+    st_relaxed(p + 1, u);
+    st_relaxed(p + 2, u);
 }
 
-// Forward: lane l of warp w holds rows b0 + 2l and b0 + 2l + 1 of the band (one
-// 16-byte load per column: the block's leading dimension and the band start are
-// even) and takes columns lo + w, lo + w + FWD_WARPS, ...; the warps' sums
-// are added in warp order.  Four-warp CTAs, eight per SM: more items in
-// flight for the latency-bound lower levels (eight-warp CTAs, four per SM,
-// measured 2 % slower per solve; two-warp CTAs 13 % slower).
-// One forward item (q: its index in the item list, which places its partial
-// sums in P).  Returns true, in every thread, in the CTA that wrote the band's
-// result, after all its writes are visible device-wide.
-// The first eight columns of each warp of a forward item (warp w takes columns
-// w, w + FWD_WARPS, ...): [Y; W] does not change during a solve, so they are
-// loaded before the item's dependency wait and its right-hand-side gather.
-constexpr int FWD_PRE = 8;
-__device__ __forceinline__ void fwd_pre(const double* __restrict__ YW, const FrontDesc& d, const SolveItem& it,
-                                        double2 (&pre)[FWD_PRE]) {
-    const int R = d.k + d.r;
-    const int nc = it.hi - it.lo;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = it.b0 + 2 * lane;
-    const double* M = YW + d.y_off + i0 + (int64_t)it.lo * d.ldy;
-#pragma unroll
-    for (int u = 0; u < FWD_PRE; ++u) {
-        const int j = warp + FWD_WARPS * u;
-        pre[u] = (i0 < R && j < nc) ? __ldg(reinterpret_cast<const double2*>(M + (int64_t)j * d.ldy))
-                                    : make_double2(0.0, 0.0);
-    }
+__global__ void k_unset(double* __restrict__ p, int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = __longlong_as_double(static_cast<long long>(kUnset));
 }
 
-__device__ __forceinline__ bool fwd_item(const double* __restrict__ B, double* __restrict__ Zb,
-                                         double* __restrict__ U, const int64_t* __restrict__ inv,
-                                         const double* __restrict__ YW, const FrontDesc& d, const SolveItem& it, int q,
-                                         double* __restrict__ P, unsigned* __restrict__ counters,
-                                         const double2 (&pre)[FWD_PRE]) {
-    __shared__ double tv[SCH * 3];
-    __shared__ double part[FWD_WARPS][TL][3];
-    const int R = d.k + d.r;
-    const int nc = it.hi - it.lo;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = it.b0 + 2 * lane;
-    const double* M = YW + d.y_off + i0 + (int64_t)it.lo * d.ldy;
-    constexpr int PRE = FWD_PRE;
-    for (int j = threadIdx.x; j < nc; j += blockDim.x) {
-        double v0, v1, v2;
-        front_rhs(B, U, inv, d, it.lo + j, v0, v1, v2);
-        tv[3 * j] = v0; tv[3 * j + 1] = v1; tv[3 * j + 2] = v2;
+// After the i-th look at entries that were not all set (i from 0): whether to
+// look again.
+__device__ __forceinline__ bool look_again(int i, unsigned long long& t0, int* status) {
+    if (*reinterpret_cast<volatile int*>(status) != 0) return false;
+    const unsigned long long now = global_ns();
+    if (i == 0) t0 = now;
+    if (now - t0 > kWaitNs || i >= kWaitPolls) {
+        atomicCAS(status, 0, WRAPD_E_TIMEOUT);
+        return false;
     }
-    __syncthreads();
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, b0 = 0.0, b1 = 0.0, b2 = 0.0;
-#pragma unroll
-    for (int u = 0; u < PRE; ++u) {
-        const int j = warp + FWD_WARPS * u;
-        if (j < nc) {
-            const double t0 = tv[3 * j], t1 = tv[3 * j + 1], t2 = tv[3 * j + 2];
-            a0 = fma(pre[u].x, t0, a0); a1 = fma(pre[u].x, t1, a1); a2 = fma(pre[u].x, t2, a2);
-            b0 = fma(pre[u].y, t0, b0); b1 = fma(pre[u].y, t1, b1); b2 = fma(pre[u].y, t2, b2);
-        }
-    }
-    if (i0 < R) {
-#pragma unroll 8
-        for (int j = warp + FWD_WARPS * PRE; j < nc; j += FWD_WARPS) {
-            const double2 m = __ldg(reinterpret_cast<const double2*>(M + (int64_t)j * d.ldy));
-            const double t0 = tv[3 * j], t1 = tv[3 * j + 1], t2 = tv[3 * j + 2];
-            a0 = fma(m.x, t0, a0); a1 = fma(m.x, t1, a1); a2 = fma(m.x, t2, a2);
-            b0 = fma(m.y, t0, b0); b1 = fma(m.y, t1, b1); b2 = fma(m.y, t2, b2);
-        }
-    }
-    part[warp][2 * lane][0] = a0; part[warp][2 * lane][1] = a1; part[warp][2 * lane][2] = a2;
-    part[warp][2 * lane + 1][0] = b0; part[warp][2 * lane + 1][1] = b1; part[warp][2 * lane + 1][2] = b2;
-    __syncthreads();
-    const int row = threadIdx.x;
-    const int i = it.b0 + row;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    if (row < TL) {
-#pragma unroll
-        for (int w = 0; w < FWD_WARPS; ++w) { s0 += part[w][row][0]; s1 += part[w][row][1]; s2 += part[w][row][2]; }
-    }
-    if (it.nchunk > 1) {
-        if (row < TL) {
-            double* p = P + 3 * ((int64_t)q * TL + row);
-            p[0] = s0; p[1] = s1; p[2] = s2;
-        }
-        if (!band_arrive(counters + it.band, it.nchunk)) return false;
-        if (row < TL) {
-            s0 = s1 = s2 = 0.0;
-            for (int c = 0; c < it.nchunk; ++c) {
-                const double* p = P + 3 * ((int64_t)(it.first + c) * TL + row);
-                s0 += __ldcg(p); s1 += __ldcg(p + 1); s2 += __ldcg(p + 2);
-            }
-        }
-    }
-    if (row < TL && i < R) {
-        if (i < d.k) {
-            double* o = Zb + 3 * ((int64_t)d.first + i);
-            o[0] = s0; o[1] = s1; o[2] = s2;
-        } else {
-            double v0, v1, v2;
-            front_rhs(B, U, inv, d, i, v0, v1, v2);
-            double* u = U + d.u_off + 3 * (int64_t)(i - d.k);
-            u[0] = v0 - s0; u[1] = v1 - s1; u[2] = v2 - s2;
-        }
-    }
-    __threadfence();
-    __syncthreads();
+    __nanosleep(32);
     return true;
 }
 
-__global__ void __launch_bounds__(32 * FWD_WARPS) k_fwd_level(const double* __restrict__ B, double* __restrict__ Zb,
-                                                   double* __restrict__ U, const int64_t* __restrict__ inv,
-                                                   const double* __restrict__ YW, const FrontDesc* __restrict__ desc,
-                                                   const SolveItem* __restrict__ items, double* __restrict__ P,
-                                                   unsigned* __restrict__ counters, const int* __restrict__ mesh_on) {
-    const SolveItem it = items[blockIdx.x];
-    const FrontDesc d = desc[it.front];
-    if (mesh_on && !mesh_on[d.mesh]) return;   // the whole band's CTAs: its counter stays 0
-    double2 pre[FWD_PRE];
-    fwd_pre(YW, d, it, pre);
-    fwd_item(B, Zb, U, inv, YW, d, it, blockIdx.x, P, counters, pre);
+// The rows of three values at p[0 .. N-1] (null: zeros), looked at until all
+// of them are set.  False when the wait gave up or the launch had already failed.
+template <int N>
+__device__ __forceinline__ bool await3(const double* const (&p)[N], double (&v)[N][3], int* status) {
+    unsigned long long t0 = 0;
+    for (int i = 0;; ++i) {
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[n][c] = p[n] ? ld_relaxed(p[n] + c) : 0.0;
+        bool all = true;
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) all = all && !unset(v[n][c]);
+        if (all) return true;
+        if (!look_again(i, t0, status)) return false;
+    }
 }
 
-// Backward: a CTA owns a band of 64 columns and a chunk [lo, hi) of the rows
-// (lo even; a chunk may cross row k): the input of row i is z_i for i < k and
-// minus the solution at the front's row i - k for i >= k.  Warp w takes the
-// eight columns b0 + w + 8m; lane l loads rows lo + 2l + 64t and the next one
-// of each as one 16-byte load.  The 8 x 3 lane sums are then added across the
-// warp by a butterfly that halves the values each lane keeps (12, 6, 3) before
-// two plain exchange steps, so the eight columns share 27 shuffles.
-// The first row pair of each of the warp's eight columns of a backward item,
-// loaded before the item's dependency wait and its input gather.
-__device__ __forceinline__ void bwd_pre(const double* __restrict__ YW, const FrontDesc& d, const SolveItem& it,
-                                        double2 (&pre)[8]) {
-    const int nr = it.hi - it.lo;
-    const int nc = min(TL, d.k - it.b0);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const double* M0 = YW + d.y_off + it.lo + (int64_t)(it.b0 + warp) * d.ldy;
+// s <- the sum of row `row`'s partial sums of a band's chunks, in chunk order,
+// the last of which is s itself (the caller's); the slots read are unset.
+__device__ __forceinline__ bool add_chunks(double* P, int first, int nchunk, int row, double (&s)[3], int* status) {
+    constexpr int NB = 6;   // rows looked at together
+    double t[3] = {0.0, 0.0, 0.0};
+    for (int c = 0; c < nchunk - 1; c += NB) {
+        const double* p[NB];
+        double v[NB][3];
 #pragma unroll
-    for (int m = 0; m < 8; ++m)
-        pre[m] = (2 * lane < nr && warp + 8 * m < nc)
-                     ? __ldg(reinterpret_cast<const double2*>(M0 + (int64_t)(8 * m) * d.ldy + 2 * lane))
-                     : make_double2(0.0, 0.0);
-}
-
-__device__ __forceinline__ bool bwd_item(double* __restrict__ x, const double* __restrict__ Zb,
-                                         const double* __restrict__ YW, const int* __restrict__ rows,
-                                         const FrontDesc& d, const SolveItem& it, int q, double* __restrict__ P,
-                                         unsigned* __restrict__ counters, const double2 (&pre)[8]) {
-    __shared__ double in[(SCH + 1) * 3];
-    __shared__ double res[TL][3];
-    const int nr = it.hi - it.lo;
-    const int nc = min(TL, d.k - it.b0);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const double* M0 = YW + d.y_off + it.lo + (int64_t)(it.b0 + warp) * d.ldy;
-    for (int t = threadIdx.x; t < nr + 1; t += blockDim.x) {
-        const int i = it.lo + t;
-        double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-        if (t < nr) {
-            if (i < d.k) {
-                const double* z = Zb + 3 * ((int64_t)d.first + i);
-                v0 = z[0]; v1 = z[1]; v2 = z[2];
-            } else {
-                const double* y = x + 3 * (int64_t)rows[d.rows_off + i - d.k];
-                v0 = -__ldcg(y); v1 = -__ldcg(y + 1); v2 = -__ldcg(y + 2);
+        for (int e = 0; e < NB; ++e) p[e] = c + e < nchunk - 1 ? P + 3 * ((int64_t)(first + c + e) * TL + row) : nullptr;
+        if (!await3(p, v, status)) return false;
+#pragma unroll
+        for (int e = 0; e < NB; ++e)
+            if (p[e]) {
+                t[0] += v[e][0]; t[1] += v[e][1]; t[2] += v[e][2];
+                st_unset3(const_cast<double*>(p[e]));
             }
-        }
-        in[3 * t] = v0; in[3 * t + 1] = v1; in[3 * t + 2] = v2;
     }
-    __syncthreads();
-    double v[24];
-#pragma unroll
-    for (int q = 0; q < 24; ++q) v[q] = 0.0;
-    if (2 * lane < nr) {
-        const int t = 2 * lane;
-        const double x0 = in[3 * t], x1 = in[3 * t + 1], x2 = in[3 * t + 2];
-        const double y0 = in[3 * t + 3], y1 = in[3 * t + 4], y2 = in[3 * t + 5];
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            v[3 * m] = fma(pre[m].y, y0, fma(pre[m].x, x0, v[3 * m]));
-            v[3 * m + 1] = fma(pre[m].y, y1, fma(pre[m].x, x1, v[3 * m + 1]));
-            v[3 * m + 2] = fma(pre[m].y, y2, fma(pre[m].x, x2, v[3 * m + 2]));
-        }
-    }
-    for (int t = 2 * lane + 64; t < nr; t += 64) {
-        const double x0 = in[3 * t], x1 = in[3 * t + 1], x2 = in[3 * t + 2];
-        const double y0 = in[3 * t + 3], y1 = in[3 * t + 4], y2 = in[3 * t + 5];
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            if (warp + 8 * m < nc) {
-                const double2 a = __ldg(reinterpret_cast<const double2*>(M0 + (int64_t)(8 * m) * d.ldy + t));
-                v[3 * m] = fma(a.y, y0, fma(a.x, x0, v[3 * m]));
-                v[3 * m + 1] = fma(a.y, y1, fma(a.x, x1, v[3 * m + 1]));
-                v[3 * m + 2] = fma(a.y, y2, fma(a.x, x2, v[3 * m + 2]));
-            }
-        }
-    }
-    // reduce-scatter: after the offsets 16, 8, 4 lane l keeps the 3 sums of
-    // column slot m = 4 (l>>4 & 1) + 2 (l>>3 & 1) + (l>>2 & 1) over 8 lanes
-#pragma unroll
-    for (int q = 0; q < 12; ++q) {
-        const bool hi = lane & 16;
-        const double send = hi ? v[q] : v[q + 12];
-        const double keep = hi ? v[q + 12] : v[q];
-        v[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const bool hi = lane & 8;
-        const double send = hi ? v[q] : v[q + 6];
-        const double keep = hi ? v[q + 6] : v[q];
-        v[q] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        const bool hi = lane & 4;
-        const double send = hi ? v[q] : v[q + 3];
-        const double keep = hi ? v[q + 3] : v[q];
-        v[q] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-    }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        v[q] += __shfl_xor_sync(0xffffffffu, v[q], 2);
-        v[q] += __shfl_xor_sync(0xffffffffu, v[q], 1);
-    }
-    if ((lane & 3) == 0) {
-        const int m = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-        const int jj = warp + 8 * m;
-        res[jj][0] = v[0]; res[jj][1] = v[1]; res[jj][2] = v[2];
-    }
-    __syncthreads();
-    const int j = threadIdx.x;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    if (j < TL) { s0 = res[j][0]; s1 = res[j][1]; s2 = res[j][2]; }
-    if (it.nchunk > 1) {
-        if (j < TL) {
-            double* p = P + 3 * ((int64_t)q * TL + j);
-            p[0] = s0; p[1] = s1; p[2] = s2;
-        }
-        if (!band_arrive(counters + it.band, it.nchunk)) return false;
-        if (j < TL) {
-            s0 = s1 = s2 = 0.0;
-            for (int c = 0; c < it.nchunk; ++c) {
-                const double* p = P + 3 * ((int64_t)(it.first + c) * TL + j);
-                s0 += __ldcg(p); s1 += __ldcg(p + 1); s2 += __ldcg(p + 2);
-            }
-        }
-    }
-    if (j < nc) {
-        double* o = x + 3 * ((int64_t)d.first + it.b0 + j);
-        o[0] = s0; o[1] = s1; o[2] = s2;
-    }
-    __threadfence();
-    __syncthreads();
+    s[0] = t[0] + s[0]; s[1] = t[1] + s[1]; s[2] = t[2] + s[2];
     return true;
 }
 
-__global__ void __launch_bounds__(256) k_bwd_level(double* __restrict__ x, const double* __restrict__ Zb,
-                                                   const double* __restrict__ YW, const int* __restrict__ rows,
-                                                   const FrontDesc* __restrict__ desc,
-                                                   const SolveItem* __restrict__ items, double* __restrict__ P,
-                                                   unsigned* __restrict__ counters, const int* __restrict__ mesh_on) {
-    const SolveItem it = items[blockIdx.x];
-    const FrontDesc d = desc[it.front];
-    if (mesh_on && !mesh_on[d.mesh]) return;
-    double2 pre[8];
-    bwd_pre(YW, d, it, pre);
-    bwd_item(x, Zb, YW, rows, d, it, blockIdx.x, P, counters, pre);
+// The CTA's item list position: thread 0 of warp `W` holds the ticket of the
+// next item (fetched once the current item's waits are over, so that a CTA
+// that waits does not sit on work another could take) and its warp copies that
+// item's record to shared memory while the others finish the current one.
+struct ItemSlot {
+    SolveWork it;
+    int q;
+};
+__device__ __forceinline__ void fetch_item(const SolveQueue& Q, int ticket, ItemSlot* slot) {
+    const int lane = threadIdx.x & 31;
+    const int q = __shfl_sync(0xffffffffu, ticket, 0);
+    if (lane == 0) slot->q = q;
+    if (q < Q.n && lane < (int)(sizeof(SolveWork) / 16))
+        reinterpret_cast<int4*>(&slot->it)[lane] = __ldg(reinterpret_cast<const int4*>(Q.items + q) + lane);
 }
 
-// ---- whole-direction solve over a work queue -------------------------------------
-// One launch per direction walks every level: the items of all levels in one
-// list (forward: leaves first; backward: root first), taken in list order by
-// persistent CTAs through an atomic head (each CTA takes its next item while
-// it works on the current one).  An item waits, in thread 0, until the fronts
-// it reads are complete -- forward: both children (their update vectors);
-// backward: the parent (and through it every ancestor, which own the front's
-// rows) -- counted by per-front band counters that each band's writer bumps
-// after its writes are visible.  Every item an item waits on comes earlier in
-// the list and was taken by a running CTA, so the earliest unfinished item
-// never waits and the queue always drains.  A wait (wait_count_geq) is bounded
-// by one second of the global timer and a poll count; one that gives up sets
-// *status to WRAPD_E_TIMEOUT and skips its item, and every later wait returns at
-// once, so the launch ends with the error for the host to read.  The results
-// are those of the per-level launches bit for bit: the same items, chunks and
-// chunk order per band.
-__device__ __forceinline__ bool wait_bands(const unsigned* done, unsigned target, int* status) {
-    return wait_count_geq(done, target, status);
-}
+// Both directions stream an item's block of [Y; W] through shared memory in
+// stages of 16 columns x 64 rows (8 KB) by cp.async, a ring of stages in flight
+// per CTA and the first ringful issued before the item's waits ([Y; W] does not
+// change during a solve).  Every warp copies exactly the values it will use
+// itself, so the stages need no CTA barrier.  Five CTAs of four warps per SM with
+// rings of four keep 160 KB in flight per SM, against 128 KB of register loads
+// before.  The backward pass has long chunks to stream at every level (a
+// front's r rows; forward a chunk is at most the front's k columns), so where a
+// level has few items its time is ringfuls: rings of eight with three CTAs per
+// SM run it in 19, 64, 168 us on the 8x8x32, 24x24x48, 32x32x128 bars against 30,
+// 100, 199 with rings of four and five CTAs, while the 64x64x160 bar has items
+// enough and takes 1.14 ms with more CTAs against 1.44 (an earlier form of the
+// kernel, 64-column bands throughout).  The line lies between the two last:
+// kBwdDeepBytes of [Y; W].
+constexpr int SOLVE_WARPS = 4;
+constexpr int SOLVE_THREADS = 32 * SOLVE_WARPS;
+constexpr int FWD_MINB = 5;           // CTAs per SM
+constexpr int FRING = 4;              // stages in flight per CTA
+constexpr int ST_C = 16;              // columns of a stage
+constexpr int FR = TL;                // doubles per staged column of a warp (4 of the stage's 16 columns)
+constexpr int ring_doubles(int stages) { return stages * ST_C * FR; }
+constexpr int FWD_RING = ring_doubles(FRING);
+constexpr int solve_smem(int stages) { return (ring_doubles(stages) + (SCH + TL) * 3) * (int)sizeof(double); }
+static_assert(ST_C % SOLVE_WARPS == 0 && TL == 64 && SOLVE_WARPS == 4, "the warps' shares of a stage");
+static_assert(3 * TL <= FRING * (ST_C / SOLVE_WARPS) * FR, "a forward warp's sums reuse its ring");
 
-// Takes the CTA's next item (in every thread).  Thread 0 keeps the index it
-// fetched for the item after it in a register (`ahead`), so the atomic's
-// round trip runs while the current item is worked on; only its use, one item
-// later, waits for it.
-__device__ __forceinline__ int next_item(const SolveQueue& Q, int* s_cur, int& ahead) {
-    __syncthreads();   // the previous item's shared-memory use is over
-    if (threadIdx.x == 0) {
-        const int cur = ahead;
-        *s_cur = cur;
-        if (cur < Q.n) ahead = static_cast<int>(atomicAdd(Q.head, 1u));
-    }
+// Forward: lane l of warp w holds rows b0 + 2l and b0 + 2l + 1 of the band and
+// takes columns w, w + 4, ... of the chunk; the warps' sums are added in warp
+// order.
+__global__ void __launch_bounds__(SOLVE_THREADS, FWD_MINB)
+    k_fwd_queue(const double* __restrict__ B, double* __restrict__ Zb, double* __restrict__ Xp, double* U,
+                const int* __restrict__ inv, const double* __restrict__ YW, SolveQueue Q, double* P,
+                const int* __restrict__ mesh_on) {
+    constexpr int NT = SOLVE_THREADS, TPT = SCH / NT, WC = ST_C / SOLVE_WARPS;
+    __shared__ __align__(16) ItemSlot slots[2];
+    extern __shared__ __align__(16) double ssm[];
+    double* tv = ssm + FWD_RING;          // [SCH][3]
+    double* vrow = tv + SCH * 3;                 // [TL][3]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double* ring = ssm + warp * (FRING * WC * FR);
+    if (blockIdx.x == 0 && tid == 0) *Q.other_head = 0u;
+    if (warp == SOLVE_WARPS - 1) fetch_item(Q, lane == 0 ? (int)atomicAdd(Q.head, 1u) : 0, &slots[0]);
     __syncthreads();
-    return *s_cur;
-}
-
-__global__ void __launch_bounds__(32 * FWD_WARPS, 8) k_fwd_queue(const double* __restrict__ B, double* __restrict__ Zb,
-                                                   double* __restrict__ U, const int64_t* __restrict__ inv,
-                                                   const double* __restrict__ YW, const FrontDesc* __restrict__ desc,
-                                                   SolveQueue Q, double* __restrict__ P, unsigned* __restrict__ counters,
-                                                   const int* __restrict__ mesh_on) {
-    __shared__ int s_cur, s_ok;
-    int ahead = threadIdx.x == 0 ? static_cast<int>(atomicAdd(Q.head, 1u)) : 0;
-    for (;;) {
-        const int q = next_item(Q, &s_cur, ahead);
+    for (int turn = 0;; turn ^= 1) {
+        const int q = slots[turn].q;
         if (q >= Q.n) break;
-        const SolveItem it = Q.items[q];
-        const FrontDesc d = desc[it.front];
-        if (mesh_on && !mesh_on[d.mesh]) continue;
-        double2 pre[FWD_PRE];
-        fwd_pre(YW, d, it, pre);   // in flight during the wait
-        if (threadIdx.x == 0) {
-            bool ok = d.child0 < 0 || wait_bands(Q.done + d.child0, Q.nbands[d.child0], Q.status);
-            ok = ok && (d.child1 < 0 || wait_bands(Q.done + d.child1, Q.nbands[d.child1], Q.status));
-            s_ok = ok;
+        const SolveWork& it = slots[turn].it;
+        int ticket = 0;
+        const bool on = !mesh_on || mesh_on[it.mesh];
+        bool ok = true;
+        if (on) {
+            const int nc = it.hi - it.lo, nst = (nc + ST_C - 1) / ST_C;
+            const int64_t ldy = it.ldy;
+            const double* M = YW + it.m_off + 2 * lane;
+            const bool live = it.b0 + 2 * lane < it.R;
+            auto issue = [&](int s) {
+                if (s < nst) {
+                    double* dst = ring + (s % FRING) * (WC * FR) + 2 * lane;
+#pragma unroll
+                    for (int u = 0; u < WC; ++u) {
+                        const int j = s * ST_C + warp + SOLVE_WARPS * u;
+                        const bool v = live && j < nc;
+                        cp_async16(dst + u * FR, v ? M + (int64_t)j * ldy : M, v ? 16 : 0);
+                    }
+                }
+                cp_async_commit();
+            };
+#pragma unroll
+            for (int s = 0; s < FRING; ++s) issue(s);
+            // the children's entries of the chunk's columns and, in the band's
+            // last item, of its rows
+            int2 iv[TPT];
+            const int2* inv2 = reinterpret_cast<const int2*>(inv) + it.aux;
+#pragma unroll
+            for (int m = 0; m < TPT; ++m) {
+                const int j = tid + m * NT;
+                iv[m] = (it.leaf || j >= nc) ? make_int2(-1, -1) : __ldg(inv2 + it.lo + j);
+            }
+            const bool owner = q == it.first + it.nchunk - 1;
+            const int vr = tid - (NT - TL);   // threads NT - TL .. NT - 1: row vr of the band
+            int2 ivr = make_int2(-1, -1);
+            if (owner && vr >= 0 && it.b0 + vr >= it.k && it.b0 + vr < it.R && !it.leaf) ivr = __ldg(inv2 + it.b0 + vr);
+            if (Q.gate && (it.gate0 >= 0 || it.gate1 >= 0)) {
+                // a large system: one thread polls until the item's inputs are about
+                // there, so that waiting CTAs leave the L2 to the streaming ones; the
+                // others poll at once, which saves a round trip per level (forward +
+                // backward on the 8x8x32, 16x16x64, 24x24x48, 32x32x128 bars: 31, 72, 103,
+                // 313 us polling at once, 35, 81, 115, 309 us gated)
+                if (tid == 0) {
+                    const double* const p[2] = {it.gate0 >= 0 ? U + 3 * (int64_t)it.gate0 : nullptr,
+                                                it.gate1 >= 0 ? U + 3 * (int64_t)it.gate1 : nullptr};
+                    double g[2][3];
+                    await3(p, g, Q.status);
+                }
+                __syncthreads();
+            }
+            if (tid == NT - 32) ticket = (int)atomicAdd(Q.head, 1u);
+            {
+                const double* p[2 * TPT + 2];
+                double c[2 * TPT + 2][3];
+#pragma unroll
+                for (int m = 0; m < TPT; ++m) {
+                    p[2 * m] = iv[m].x >= 0 ? U + 3 * (int64_t)iv[m].x : nullptr;
+                    p[2 * m + 1] = iv[m].y >= 0 ? U + 3 * (int64_t)iv[m].y : nullptr;
+                }
+                p[2 * TPT] = ivr.x >= 0 ? U + 3 * (int64_t)ivr.x : nullptr;
+                p[2 * TPT + 1] = ivr.y >= 0 ? U + 3 * (int64_t)ivr.y : nullptr;
+                ok = await3(p, c, Q.status);
+#pragma unroll
+                for (int m = 0; m < TPT; ++m) {
+                    const int j = tid + m * NT;
+                    double v[3] = {0.0, 0.0, 0.0};
+                    if (j < nc && it.lo + j < it.k) {
+                        const double* b = B + 3 * ((int64_t)it.col + it.lo + j);
+                        v[0] = b[0]; v[1] = b[1]; v[2] = b[2];
+                    }
+                    if (j < nst * ST_C)
+#pragma unroll
+                        for (int e = 0; e < 3; ++e) tv[3 * j + e] = v[e] + c[2 * m][e] + c[2 * m + 1][e];
+                }
+                if (owner && vr >= 0)
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) vrow[3 * vr + e] = c[2 * TPT][e] + c[2 * TPT + 1][e];
+            }
+            ok = __syncthreads_and(ok);
+            double a0 = 0.0, a1 = 0.0, a2 = 0.0, b0 = 0.0, b1 = 0.0, b2 = 0.0;
+            for (int s = 0; s < nst; ++s) {
+                cp_async_wait<FRING - 1>();   // own copies only: no barrier
+                const double* src = ring + (s % FRING) * (WC * FR) + 2 * lane;
+                const double* t = tv + 3 * (s * ST_C + warp);
+#pragma unroll
+                for (int u = 0; u < WC; ++u) {
+                    const double2 m = *reinterpret_cast<const double2*>(src + u * FR);
+                    const double t0 = t[12 * u], t1 = t[12 * u + 1], t2 = t[12 * u + 2];
+                    a0 = fma(m.x, t0, a0); a1 = fma(m.x, t1, a1); a2 = fma(m.x, t2, a2);
+                    b0 = fma(m.y, t0, b0); b1 = fma(m.y, t1, b1); b2 = fma(m.y, t2, b2);
+                }
+                asm volatile("" ::: "memory");   // the stage is read before it is refilled
+                issue(s + FRING);
+            }
+            cp_async_wait<0>();
+            __syncwarp();
+            // the warp's sums, in its own ring
+            ring[6 * lane] = a0; ring[6 * lane + 1] = a1; ring[6 * lane + 2] = a2;
+            ring[6 * lane + 3] = b0; ring[6 * lane + 4] = b1; ring[6 * lane + 5] = b2;
+            __syncthreads();
+            const int row = tid, i = it.b0 + row;
+            if (ok && row < TL && i < it.R) {
+                double s[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+                for (int w = 0; w < SOLVE_WARPS; ++w) {
+                    const double* pw = ssm + w * (FRING * WC * FR) + 3 * row;
+                    s[0] += pw[0]; s[1] += pw[1]; s[2] += pw[2];
+                }
+                if (!owner) {
+                    double* p = P + 3 * ((int64_t)q * TL + row);
+                    st_relaxed(p, s[0]); st_relaxed(p + 1, s[1]); st_relaxed(p + 2, s[2]);
+                } else if (it.nchunk == 1 || add_chunks(P, it.first, it.nchunk, row, s, Q.status)) {
+                    if (i < it.k) {
+                        const int64_t o = 3 * ((int64_t)it.col + i);
+                        Zb[o] = s[0]; Zb[o + 1] = s[1]; Zb[o + 2] = s[2];
+                        st_unset3(Xp + o);
+                    } else if (it.col != Q.hold) {
+                        double* u = U + 3 * ((int64_t)it.u_row + i - it.k);
+                        st_relaxed(u, vrow[3 * row] - s[0]);
+                        st_relaxed(u + 1, vrow[3 * row + 1] - s[1]);
+                        st_relaxed(u + 2, vrow[3 * row + 2] - s[2]);
+                    }
+                }
+            }
+        } else if (tid == NT - 32) {
+            ticket = (int)atomicAdd(Q.head, 1u);
         }
-        __syncthreads();
-        if (!s_ok) continue;
-        if (fwd_item(B, Zb, U, inv, YW, d, it, q, P, counters, pre) && threadIdx.x == 0 && it.front != Q.hold)
-            atomicAdd(Q.done + it.front, 1u);
+        if (warp == SOLVE_WARPS - 1) fetch_item(Q, ticket, &slots[turn ^ 1]);
+        __syncthreads();   // the next record is there; this item's shared memory is free
     }
 }
 
-__global__ void __launch_bounds__(256) k_bwd_queue(double* __restrict__ x, const double* __restrict__ Zb,
-                                                   const double* __restrict__ YW, const int* __restrict__ rows,
-                                                   const FrontDesc* __restrict__ desc, SolveQueue Q,
-                                                   double* __restrict__ P, unsigned* __restrict__ counters,
-                                                   const int* __restrict__ mesh_on) {
-    __shared__ int s_cur, s_ok;
-    int ahead = threadIdx.x == 0 ? static_cast<int>(atomicAdd(Q.head, 1u)) : 0;
-    for (;;) {
-        const int q = next_item(Q, &s_cur, ahead);
+// Backward: warp w takes columns 4 w .. 4 w + 3 of each stage (16 of the band's
+// 64 columns, one 64-row block of the chunk; a column group's row blocks follow
+// each other).  Lane 8 c + p has column c and row pairs p, p + 8, p + 16, p + 24 of the
+// block, a sum for each: the pairs are added as a tree over pair bits 16, 8 (in
+// the lane), 4, 2, 1 (across lanes).  The input of row i is z_i for i < k and
+// minus the solution at the front's row i - k for i >= k.
+template <int BRING, int MINB>
+__global__ void __launch_bounds__(SOLVE_THREADS, MINB)
+    k_bwd_queue(double* __restrict__ x, const double* __restrict__ Zb, double* Xp, double* __restrict__ U,
+                const double* __restrict__ YW, const int* __restrict__ rows, SolveQueue Q, double* P,
+                const int* __restrict__ mesh_on) {
+    constexpr int NT = SOLVE_THREADS, TPT = SCH / NT, WC = ST_C / SOLVE_WARPS, NG = TL / ST_C;
+    __shared__ __align__(16) ItemSlot slots[2];
+    extern __shared__ __align__(16) double ssm[];
+    double* in = ssm + BRING * SOLVE_WARPS * WC * FR;   // [SCH][3], zero past the chunk
+    double* res = in + SCH * 3;                                // [TL][3]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double* ring = ssm + warp * (BRING * WC * FR);
+    if (blockIdx.x == 0 && tid == 0) *Q.other_head = 0u;
+    if (warp == SOLVE_WARPS - 1) fetch_item(Q, lane == 0 ? (int)atomicAdd(Q.head, 1u) : 0, &slots[0]);
+    __syncthreads();
+    for (int turn = 0;; turn ^= 1) {
+        const int q = slots[turn].q;
         if (q >= Q.n) break;
-        const SolveItem it = Q.items[q];
-        const FrontDesc d = desc[it.front];
-        if (mesh_on && !mesh_on[d.mesh]) continue;
-        double2 pre[8];
-        bwd_pre(YW, d, it, pre);   // in flight during the wait
-        if (threadIdx.x == 0)
-            s_ok = d.parent < 0 || wait_bands(Q.done + d.parent, Q.nbands[d.parent], Q.status);
+        const SolveWork& it = slots[turn].it;
+        int ticket = 0;
+        const bool on = !mesh_on || mesh_on[it.mesh];
+        bool ok = true;
+        if (on) {
+            const int nr = it.hi - it.lo, nc = min(it.w, it.k - it.b0);
+            const int nrb = (nr + TL - 1) / TL, ng = (nc + ST_C - 1) / ST_C;   // row blocks, column groups
+            const int64_t ldy = it.ldy;
+            const double* M = YW + it.m_off + 2 * lane + (int64_t)(WC * warp) * ldy;
+            // the next stage to copy: its group and row block, its place in the ring
+            int ig = 0, irb = 0, is = 0;
+            auto issue = [&]() {
+                if (ig < ng) {
+                    double* dst = ring + is * (WC * FR) + 2 * lane;
+                    const double* src = M + irb * TL + (int64_t)(ig * ST_C) * ldy;
+                    const bool live = irb * TL + 2 * lane < nr;
+#pragma unroll
+                    for (int u = 0; u < WC; ++u) {
+                        const bool v = live && ig * ST_C + WC * warp + u < nc;
+                        cp_async16(dst + u * FR, v ? src + (int64_t)u * ldy : M, v ? 16 : 0);
+                    }
+                    if (++irb == nrb) { irb = 0; ++ig; }
+                    is = is + 1 == BRING ? 0 : is + 1;
+                }
+                cp_async_commit();
+            };
+#pragma unroll
+            for (int s = 0; s < BRING; ++s) issue();
+            const bool owner = q == it.first + it.nchunk - 1;
+            int row[TPT];
+            double v[TPT][3];
+#pragma unroll
+            for (int m = 0; m < TPT; ++m) {
+                const int t = tid + m * NT, i = it.lo + t;
+                row[m] = -1;
+                v[m][0] = v[m][1] = v[m][2] = 0.0;
+                if (t < nr) {
+                    if (i < it.k) {
+                        const double* z = Zb + 3 * ((int64_t)it.col + i);
+                        v[m][0] = z[0]; v[m][1] = z[1]; v[m][2] = z[2];
+                    } else {
+                        row[m] = __ldg(rows + it.aux + i - it.k);
+                        // the forward pass is done with U: unset it for the next solve
+                        if (it.b0 == 0) st_unset3(U + 3 * ((int64_t)it.u_row + i - it.k));
+                    }
+                }
+            }
+            if (Q.gate && it.gate0 >= 0) {
+                if (tid == 0) {
+                    const double* const p[1] = {Xp + 3 * (int64_t)it.gate0};
+                    double g[1][3];
+                    await3(p, g, Q.status);
+                }
+                __syncthreads();
+            }
+            if (tid == NT - 32) ticket = (int)atomicAdd(Q.head, 1u);
+            {
+                const double* p[TPT];
+                double y[TPT][3];
+#pragma unroll
+                for (int m = 0; m < TPT; ++m) p[m] = row[m] >= 0 ? Xp + 3 * (int64_t)row[m] : nullptr;
+                ok = await3(p, y, Q.status);
+#pragma unroll
+                for (int m = 0; m < TPT; ++m) {
+                    const int t = tid + m * NT;
+                    if (t < nrb * TL)
+#pragma unroll
+                        for (int e = 0; e < 3; ++e) in[3 * t + e] = row[m] >= 0 ? -y[m][e] : v[m][e];
+                }
+            }
+            ok = __syncthreads_and(ok);
+            const int cl = lane >> 3, pr = lane & 7;
+            int cs = 0;   // the stage's place in the ring
+            for (int g = 0; g < ng; ++g) {
+                double a[4][3];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) a[e][0] = a[e][1] = a[e][2] = 0.0;
+                for (int rb = 0; rb < nrb; ++rb) {
+                    cp_async_wait<BRING - 1>();
+                    __syncwarp();   // the warp's copies are all there
+                    const double* src = ring + cs * (WC * FR) + cl * FR + 2 * pr;
+                    const double2* xin = reinterpret_cast<const double2*>(in + 3 * (rb * TL + 2 * pr));
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const double2 m = *reinterpret_cast<const double2*>(src + 16 * e);
+                        const double2 x0 = xin[24 * e], x1 = xin[24 * e + 1], x2 = xin[24 * e + 2];   // rows 2l, 2l + 1
+                        a[e][0] = fma(m.y, x1.y, fma(m.x, x0.x, a[e][0]));
+                        a[e][1] = fma(m.y, x2.x, fma(m.x, x0.y, a[e][1]));
+                        a[e][2] = fma(m.y, x2.y, fma(m.x, x1.x, a[e][2]));
+                    }
+                    cs = cs + 1 == BRING ? 0 : cs + 1;
+                    __syncwarp();   // the stage is read
+                    issue();
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    double t = (a[0][c] + a[2][c]) + (a[1][c] + a[3][c]);
+                    t += __shfl_xor_sync(0xffffffffu, t, 4);
+                    t += __shfl_xor_sync(0xffffffffu, t, 2);
+                    t += __shfl_xor_sync(0xffffffffu, t, 1);
+                    if (pr == 0) res[3 * (g * ST_C + WC * warp + cl) + c] = t;
+                }
+            }
+            __syncthreads();
+            const int j = tid;
+            if (ok && j < nc) {
+                double s[3] = {res[3 * j], res[3 * j + 1], res[3 * j + 2]};
+                if (!owner) {
+                    double* p = P + 3 * ((int64_t)q * TL + j);
+                    st_relaxed(p, s[0]); st_relaxed(p + 1, s[1]); st_relaxed(p + 2, s[2]);
+                } else if (it.nchunk == 1 || add_chunks(P, it.first, it.nchunk, j, s, Q.status)) {
+                    const int64_t o = 3 * ((int64_t)it.col + it.b0 + j);
+                    if (it.col != Q.hold) {
+                        st_relaxed(Xp + o, s[0]); st_relaxed(Xp + o + 1, s[1]); st_relaxed(Xp + o + 2, s[2]);
+                    }
+                    x[o] = s[0]; x[o + 1] = s[1]; x[o + 2] = s[2];
+                }
+            }
+        } else if (tid == NT - 32) {
+            ticket = (int)atomicAdd(Q.head, 1u);
+        }
+        if (warp == SOLVE_WARPS - 1) fetch_item(Q, ticket, &slots[turn ^ 1]);
         __syncthreads();
-        if (!s_ok) continue;
-        if (bwd_item(x, Zb, YW, rows, d, it, q, P, counters, pre) && threadIdx.x == 0 && it.front != Q.hold)
-            atomicAdd(Q.done + it.front, 1u);
     }
 }
 
@@ -1019,6 +1093,12 @@ CholGPU::~CholGPU() {
     if (factor_graph_) cudaGraphExecDestroy(factor_graph_);
     if (solve_graph_) cudaGraphExecDestroy(solve_graph_);
     for (void* p : allocs_) cudaFree(p);
+}
+
+void CholGPU::release(void* p) {
+    if (!p) return;
+    cudaFree(p);
+    allocs_.erase(std::remove(allocs_.begin(), allocs_.end(), p), allocs_.end());
 }
 
 template <typename X>
@@ -1071,6 +1151,13 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
                     const std::vector<int>& A_contrib, cudaStream_t st) {
     WRAPD_CUDA(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM));
     WRAPD_CUDA(cudaFuncSetAttribute(k_wgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM));
+    WRAPD_CUDA(cudaFuncSetAttribute(k_fwd_queue, cudaFuncAttributeMaxDynamicSharedMemorySize, solve_smem(FRING)));
+    // deep rings for latency, or more CTAs per SM for throughput (see k_bwd_queue)
+    const size_t yw_bytes = (size_t)S.y_pool * sizeof(double);
+    bwd_smem_ = yw_bytes <= kBwdDeepBytes ? solve_smem(8) : solve_smem(4);
+    bwd_fn_ = yw_bytes <= kBwdDeepBytes ? k_bwd_queue<8, 3> : k_bwd_queue<4, 5>;
+    solve_gate_ = yw_bytes > kGateBytes;
+    WRAPD_CUDA(cudaFuncSetAttribute(bwd_fn_, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem_));
     n = S.n;
     nfronts = static_cast<int>(S.fronts.size());
     nlevels = static_cast<int>(S.levels.size());
@@ -1096,16 +1183,19 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
         d.mesh = front_mesh.empty() ? 0 : front_mesh[f];
         d.parent = F.parent;
     }
-    std::vector<int64_t> inv(ioff, -1);
+    if (S.u_pool / 3 > INT32_MAX) throw CudaError(WRAPD_E_INPUT, "solve update vectors exceed 32-bit row indexes");
+    h_inv_.assign(ioff, -1);
     for (int f = 0; f < nfronts; ++f) {
         const Front& F = S.fronts[f];
         for (size_t q = 0; q < F.children.size(); ++q) {
             const Front& C = S.fronts[F.children[q]];
             for (int i = 0; i < C.nrows(); ++i)
-                inv[h_desc_[f].inv_off + 2 * (int64_t)S.relmap[C.rel_off + i] + (int64_t)q] = C.u_off + 3 * (int64_t)i;
+                h_inv_[h_desc_[f].inv_off + 2 * (int64_t)S.relmap[C.rel_off + i] + (int64_t)q] =
+                    static_cast<int>(C.u_off / 3) + i;
         }
     }
-    d_inv_ = upload(inv, st);
+    d_inv_ = upload(h_inv_, st);
+    h_rows_ = rows;
     d_desc_ = upload(h_desc_, st);
     d_rows_ = upload(rows, st);
     d_rel_ = upload(S.relmap, st);
@@ -1127,7 +1217,7 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
     d_F_ = dalloc(f_pool_);
     d_Y_ = dalloc(y_pool_);
     d_U_ = dalloc(u_pool_);
-    d_T_ = dalloc(3 * (size_t)n);
+    d_Xp_ = dalloc(3 * (size_t)n);
     d_Z_ = dalloc(3 * (size_t)n);
     int* st_ptr = nullptr;
     WRAPD_CUDA(cudaMalloc(&st_ptr, sizeof(int)));
@@ -1191,9 +1281,8 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
             wg[q] = ceil_div(d.r, TL) * ceil_div(d.k, TL);
         }
         // Solve items with chunks of sch_of(front) (<= SCH) along the streamed dimension.
-        auto fwd_items = [&](auto sch_of, std::vector<SolveItem>& fwd, int& fbands) {
+        auto fwd_items = [&](auto sch_of, std::vector<SolveItem>& fwd) {
             fwd.clear();
-            fbands = 0;
             for (int f : fs) {
                 const int sch = sch_of(f);
                 const FrontDesc& d = h_desc_[f];
@@ -1203,14 +1292,12 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
                     const int cend = b0 < d.k ? std::min(d.k, b0 + TL) : d.k;
                     const int nch = ceil_div(cend, sch), first = static_cast<int>(fwd.size());
                     for (int c = 0; c < nch; ++c)
-                        fwd.push_back({f, b0, c * sch, std::min(cend, (c + 1) * sch), nch, first, fbands});
-                    fbands++;
+                        fwd.push_back({f, b0, c * sch, std::min(cend, (c + 1) * sch), nch, first});
                 }
             }
         };
-        auto bwd_items = [&](auto sch_of, std::vector<SolveItem>& bwd, int& bbands) {
+        auto bwd_items = [&](auto sch_of, std::vector<SolveItem>& bwd) {
             bwd.clear();
-            bbands = 0;
             for (int f : fs) {
                 const int sch = sch_of(f);
                 const FrontDesc& d = h_desc_[f];
@@ -1218,20 +1305,19 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
                 // backward: column bands over rows [b0, R) (Y rows below the band, then the W rows)
                 for (int b0 = 0; b0 < d.k; b0 += TL) {
                     const int nch = ceil_div(R - b0, sch), first = static_cast<int>(bwd.size());
-                    for (int lo = b0; lo < R; lo += sch) bwd.push_back({f, b0, lo, std::min(R, lo + sch), nch, first, bbands});
-                    bbands++;
+                    for (int lo = b0; lo < R; lo += sch) bwd.push_back({f, b0, lo, std::min(R, lo + sch), nch, first});
                 }
             }
         };
-        // Candidate chunk lengths SCH, SCH/2, ..., SCH_MIN, all uploaded.  The fixed
-        // rule takes chunks as long as possible (fewer partial sums) while the
-        // launch still has kSolveCtas CTAs: the upper levels of a large system
-        // hold a few large fronts, and long chunks there leave most SMs idle with
-        // each CTA latency-bound.  When not even the shortest chunks fill the GPU
-        // (a small system) the longest are kept.  autotune() may pick another
-        // candidate by timing.
+        // Candidate chunk lengths SCH, SCH/2, ..., SCH_MIN.  The fixed rule takes
+        // chunks as long as possible (fewer partial sums to hand over) while the
+        // level still has kSolveItems items: the levels near the root of a large
+        // system hold a few large fronts, and long chunks there leave most SMs
+        // idle.  When not even the shortest chunks give that many (a small system)
+        // the longest are kept.  The chunks alone decide the order in which a sum
+        // is added, so that they are the same for a mesh of a batch as for the mesh
+        // alone.  autotune() may pick another candidate by timing.
         std::vector<SolveItem> fwd, bwd;
-        int fbands = 0, bbands = 0;
         L.cfwd = -1;
         L.cbwd = -1;
         // per mesh of a batch: its item counts for each candidate (the rule
@@ -1239,14 +1325,11 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
         const int nmesh = front_mesh.empty() ? 1 : 1 + *std::max_element(front_mesh.begin(), front_mesh.end());
         std::vector<std::vector<int>> mfwd(nmesh), mbwd(nmesh);
         for (int sch = SCH, c = 0; sch >= SCH_MIN; sch /= 2, ++c) {
-            fwd_items([&](int) { return sch; }, fwd, fbands);
-            bwd_items([&](int) { return sch; }, bwd, bbands);
-            L.cand.push_back({sch, upload(fwd, st), static_cast<int>(fwd.size()), upload(bwd, st),
-                              static_cast<int>(bwd.size()), fwd, bwd});
-            if (L.cfwd < 0 && (int)fwd.size() >= kSolveCtas) L.cfwd = c;
-            if (L.cbwd < 0 && (int)bwd.size() >= kSolveCtas) L.cbwd = c;
-            solve_parts_ = std::max<int64_t>(solve_parts_, std::max<int64_t>(fwd.size(), bwd.size()));
-            solve_bands_ = std::max(solve_bands_, std::max(fbands, bbands));
+            fwd_items([&](int) { return sch; }, fwd);
+            bwd_items([&](int) { return sch; }, bwd);
+            L.cand.push_back({sch, fwd, bwd});
+            if (L.cfwd < 0 && (int)fwd.size() >= kSolveItems) L.cfwd = c;
+            if (L.cbwd < 0 && (int)bwd.size() >= kSolveItems) L.cbwd = c;
             if (nmesh > 1) {
                 for (int m = 0; m < nmesh; ++m) { mfwd[m].push_back(0); mbwd[m].push_back(0); }
                 for (const SolveItem& it : fwd) mfwd[front_mesh[it.front]][c]++;
@@ -1261,19 +1344,16 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
             for (int m = 0; m < nmesh; ++m) {
                 int cf = -1, cb = -1;
                 for (int c = 0; c < (int)mfwd[m].size(); ++c) {
-                    if (cf < 0 && mfwd[m][c] >= kSolveCtas) cf = c;
-                    if (cb < 0 && mbwd[m][c] >= kSolveCtas) cb = c;
+                    if (cf < 0 && mfwd[m][c] >= kSolveItems) cf = c;
+                    if (cb < 0 && mbwd[m][c] >= kSolveItems) cb = c;
                 }
                 sf[m] = SCH >> std::max(cf, 0);
                 sb[m] = SCH >> std::max(cb, 0);
             }
-            fwd_items([&](int f) { return sf[front_mesh[f]]; }, fwd, fbands);
-            bwd_items([&](int f) { return sb[front_mesh[f]]; }, bwd, bbands);
-            L.cand.push_back({0, upload(fwd, st), static_cast<int>(fwd.size()), upload(bwd, st),
-                              static_cast<int>(bwd.size()), fwd, bwd});
+            fwd_items([&](int f) { return sf[front_mesh[f]]; }, fwd);
+            bwd_items([&](int f) { return sb[front_mesh[f]]; }, bwd);
+            L.cand.push_back({0, fwd, bwd});
             L.cfwd = L.cbwd = static_cast<int>(L.cand.size()) - 1;
-            solve_parts_ = std::max<int64_t>(solve_parts_, std::max<int64_t>(fwd.size(), bwd.size()));
-            solve_bands_ = std::max(solve_bands_, std::max(fbands, bbands));
         }
         L.wgemm = make_list(fs, wg, st);
     }
@@ -1284,44 +1364,13 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
         trsm_nP_.push_back(w);
     }
     count_launches();
-    // work queues: room for every level's longest candidate list; the band
-    // counts do not depend on the chunk length
-    int64_t qcap_f = 0, qcap_b = 0;
-    qbands_f_ = qbands_b_ = 0;
-    for (const Level& L : levels_) {
-        int64_t mf = 0, mb = 0;
-        for (const Level::SolveCand& c : L.cand) { mf = std::max<int64_t>(mf, c.nfwd); mb = std::max<int64_t>(mb, c.nbwd); }
-        qcap_f += mf;
-        qcap_b += mb;
-        if (!L.cand.empty()) {
-            const Level::SolveCand& c = L.cand[0];
-            qbands_f_ += c.hfwd.empty() ? 0 : c.hfwd.back().band + 1;
-            qbands_b_ += c.hbwd.empty() ? 0 : c.hbwd.back().band + 1;
-        }
-    }
-    solve_parts_ = std::max<int64_t>(solve_parts_, std::max(qcap_f, qcap_b));
-    d_P_ = dalloc(3 * TL * (size_t)solve_parts_);
-    {
-        unsigned* c = nullptr;
-        WRAPD_CUDA(cudaMalloc(&c, std::max(1, solve_bands_) * sizeof(unsigned)));
-        allocs_.push_back(c);
-        device_bytes += std::max(1, solve_bands_) * sizeof(unsigned);
-        d_cnt_ = c;
-        WRAPD_CUDA(cudaMemsetAsync(d_cnt_, 0, std::max(1, solve_bands_) * sizeof(unsigned), st));
-    }
-    d_qf_ = upload(std::vector<SolveItem>(std::max<int64_t>(1, qcap_f)), st);
-    d_qb_ = upload(std::vector<SolveItem>(std::max<int64_t>(1, qcap_b)), st);
-    d_qnb_ = upload(std::vector<unsigned>(2 * (size_t)std::max(1, nfronts)), st);
-    qcap_f_ = qcap_f;
-    qcap_b_ = qcap_b;
-    qctl_words_ = 2 + 2 * (size_t)nfronts + qbands_f_ + qbands_b_;
-    d_qctl_ = upload(std::vector<unsigned>(qctl_words_), st);
+    d_heads_ = upload(std::vector<unsigned>(2, 0u), st);
     {
         int dev = 0, sms = 0, bf = 0, bb = 0;
         WRAPD_CUDA(cudaGetDevice(&dev));
         WRAPD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        WRAPD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bf, k_fwd_queue, 32 * FWD_WARPS, 0));
-        WRAPD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, k_bwd_queue, 256, 0));
+        WRAPD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bf, k_fwd_queue, SOLVE_THREADS, solve_smem(FRING)));
+        WRAPD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, bwd_fn_, SOLVE_THREADS, bwd_smem_));
         qgrid_f_ = std::max(1, bf) * sms;
         qgrid_b_ = std::max(1, bb) * sms;
     }
@@ -1330,58 +1379,134 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
 }
 
 // The chosen candidate of every level, concatenated: forward leaves first,
-// backward root first, with item and band indexes made global (each
-// direction's bands numbered from 0 in its own counter range).  Every index
-// the kernels will use is checked against its buffer here.
+// backward root first, each item with the front's numbers it needs and the
+// entries its first poll looks at: the last of its inputs that each child
+// writes (forward), the nearest ancestor's (backward).  Every index the kernels
+// will use is checked against its buffer here.
 void CholGPU::build_queues(cudaStream_t st) {
-    std::vector<SolveItem> qf, qb;
-    std::vector<unsigned> nb(2 * (size_t)std::max(1, nfronts), 0u);
-    auto append = [&](const std::vector<SolveItem>& src, std::vector<SolveItem>& q, int& bands, unsigned* nbands) {
-        const int i0 = static_cast<int>(q.size()), b0 = bands;
-        for (size_t i = 0; i < src.size(); ++i) {
-            SolveItem g = src[i];
-            if ((int)i == g.first) nbands[g.front]++;   // the first chunk of a band
-            g.first += i0;
-            g.band += b0;
-            bands = std::max(bands, g.band + 1);
-            q.push_back(g);
-        }
+    std::vector<SolveWork> qf, qb;
+    auto work = [&](const SolveItem& g, int first) {
+        const FrontDesc& d = h_desc_[g.front];
+        SolveWork w{};
+        w.ldy = d.ldy; w.k = d.k; w.R = d.k + d.r; w.col = d.first;
+        w.b0 = g.b0; w.lo = g.lo; w.hi = g.hi; w.nchunk = g.nchunk; w.w = TL;
+        w.first = first; w.gate0 = w.gate1 = -1; w.mesh = d.mesh;
+        w.u_row = static_cast<int>(d.u_off / 3);
+        w.leaf = d.child0 < 0 && d.child1 < 0;
+        return w;
     };
-    int bf = 0, bb = 0;
     for (int l = 0; l < nlevels; ++l) {
         const Level& L = levels_[l];
-        if (!L.cand.empty()) append(L.cand[L.cfwd].hfwd, qf, bf, nb.data());
+        if (L.cand.empty()) continue;
+        const int base = static_cast<int>(qf.size());
+        for (const SolveItem& g : L.cand[L.cfwd].fwd) {
+            const FrontDesc& d = h_desc_[g.front];
+            SolveWork w = work(g, base + g.first);
+            w.m_off = d.y_off + g.b0 + (int64_t)g.lo * d.ldy;
+            w.aux = d.inv_off / 2;
+            for (int i = g.hi - 1; i >= g.lo && !w.leaf && (w.gate0 < 0 || w.gate1 < 0); --i) {
+                if (w.gate0 < 0) w.gate0 = h_inv_[d.inv_off + 2 * (int64_t)i];
+                if (w.gate1 < 0) w.gate1 = h_inv_[d.inv_off + 2 * (int64_t)i + 1];
+            }
+            qf.push_back(w);
+        }
     }
     for (int l = nlevels - 1; l >= 0; --l) {
         const Level& L = levels_[l];
-        if (!L.cand.empty()) append(L.cand[L.cbwd].hbwd, qb, bb, nb.data() + nfronts);
+        if (L.cand.empty()) continue;
+        const std::vector<SolveItem>& items = L.cand[L.cbwd].bwd;
+        // A level with few items works on bands of 16 columns, four times the items
+        // (a column's sum does not depend on its band's width): backward, 8x8x32,
+        // 13x11x37, 16x16x64, 24x24x48 and 32x32x128 bars, 12, 22, 36, 69, 164 us
+        // against 19, 33, 62, 80, 175 with bands of 64 (32: 14, 25, 45, 71, 165).
+        // With the line at twice kSolveItems: 12, 22, 36, 84, 216.
+        const int nsub = (int)items.size() < kSolveItems ? kBwdSub : 1, wd = TL / nsub;
+        for (size_t i = 0; i < items.size();) {
+            const int nch = items[i].nchunk;
+            for (int sub = 0; sub < nsub; ++sub) {
+                const int first = static_cast<int>(qb.size());
+                for (int c = 0; c < nch; ++c) {
+                    const SolveItem& g = items[i + c];
+                    const FrontDesc& d = h_desc_[g.front];
+                    if (g.b0 + sub * wd >= d.k) break;
+                    SolveWork w = work(g, first);
+                    w.b0 = g.b0 + sub * wd;
+                    w.w = wd;
+                    w.m_off = d.y_off + g.lo + (int64_t)w.b0 * d.ldy;
+                    w.aux = d.rows_off;
+                    if (g.hi > d.k) w.gate0 = h_rows_[d.rows_off + std::max(g.lo, d.k) - d.k];
+                    qb.push_back(w);
+                }
+            }
+            i += nch;
+        }
     }
-    auto check = [&](const std::vector<SolveItem>& q, int64_t cap, int nbands, const char* what) {
-        if ((int64_t)q.size() > cap || (int64_t)q.size() > solve_parts_)
-            throw CudaError(WRAPD_E_INPUT, std::string("solve queue longer than its buffers: ") + what);
+    auto check = [&](const std::vector<SolveWork>& q, bool fwd) {
+        if (q.size() > (size_t)INT32_MAX / (3 * TL)) throw CudaError(WRAPD_E_INPUT, "solve queue too long");
+        const int64_t gmax = fwd ? u_pool_ / 3 : n;
         for (size_t i = 0; i < q.size(); ++i) {
-            const SolveItem& g = q[i];
-            const bool ok = g.front >= 0 && g.front < nfronts && g.band >= 0 && g.band < nbands && g.nchunk >= 1 &&
-                            g.first >= 0 && g.first <= (int)i && (int64_t)g.first + g.nchunk <= (int64_t)q.size() &&
-                            (int)i < g.first + g.nchunk;
-            if (!ok) throw CudaError(WRAPD_E_INPUT, std::string("solve queue item out of range: ") + what);
+            const SolveWork& g = q[i];
+            const int64_t last = fwd ? g.m_off + std::min(g.w, g.R - g.b0) - 1 + (int64_t)(g.hi - g.lo - 1) * g.ldy
+                                     : g.m_off + (g.hi - g.lo) - 1 + (int64_t)(std::min(g.w, g.k - g.b0) - 1) * g.ldy;
+            const bool ok = g.nchunk >= 1 && g.first >= 0 && g.first <= (int)i && (int)i < g.first + g.nchunk &&
+                            (int64_t)g.first + g.nchunk <= (int64_t)q.size() && g.lo >= 0 && g.lo < g.hi &&
+                            g.hi - g.lo <= SCH && (fwd ? g.hi <= g.k && g.b0 < g.R : g.hi <= g.R && g.b0 < g.k) &&
+                            g.m_off >= 0 && last < y_pool_ && (g.m_off & 1) == 0 && (g.ldy & 1) == 0 &&
+                            g.gate0 < gmax && g.gate1 < gmax && g.col >= 0 && g.col + g.k <= n &&
+                            (int64_t)g.u_row + (g.R - g.k) <= u_pool_ / 3;
+            if (!ok) throw CudaError(WRAPD_E_INPUT, "solve queue item out of range");
         }
     };
-    if (bf != qbands_f_ || bb != qbands_b_) throw CudaError(WRAPD_E_INPUT, "solve queue band count mismatch");
-    check(qf, qcap_f_, qbands_f_, "forward");
-    check(qb, qcap_b_, qbands_b_, "backward");
+    check(qf, true);
+    check(qb, false);
+    // (the buffers grow when the autotuner tries a choice with more items)
+    WRAPD_CUDA(cudaStreamSynchronize(st));
+    auto grow = [&](auto*& p, int64_t& cap, int64_t want, size_t bytes) {
+        if (want <= cap) return;
+        release(p);
+        device_bytes -= (size_t)cap * bytes;
+        p = nullptr;
+        cap = 0;
+        void* q = nullptr;
+        if (cudaMalloc(&q, (size_t)want * bytes) != cudaSuccess) {
+            cudaGetLastError();
+            throw CudaError(WRAPD_E_OOM, "cudaMalloc failed (solve queues)");
+        }
+        allocs_.push_back(q);
+        p = static_cast<std::remove_reference_t<decltype(p)>>(q);
+        cap = want;
+        device_bytes += (size_t)cap * bytes;
+    };
+    grow(d_qf_, qcap_f_, static_cast<int64_t>(qf.size()), sizeof(SolveWork));
+    grow(d_qb_, qcap_b_, static_cast<int64_t>(qb.size()), sizeof(SolveWork));
+    grow(d_P_, solve_parts_, static_cast<int64_t>(std::max(qf.size(), qb.size())), 3 * TL * sizeof(double));
+    reset_solve();
     nqf_ = static_cast<int>(qf.size());
     nqb_ = static_cast<int>(qb.size());
-    if (!qf.empty()) WRAPD_CUDA(cudaMemcpyAsync(d_qf_, qf.data(), qf.size() * sizeof(SolveItem), cudaMemcpyHostToDevice, st));
-    if (!qb.empty()) WRAPD_CUDA(cudaMemcpyAsync(d_qb_, qb.data(), qb.size() * sizeof(SolveItem), cudaMemcpyHostToDevice, st));
-    WRAPD_CUDA(cudaMemcpyAsync(d_qnb_, nb.data(), nb.size() * sizeof(unsigned), cudaMemcpyHostToDevice, st));
+    if (!qf.empty()) WRAPD_CUDA(cudaMemcpyAsync(d_qf_, qf.data(), qf.size() * sizeof(SolveWork), cudaMemcpyHostToDevice, st));
+    if (!qb.empty()) WRAPD_CUDA(cudaMemcpyAsync(d_qb_, qb.data(), qb.size() * sizeof(SolveWork), cudaMemcpyHostToDevice, st));
     WRAPD_CUDA(cudaStreamSynchronize(st));   // the host vectors go out of scope
     if (solve_graph_) { cudaGraphExecDestroy(solve_graph_); solve_graph_ = nullptr; }
 }
 
+// The state that a solve starts from and leaves behind: every hand-over entry
+// unset, both queue heads 0.
+void CholGPU::fill_unset(cudaStream_t st) {
+    auto fill = [&](double* p, int64_t count) {
+        if (count <= 0) return;
+        k_unset<<<ceil_div(count, 256), 256, 0, st>>>(p, count);
+        WRAPD_LAUNCH_CHECK();
+    };
+    fill(d_U_, u_pool_);
+    fill(d_Xp_, 3 * (int64_t)n);
+    fill(d_P_, 3 * TL * solve_parts_);
+    WRAPD_CUDA(cudaMemsetAsync(d_heads_, 0, 2 * sizeof(unsigned), st));
+    solve_stale_ = false;
+}
+
 void CholGPU::count_launches() {
     launches_factor = 4;   // memsets + assembly + identity
-    launches_solve = 2;    // the two queue launches (plus a copy and a memset)
+    launches_solve = 2;    // the two queue launches
     for (const Level& L : levels_) {
         for (const WorkList& e : L.extend) launches_factor += e.total ? 1 : 0;
         for (size_t p = 0; p < L.trsm.size(); ++p) {
@@ -1399,45 +1524,34 @@ std::vector<int> CholGPU::tuning() const {
     return t;
 }
 
-// Each candidate is timed by CUDA events on the handle's stream: one level's
-// solve launch (the mean of three after one untimed), or one whole
-// factorization launched directly (after one untimed at the fixed rule).  The
-// solve launches run on scratch vectors; the factorizations on the current
-// weights, so the factor is valid afterwards whatever the choice.
+// Each candidate is timed by CUDA events on the handle's stream: one whole
+// factorization launched directly (after one untimed at the fixed rule), or,
+// level by level, the solves (the mean of three after one untimed) with that
+// candidate on the level and the choices so far on the others.  The solves run
+// on a scratch vector; the factorizations on the current weights, so the
+// factor is valid afterwards whatever the choice.
 void CholGPU::autotune(const double* d_w2, const double* d_Di, int ne, cudaStream_t st) {
-    cudaEvent_t e0, e1;
-    WRAPD_CUDA(cudaEventCreate(&e0));
-    WRAPD_CUDA(cudaEventCreate(&e1));
+    struct Scratch {   // freed on every path
+        double* x = nullptr;
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        ~Scratch() {
+            if (x) cudaFree(x);
+            if (e0) cudaEventDestroy(e0);
+            if (e1) cudaEventDestroy(e1);
+        }
+    } s;
+    WRAPD_CUDA(cudaEventCreate(&s.e0));
+    WRAPD_CUDA(cudaEventCreate(&s.e1));
     auto timed = [&](int reps, auto&& launch) {
         launch();
-        WRAPD_CUDA(cudaEventRecord(e0, st));
+        WRAPD_CUDA(cudaEventRecord(s.e0, st));
         for (int r = 0; r < reps; ++r) launch();
-        WRAPD_CUDA(cudaEventRecord(e1, st));
-        WRAPD_CUDA(cudaEventSynchronize(e1));
+        WRAPD_CUDA(cudaEventRecord(s.e1, st));
+        WRAPD_CUDA(cudaEventSynchronize(s.e1));
         float ms = 0.f;
-        WRAPD_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        WRAPD_CUDA(cudaEventElapsedTime(&ms, s.e0, s.e1));
         return ms / reps;
     };
-    // (a batch keeps its per-mesh chunk lengths: a mesh's solve stays its own)
-    for (Level& L : levels_) {
-        if (!front_mesh.empty()) break;
-        float best_f = 1e30f, best_b = 1e30f;
-        for (int c = 0; c < (int)L.cand.size(); ++c) {
-            const Level::SolveCand& C = L.cand[c];
-            const float tf = timed(3, [&] {
-                k_fwd_level<<<C.nfwd, 32 * FWD_WARPS, 0, st>>>(d_T_, d_Z_, d_U_, d_inv_, d_Y_, d_desc_, C.fwd, d_P_, d_cnt_,
-                                                    nullptr);
-            });
-            const float tb = timed(3, [&] {
-                k_bwd_level<<<C.nbwd, 256, 0, st>>>(d_T_, d_Z_, d_Y_, d_rows_, d_desc_, C.bwd, d_P_, d_cnt_,
-                                                    nullptr);
-            });
-            WRAPD_LAUNCH_CHECK();
-            if (tf < best_f) { best_f = tf; L.cfwd = c; }
-            if (tb < best_b) { best_b = tb; L.cbwd = c; }
-        }
-    }
-    if (front_mesh.empty()) build_queues(st);
     const int candidates[] = {0, kNumSMs, kFusedPanelCtas, 4 * kFusedPanelCtas, 1 << 30};
     float best = 1e30f;
     int pick = kFusedPanelCtas;
@@ -1451,9 +1565,32 @@ void CholGPU::autotune(const double* d_w2, const double* d_Di, int ne, cudaStrea
     fused_ctas_ = pick;
     count_launches();
     WRAPD_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
+    // (a batch keeps its per-mesh chunk lengths: a mesh's solve stays its own)
+    if (front_mesh.empty()) {
+        const size_t bytes = 3 * (size_t)n * sizeof(double);
+        if (cudaMalloc(&s.x, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            throw CudaError(WRAPD_E_OOM, "cudaMalloc failed (autotuner)");
+        }
+        WRAPD_CUDA(cudaMemsetAsync(s.x, 0, bytes, st));
+        for (Level& L : levels_) {
+            for (int* choice : {&L.cfwd, &L.cbwd}) {
+                float best_t = 1e30f;
+                int best_c = *choice;
+                for (int c = 0; c < (int)L.cand.size(); ++c) {
+                    *choice = c;
+                    build_queues(st);
+                    const float t = timed(3, [&] { solve_launches(s.x, st, nullptr); });
+                    if (t < best_t) { best_t = t; best_c = c; }
+                }
+                *choice = best_c;
+            }
+        }
+        build_queues(st);
+    }
+    WRAPD_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
+    reset_solve();
     WRAPD_CUDA(cudaStreamSynchronize(st));
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
 }
 
 void CholGPU::factor_launches(const double* d_w2, const double* d_Di, int ne, cudaStream_t st) {
@@ -1521,29 +1658,30 @@ void CholGPU::factor(const double* d_w2, const double* d_Di, int ne, cudaStream_
 }
 
 void CholGPU::solve_launches(double* d_x, cudaStream_t st, const int* mesh_on, int hold) {
-    WRAPD_CUDA(cudaMemcpyAsync(d_T_, d_x, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    WRAPD_CUDA(cudaMemsetAsync(d_qctl_, 0, qctl_words_ * sizeof(unsigned), st));
-    unsigned* bands = d_qctl_ + 2 + 2 * (size_t)nfronts;
+    const int hold_col = hold < 0 ? -1 : h_desc_[hold].first;
     if (nqf_ > 0) {
-        const SolveQueue Q{d_qf_, nqf_, d_qctl_, d_qctl_ + 2, d_qnb_, d_status, hold};
-        k_fwd_queue<<<std::min(qgrid_f_, nqf_), 32 * FWD_WARPS, 0, st>>>(d_T_, d_Z_, d_U_, d_inv_, d_Y_, d_desc_, Q, d_P_, bands,
-                                                           mesh_on);
+        const SolveQueue Q{d_qf_, nqf_, d_heads_, d_heads_ + 1, d_status, hold_col, solve_gate_};
+        k_fwd_queue<<<std::min(qgrid_f_, nqf_), SOLVE_THREADS, solve_smem(FRING), st>>>(d_x, d_Z_, d_Xp_, d_U_, d_inv_, d_Y_, Q,
+                                                                               d_P_, mesh_on);
         WRAPD_LAUNCH_CHECK();
     }
     if (nqb_ > 0) {
-        const SolveQueue Q{d_qb_, nqb_, d_qctl_ + 1, d_qctl_ + 2 + nfronts, d_qnb_ + nfronts, d_status, hold};
-        k_bwd_queue<<<std::min(qgrid_b_, nqb_), 256, 0, st>>>(d_x, d_Z_, d_Y_, d_rows_, d_desc_, Q, d_P_,
-                                                           bands + qbands_f_, mesh_on);
+        const SolveQueue Q{d_qb_, nqb_, d_heads_ + 1, d_heads_, d_status, hold_col, solve_gate_};
+        bwd_fn_<<<std::min(qgrid_b_, nqb_), SOLVE_THREADS, bwd_smem_, st>>>(d_x, d_Z_, d_Xp_, d_U_, d_Y_, d_rows_, Q,
+                                                                               d_P_, mesh_on);
         WRAPD_LAUNCH_CHECK();
     }
 }
 
 void CholGPU::solve_holding(double* d_x, int hold, cudaStream_t st) {
     if (hold < 0 || hold >= nfronts) throw CudaError(WRAPD_E_INPUT, "front index out of range");
+    if (solve_stale_) fill_unset(st);
     solve_launches(d_x, st, nullptr, hold);
+    solve_stale_ = true;
 }
 
 void CholGPU::solve(double* d_x, cudaStream_t st, const int* mesh_on) {
+    if (solve_stale_) fill_unset(st);
     if (!use_graphs) { solve_launches(d_x, st, mesh_on); return; }
     if (!solve_graph_ || solve_graph_x_ != d_x || solve_graph_mask_ != mesh_on) {
         if (solve_graph_) { cudaGraphExecDestroy(solve_graph_); solve_graph_ = nullptr; }

@@ -37,31 +37,47 @@ struct FrontDesc {
 // of panel columns.  kind 0: C is F[r0:r1, c0:c1] of the front (lower part
 // where rows and columns overlap), A = F[r0:r1, k0:k1], B' = F[c0:c1, k0:k1];
 // kind 1: C is Y[r0:r1, c0:c1], A = F[r0:r1, k0:k1], B'(j, t) = Y[k0 + t, c0 + j].
-// A solve work item: a 64-wide band starting at b0 (rows forward, columns
-// backward) times the chunk [lo, hi) of the other dimension.  The band's items
-// are contiguous, starting at `first`, `nchunk` of them; `band` indexes the
-// arrival counter.
-struct SolveItem {
-    int front, b0, lo, hi, nchunk, first, band;
-};
-
-// The items of every level of one direction as one work list (see k_fwd_queue):
-// head is the next item to take; done[f] counts the bands of front f written,
-// complete at nbands[f]; status receives WRAPD_E_TIMEOUT from a wait that gave
-// up; hold is a front whose completion is never counted (-1: none), which
-// makes the waits on it run out (the test of that path).
-struct SolveQueue {
-    const SolveItem* items;
-    int n;
-    unsigned* head;
-    unsigned* done;
-    const unsigned* nbands;
-    int* status;
-    int hold;
-};
-
 struct GemmJob {
     int front, kind, r0, r1, c0, c1, k0, k1;
+};
+
+// A solve work item on the host: a 64-wide band starting at b0 (rows forward,
+// columns backward) times the chunk [lo, hi) of the other dimension.  The
+// band's items are contiguous, starting at `first`, `nchunk` of them.
+struct SolveItem {
+    int front, b0, lo, hi, nchunk, first;
+};
+
+// The same item with what the kernels need of its front, one record a CTA
+// copies to shared memory (see k_fwd_queue).
+struct __align__(16) SolveWork {
+    int64_t m_off;        // [Y; W] offset of the item's first value: row b0 column lo (forward), row lo column b0 (backward)
+    int64_t aux;          // forward: the front's first row in inv; backward: its first entry in rows
+    int ldy, k, R, col;   // leading dimension, columns, rows (k + r) and first column of the front
+    int b0, lo, hi, nchunk;
+    int first;            // queue index of the band's first item
+    int gate0, gate1;     // rows of U (forward) or x (backward) polled first, -1: none
+    int mesh;
+    int u_row;            // the front's first row in U
+    int leaf;             // no children
+    int w;                // the band's width
+    int pad;
+};
+static_assert(sizeof(SolveWork) == 80, "copied as five 16-byte words");
+
+// The items of every level of one direction as one work list (see k_fwd_queue):
+// head is the next item to take, other_head the other direction's head, which
+// the launch zeroes; status receives WRAPD_E_TIMEOUT from a wait that gave up;
+// hold is the first column of a front whose results are not handed on (-1:
+// none), which makes the waits for them run out (the test of that path).
+struct SolveQueue {
+    const SolveWork* items;
+    int n;
+    unsigned* head;
+    unsigned* other_head;
+    int* status;
+    int hold;
+    bool gate;      // items wait behind one thread's poll first
 };
 
 struct JobList {
@@ -114,6 +130,9 @@ public:
     // its diagonal block inside the tile launch) and keeps the fastest.  Runs
     // real factorizations of the current weights; call before the first factor.
     void autotune(const double* d_w2, const double* d_Di, int ne, cudaStream_t st);
+    // After a launch that failed (a non-zero *d_status): the next solve first
+    // refills the buffers its items hand values over in.
+    void reset_solve() { solve_stale_ = true; }
     // [fused panel-step limit, levels, forward chunk per level..., backward chunk per level...]
     std::vector<int> tuning() const;
 
@@ -144,11 +163,7 @@ private:
         // column chunk) and backward (64-column band, row chunk)
         struct SolveCand {
             int sch;
-            SolveItem* fwd;
-            int nfwd;
-            SolveItem* bwd;
-            int nbwd;
-            std::vector<SolveItem> hfwd, hbwd;   // host copies, for the work queues
+            std::vector<SolveItem> fwd, bwd;
         };
         std::vector<SolveCand> cand;
         int cfwd = 0, cbwd = 0;          // the candidates in use
@@ -157,7 +172,8 @@ private:
     FrontDesc* d_desc_ = nullptr;
     int* d_rows_ = nullptr;
     int* d_rel_ = nullptr;
-    int64_t* d_inv_ = nullptr;   // per front row: the (up to 2) children's update-vector entries that add into it
+    int* d_inv_ = nullptr;       // per front row: the (up to 2) rows of U that add into it, or -1
+    std::vector<int> h_inv_, h_rows_;
     int64_t* d_Apos_ = nullptr;
     int* d_Aptr_ = nullptr;
     int* d_Acon_ = nullptr;
@@ -165,12 +181,11 @@ private:
     double* d_F_ = nullptr;
     double* d_Y_ = nullptr;
     double* d_U_ = nullptr;      // solve update vectors
-    double* d_T_ = nullptr;      // solve: copy of the right-hand side (n x 3)
+    double* d_Xp_ = nullptr;     // solve: the solution as it is handed down the tree (n x 3)
     double* d_Z_ = nullptr;      // solve: forward result (n x 3)
     double* d_P_ = nullptr;      // solve: per-item partial sums (64 x 3 per item)
-    unsigned* d_cnt_ = nullptr;  // solve: per-band arrival counters (zero between launches)
     int64_t solve_parts_ = 0;
-    int solve_bands_ = 0;
+    bool solve_stale_ = true;    // U, Xp, P and the heads are to be refilled before the next solve
     int64_t f_pool_ = 0, y_pool_ = 0, u_pool_ = 0;
     cudaGraphExec_t factor_graph_ = nullptr;
     cudaGraphExec_t solve_graph_ = nullptr;
@@ -182,14 +197,17 @@ private:
     void solve_launches(double* d_x, cudaStream_t st, const int* mesh_on, int hold = -1);
     // the work queues of the chosen per-level candidates (after build and autotune)
     void build_queues(cudaStream_t st);
-    SolveItem* d_qf_ = nullptr;   // forward items, leaves first (capacity: the longest candidates)
-    SolveItem* d_qb_ = nullptr;   // backward items, root first
+    void fill_unset(cudaStream_t st);
+    void release(void* p);
+    SolveWork* d_qf_ = nullptr;   // forward items, leaves first
+    SolveWork* d_qb_ = nullptr;   // backward items, root first
     int nqf_ = 0, nqb_ = 0;
-    unsigned* d_qnb_ = nullptr;   // bands per front: forward [0, nfronts), backward [nfronts, 2 nfronts)
-    unsigned* d_qctl_ = nullptr;  // zeroed per solve: 2 heads, done counters (2 nfronts), band counters
-    size_t qctl_words_ = 0;
-    int qbands_f_ = 0, qbands_b_ = 0;   // band counters: forward, then backward
+    unsigned* d_heads_ = nullptr; // the forward and the backward queue's head
     int64_t qcap_f_ = 0, qcap_b_ = 0;   // item capacity of d_qf_, d_qb_
+    bool solve_gate_ = false;
+    int bwd_smem_ = 0;
+    void (*bwd_fn_)(double*, const double*, double*, double*, const double*, const int*, SolveQueue, double*,
+                    const int*) = nullptr;   // the backward kernel's instance for this system's size
     int qgrid_f_ = 0, qgrid_b_ = 0;   // persistent CTAs per queue launch (resident at once)
     std::vector<void*> allocs_;
     std::vector<FrontDesc> h_desc_;

@@ -826,6 +826,7 @@ void SolverGPU::sync_read() {
     if (*h_status_ != 0) {
         const int status = *h_status_;
         *h_status_ = 0;
+        chol.reset_solve();
         WRAPD_CUDA(cudaMemsetAsync(chol.d_status, 0, sizeof(int), st_));
         throw_status(status);
     }
@@ -837,6 +838,7 @@ void SolverGPU::check_status() {
     WRAPD_CUDA(cudaStreamSynchronize(st_));
     ctl_pending_ = false;
     if (status != 0) {
+        chol.reset_solve();
         WRAPD_CUDA(cudaMemsetAsync(chol.d_status, 0, sizeof(int), st_));
         throw_status(status);
     }
