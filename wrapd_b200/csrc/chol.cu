@@ -1,8 +1,7 @@
 // GPU multifrontal Cholesky and 3-RHS solve; see chol.cuh.
 //
 // Factorization, per level of the assembly tree (leaves first):
-//   extend-add   children's update matrices into the fronts (one launch per
-//                child slot, so two children never write one entry at once);
+//   assemble     the fronts' entries from A and the children's update matrices;
 //   then per panel of NB = 32 columns (right-looking partial Cholesky):
 //   panel        every CTA factors the NB x NB diagonal block in registers
 //                (one warp) and forms its inverse Li (also stored as a diagonal
@@ -16,7 +15,7 @@
 //                K = OB (FP64 DMMA tiles, K-looped), so the large trailing
 //                matrix is read and written once per OB columns, not per panel;
 //   then         W = L_rs Y for the level's fronts (FP64 DMMA, K-looped).
-// A is assembled once per factorization straight into the zeroed F pool.
+// A's values are computed once per factorization, ahead of the levels.
 //
 // Every tile product is mma.sync.m8n8k4 f64 (the FP64 tensor-core path of
 // sm_100a; tcgen05 has no f64 kind).
@@ -234,7 +233,8 @@ __device__ __forceinline__ void gemm_pipelined(const double* A0, int64_t lda, in
 }
 
 // ---- assembly ----------------------------------------------------------------
-__global__ void k_assemble_A(double* __restrict__ F, const int64_t* __restrict__ pos, const int* __restrict__ ptr,
+// The values of A's lower-triangle entries, by front column (see build).
+__global__ void k_assemble_A(double* __restrict__ Aval, const int* __restrict__ slot, const int* __restrict__ ptr,
                              const int* __restrict__ con, int nA, const double* __restrict__ w2,
                              const double* __restrict__ Di, int ne) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -248,47 +248,100 @@ __global__ void k_assemble_A(double* __restrict__ F, const int64_t* __restrict__
         for (int r = 0; r < 3; ++r) d += Di[(int64_t)(r + 3 * a) * ne + e] * Di[(int64_t)(r + 3 * b) * ne + e];
         v += w2[e] * d;
     }
-    F[pos[t]] = v;
+    Aval[slot[t]] = v;
 }
 
-__global__ void k_y_identity(double* __restrict__ Y, const FrontDesc* __restrict__ desc, int nfronts) {
-    const int f = blockIdx.x;
-    if (f >= nfronts) return;
-    const FrontDesc d = desc[f];
-    for (int i = threadIdx.x; i < d.k; i += blockDim.x) Y[d.y_off + i + (int64_t)i * d.ldy] = 1.0;
+// The front column of entry t of A (at F-pool offset pos[t]): counted, or, with the
+// columns' first places ptr, given the next place of its column.
+__global__ void k_A_places(int nA, const int64_t* __restrict__ pos, const FrontDesc* __restrict__ desc, int nfronts,
+                           const int* __restrict__ ptr, int* cnt, int* __restrict__ slot, int* __restrict__ row) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nA) return;
+    int lo = 0, hi = nfronts;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (desc[mid].f_off <= pos[t]) lo = mid; else hi = mid;
+    }
+    const int64_t o = pos[t] - desc[lo].f_off;
+    const int ld = desc[lo].ld, col = desc[lo].first + static_cast<int>(o / ld);
+    const int k = atomicAdd(cnt + col, 1);
+    if (!ptr) return;
+    slot[t] = ptr[col] + k;
+    row[ptr[col] + k] = static_cast<int>(o % ld);
 }
 
-// children slot `slot` of each front in the list: F_s[rel[i], rel[j]] += U_c[i, j], i >= j
-__global__ void k_extend_add(double* __restrict__ F, const FrontDesc* __restrict__ desc, const int* __restrict__ rel,
-                             WorkList wl, int slot) {
+// The k x k part of every front's Y block: the identity (a warp per column).
+__global__ void __launch_bounds__(32 * COLS_PER_CTA) k_y_identity(double* __restrict__ Y, const FrontDesc* __restrict__ desc,
+                                                                  WorkList wl) {
     const int item = find_item(wl.d_prefix, wl.n, blockIdx.x);
-    const int s = wl.d_fronts[item];
-    const FrontDesc ds = desc[s];
-    const int c = slot == 0 ? ds.child0 : ds.child1;
-    const FrontDesc dc = desc[c];
+    const FrontDesc d = desc[wl.d_fronts[item]];
+    const int j = (blockIdx.x - wl.d_prefix[item]) * COLS_PER_CTA + (threadIdx.x >> 5);
+    if (j >= d.k) return;
+    double* Yj = Y + d.y_off + (int64_t)j * d.ldy;
+    for (int i = threadIdx.x & 31; i < d.k; i += 32) Yj[i] = i == j ? 1.0 : 0.0;
+}
+
+// The fronts of a level: F(i, j), i >= j, = A(i, j) + U_c0(., .) + U_c1(., .), the
+// entries of A (front columns only) and of the children's update matrices that
+// land there, added in that order; zeros elsewhere.  A warp writes a column, so
+// the front is written once and nothing is read but the children's update
+// matrices and the row map, which a CTA's eight columns share in L1: 8 bytes
+// per front entry and 8 per child entry.  (The form before zeroed whole squares
+// and added each child in place, 8 bytes per square entry and 24 per child
+// entry: memset and extend-add took 1.72 ms of a factorization of the 32x32x128
+// bar and 14.6 ms on the 64x64x160 one, this takes 0.70 and 5.4.)  The strict
+// upper triangle is never read; the padding row is, into itself alone, and is
+// written as zero.
+__global__ void __launch_bounds__(32 * COLS_PER_CTA) k_assemble_front(double* F, const FrontDesc* __restrict__ desc,
+                                                                      const int* __restrict__ inv,
+                                                                      const double* __restrict__ Aval,
+                                                                      const int* __restrict__ Acol,
+                                                                      const int* __restrict__ Arow, WorkList wl) {
+    const int item = find_item(wl.d_prefix, wl.n, blockIdx.x);
+    const FrontDesc d = desc[wl.d_fronts[item]];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = (blockIdx.x - wl.d_prefix[item]) * COLS_PER_CTA + warp;
-    if (j >= dc.r) return;
-    const int* rc = rel + dc.rel_off;
-    const double* Uc = F + dc.f_off + dc.k + (int64_t)(dc.k + j) * dc.ld;
-    double* Fs = F + ds.f_off + (int64_t)rc[j] * ds.ld;
-    // Uc and Fs live in one pool, so the loads are batched by hand ahead of the
-    // stores (rel maps a column's rows to distinct parent rows)
-    constexpr int U = 4;
-    for (int i0 = j + lane; i0 < dc.r; i0 += 32 * U) {
-        double u[U], f[U];
-        int ri[U];
+    const int R = d.k + d.r;
+    if (j >= R) return;
+    const int2* iv = reinterpret_cast<const int2*>(inv + d.inv_off);
+    double* Fj = F + d.f_off + (int64_t)j * d.ld;
+    // the children's update columns landing on column j (null: none), indexed by row of U
+    const double *C0 = nullptr, *C1 = nullptr;
+    const int2 ij = iv[j];
+    if (ij.x >= 0) {
+        const FrontDesc& c = desc[d.child0];
+        const int u0 = static_cast<int>(c.u_off / 3);
+        C0 = F + c.f_off + c.k + (int64_t)(c.k + ij.x - u0) * c.ld - u0;
+    }
+    if (ij.y >= 0) {
+        const FrontDesc& c = desc[d.child1];
+        const int u0 = static_cast<int>(c.u_off / 3);
+        C1 = F + c.f_off + c.k + (int64_t)(c.k + ij.y - u0) * c.ld - u0;
+    }
+    constexpr int U = 4;   // rows per lane whose reads go out together
+    for (int i0 = j + lane; i0 < d.ld; i0 += 32 * U) {
+        double c0[U], c1[U];
 #pragma unroll
         for (int q = 0; q < U; ++q) {
             const int i = i0 + 32 * q;
-            ri[q] = i < dc.r ? rc[i] : 0;
-            u[q] = i < dc.r ? Uc[i] : 0.0;
+            const int2 m = (i < R && (C0 || C1)) ? iv[i] : make_int2(-1, -1);
+            c0[q] = (C0 && m.x >= 0) ? C0[m.x] : 0.0;
+            c1[q] = (C1 && m.y >= 0) ? C1[m.y] : 0.0;
         }
 #pragma unroll
-        for (int q = 0; q < U; ++q) f[q] = (i0 + 32 * q < dc.r) ? Fs[ri[q]] : 0.0;
-#pragma unroll
         for (int q = 0; q < U; ++q)
-            if (i0 + 32 * q < dc.r) Fs[ri[q]] = f[q] + u[q];
+            if (i0 + 32 * q < d.ld) Fj[i0 + 32 * q] = c0[q] + c1[q];
+    }
+    if (j >= d.k) return;
+    __syncwarp();   // the column's entries of A over what the loop wrote there
+    const int t1 = Acol[d.first + j + 1];
+    for (int t = Acol[d.first + j] + lane; t < t1; t += 32) {
+        const int i = Arow[t];
+        const int2 m = iv[i];
+        double v = Aval[t];
+        if (C0 && m.x >= 0) v += C0[m.x];
+        if (C1 && m.y >= 0) v += C1[m.y];
+        Fj[i] = v;
     }
 }
 
@@ -1198,9 +1251,30 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
     h_rows_ = rows;
     d_desc_ = upload(h_desc_, st);
     d_rows_ = upload(rows, st);
-    d_rel_ = upload(S.relmap, st);
+    // A's entries by front column: entry t's place, and each place's row in the
+    // front (a counting sort over the columns; the order within a column, which
+    // nothing depends on, is left to the atomics)
     nA_ = static_cast<int>(A_pos.size());
-    d_Apos_ = upload(A_pos, st);
+    {
+        int64_t* pos = upload(A_pos, st);
+        int* cnt = upload(std::vector<int>(n, 0), st);
+        d_Aslot_ = upload(std::vector<int>(nA_), st);
+        d_Arow_ = upload(std::vector<int>(nA_), st);
+        std::vector<int> ptr(n + 1, 0);
+        if (nA_ > 0) k_A_places<<<ceil_div(nA_, 256), 256, 0, st>>>(nA_, pos, d_desc_, nfronts, nullptr, cnt, nullptr, nullptr);
+        WRAPD_LAUNCH_CHECK();
+        WRAPD_CUDA(cudaMemcpyAsync(ptr.data() + 1, cnt, n * sizeof(int), cudaMemcpyDeviceToHost, st));
+        WRAPD_CUDA(cudaMemsetAsync(cnt, 0, n * sizeof(int), st));
+        WRAPD_CUDA(cudaStreamSynchronize(st));
+        for (int c = 0; c < n; ++c) ptr[c + 1] += ptr[c];
+        d_Acol_ = upload(ptr, st);
+        if (nA_ > 0) k_A_places<<<ceil_div(nA_, 256), 256, 0, st>>>(nA_, pos, d_desc_, nfronts, d_Acol_, cnt, d_Aslot_, d_Arow_);
+        WRAPD_LAUNCH_CHECK();
+        WRAPD_CUDA(cudaStreamSynchronize(st));
+        release(pos);
+        release(cnt);
+        device_bytes -= A_pos.size() * sizeof(int64_t) + n * sizeof(int);
+    }
     d_Aptr_ = upload(A_ptr, st);
     d_Acon_ = upload(A_contrib, st);
     f_pool_ = S.f_pool; y_pool_ = S.y_pool; u_pool_ = S.u_pool;
@@ -1214,8 +1288,11 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
         device_bytes += std::max<size_t>(1, count) * sizeof(double);
         return p;
     };
+    d_Aval_ = dalloc(nA_);
     d_F_ = dalloc(f_pool_);
     d_Y_ = dalloc(y_pool_);
+    // the padding rows of [Y; W] stay zero; a factorization writes all the rest
+    WRAPD_CUDA(cudaMemsetAsync(d_Y_, 0, y_pool_ * sizeof(double), st));
     d_U_ = dalloc(u_pool_);
     d_Xp_ = dalloc(3 * (size_t)n);
     d_Z_ = dalloc(3 * (size_t)n);
@@ -1225,6 +1302,11 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
     d_status = st_ptr;
     WRAPD_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
 
+    {
+        std::vector<int> all(nfronts), cnt(nfronts);
+        for (int f = 0; f < nfronts; ++f) { all[f] = f; cnt[f] = ceil_div(h_desc_[f].k, COLS_PER_CTA); }
+        y_cols_ = make_list(all, cnt, st);
+    }
     levels_.assign(nlevels, Level());
     fused_ctas_ = kFusedPanelCtas;
     for (int l = 0; l < nlevels; ++l) {
@@ -1235,14 +1317,9 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
         const auto& fs = L.fronts_sorted;
         L.kmax = fs.empty() ? 0 : h_desc_[fs[0]].k;
         std::vector<int> cnt(fs.size());
-        for (int slot = 0; slot < 2; ++slot) {
-            for (size_t i = 0; i < fs.size(); ++i) {
-                const FrontDesc& d = h_desc_[fs[i]];
-                const int c = slot == 0 ? d.child0 : d.child1;
-                cnt[i] = c < 0 ? 0 : ceil_div(h_desc_[c].r, COLS_PER_CTA);
-            }
-            L.extend.push_back(make_list(fs, cnt, st));
-        }
+        for (size_t i = 0; i < fs.size(); ++i)
+            cnt[i] = ceil_div(h_desc_[fs[i]].k + h_desc_[fs[i]].r, COLS_PER_CTA);
+        L.assemble = make_list(fs, cnt, st);
         const int steps = ceil_div(L.kmax, NB);
         for (int p = 0; p < steps; ++p) {
             std::vector<int> act, ct, nP;
@@ -1505,10 +1582,10 @@ void CholGPU::fill_unset(cudaStream_t st) {
 }
 
 void CholGPU::count_launches() {
-    launches_factor = 4;   // memsets + assembly + identity
+    launches_factor = 2;   // A's values + identity
     launches_solve = 2;    // the two queue launches
     for (const Level& L : levels_) {
-        for (const WorkList& e : L.extend) launches_factor += e.total ? 1 : 0;
+        launches_factor += L.assemble.total ? 1 : 0;
         for (size_t p = 0; p < L.trsm.size(); ++p) {
             if (L.trsm[p].total > fused_ctas_) launches_factor += L.diag[p].n ? 1 : 0;
             launches_factor += (L.trsm[p].total ? 1 : 0) + (L.update[p].total ? 1 : 0);
@@ -1594,21 +1671,19 @@ void CholGPU::autotune(const double* d_w2, const double* d_Di, int ne, cudaStrea
 }
 
 void CholGPU::factor_launches(const double* d_w2, const double* d_Di, int ne, cudaStream_t st) {
-    WRAPD_CUDA(cudaMemsetAsync(d_F_, 0, f_pool_ * sizeof(double), st));
-    WRAPD_CUDA(cudaMemsetAsync(d_Y_, 0, y_pool_ * sizeof(double), st));
     if (nA_ > 0) {
-        k_assemble_A<<<ceil_div(nA_, 256), 256, 0, st>>>(d_F_, d_Apos_, d_Aptr_, d_Acon_, nA_, d_w2, d_Di, ne);
+        k_assemble_A<<<ceil_div(nA_, 256), 256, 0, st>>>(d_Aval_, d_Aslot_, d_Aptr_, d_Acon_, nA_, d_w2, d_Di, ne);
         WRAPD_LAUNCH_CHECK();
     }
-    k_y_identity<<<nfronts, 128, 0, st>>>(d_Y_, d_desc_, nfronts);
+    k_y_identity<<<y_cols_.total, 32 * COLS_PER_CTA, 0, st>>>(d_Y_, d_desc_, y_cols_);
     WRAPD_LAUNCH_CHECK();
     for (int l = 0; l < nlevels; ++l) {
         Level& L = levels_[l];
-        for (int slot = 0; slot < 2; ++slot)
-            if (L.extend[slot].total) {
-                k_extend_add<<<L.extend[slot].total, 32 * COLS_PER_CTA, 0, st>>>(d_F_, d_desc_, d_rel_, L.extend[slot], slot);
-                WRAPD_LAUNCH_CHECK();
-            }
+        if (L.assemble.total) {
+            k_assemble_front<<<L.assemble.total, 32 * COLS_PER_CTA, 0, st>>>(d_F_, d_desc_, d_inv_, d_Aval_, d_Acol_,
+                                                                             d_Arow_, L.assemble);
+            WRAPD_LAUNCH_CHECK();
+        }
         for (size_t p = 0; p < L.trsm.size(); ++p) {
             if (L.trsm[p].total <= fused_ctas_) {
                 if (L.trsm[p].total) {

@@ -153,7 +153,7 @@ private:
     struct Level {
         std::vector<int> fronts_sorted;   // by k descending
         int kmax = 0;
-        std::vector<WorkList> extend;    // per child slot: CTAs over child columns
+        WorkList assemble;               // CTAs over front columns
         std::vector<WorkList> diag;      // per panel step (steps not fused): one CTA per front
         std::vector<WorkList> trsm;      // per panel step: panel row tiles + Y row-block tiles
         std::vector<JobList> update;     // per panel step: blocked trailing-update jobs (F and Y)
@@ -171,10 +171,13 @@ private:
     std::vector<Level> levels_;
     FrontDesc* d_desc_ = nullptr;
     int* d_rows_ = nullptr;
-    int* d_rel_ = nullptr;
     int* d_inv_ = nullptr;       // per front row: the (up to 2) rows of U that add into it, or -1
     std::vector<int> h_inv_, h_rows_;
-    int64_t* d_Apos_ = nullptr;
+    double* d_Aval_ = nullptr;   // A's lower-triangle entries by front column
+    int* d_Aslot_ = nullptr;     // entry -> place in d_Aval_
+    int* d_Acol_ = nullptr;      // n + 1: the places of each column
+    int* d_Arow_ = nullptr;      // place -> row in the column's front
+    WorkList y_cols_;            // CTAs over every front's columns
     int* d_Aptr_ = nullptr;
     int* d_Acon_ = nullptr;
     int nA_ = 0;
