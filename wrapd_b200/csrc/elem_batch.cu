@@ -17,7 +17,8 @@ __global__ void k_svd_batch(int n, const double* __restrict__ F, double* __restr
     T f[9], s[3], u[9], v[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) f[i] = T(F[9 * (size_t)e + i]);
-    svd3(f, s, u, v);
+    if constexpr (sizeof(T) == sizeof(double)) svd3_fast(f, s, u, v);
+    else svd3(f, s, u, v);
 #pragma unroll
     for (int i = 0; i < 3; ++i) sig[3 * (size_t)e + i] = s[i];
 #pragma unroll
@@ -85,7 +86,7 @@ __global__ void k_hess_batch(int n, double mu, double lambda, const double* __re
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     const double x[3] = {s[3 * (size_t)e], s[3 * (size_t)e + 1], s[3 * (size_t)e + 2]};
-    out[e] = NH<double>{mu, lambda}.hess_lmax(x);
+    out[e] = NH<double>{mu, lambda}.hess_lmax<true>(x);
 }
 
 struct DevBuf {

@@ -89,7 +89,10 @@ __device__ __forceinline__ double elastic_energy(const Material& m, const double
 // in uv (U then V, 9 SoA components each); 2 = x is the point of the last
 // UV = 1 launch, so F's SVD is that launch's: sig, U, V and symF are read
 // back instead of recomputed (the same values, so the same results).
-template <bool SEG, int UV = 0>
+// FAST: the SVD's rotations from rsqrt (svd3_fast).  Mixed precision keeps the
+// general form's operations: there the FP32 local step turns a last bit of the
+// gradient into 1e-8 of the positions within twenty iterations.
+template <bool FAST, bool SEG, int UV = 0>
 static __global__ void __launch_bounds__(256, (SEG || UV != 0) ? 2 : 0) k_grad(ElemView E, Tiles T, const int* on, const double* __restrict__ x,
                                               const double* __restrict__ xfix, Material mat0, int write_gel,
                                               double* partials, unsigned* counters, double* out, int stride,
@@ -113,7 +116,7 @@ static __global__ void __launch_bounds__(256, (SEG || UV != 0) ? 2 : 0) k_grad(E
             for (int i = 0; i < 3; ++i) s[i] = E.sig[(size_t)i * E.ne + e];
             load9(E.symF, E.ne, e, S);
         } else {
-            svd3(F, s, Us, Vs);
+            svd3_of<FAST>(F, s, Us, Vs);
 #pragma unroll
             for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -318,7 +321,8 @@ __global__ void __launch_bounds__(512, 1) k_local(ElemView E, Tiles T, const int
                 bef += d * d;
             }
         red[0] += 0.5 * w2 * bef;
-        svd3(Sin, sg, Ue, Ve);
+        if constexpr (sizeof(C) == sizeof(double)) svd3_fast(Sin, sg, Ue, Ve);
+        else svd3(Sin, sg, Ue, Ve);
     }
     Prox<C> P;
     P.nh.mu = C(mat.mu);
@@ -347,12 +351,14 @@ __global__ void __launch_bounds__(512, 1) k_local(ElemView E, Tiles T, const int
     }
     if (valid) {
         int iters;
+        LsPoint<C> end;   // the log term at the solution, where the prox leaves it
+        end.ok = false;
         if constexpr (sizeof(C) == sizeof(double)) {
             if (NET || prox_mode == 1) {
                 iters = prox_newton(P, xs, prox_iters, C(1e-12));
             } else {
                 extern __shared__ double prox_hist[];   // 48 x blockDim doubles
-                iters = prox_lbfgs(P, xs, prox_iters, ProxHistory<double>{prox_hist + threadIdx.x, (int)blockDim.x});
+                iters = prox_lbfgs(P, xs, prox_iters, ProxHistory<double>{prox_hist + threadIdx.x, (int)blockDim.x}, &end);
                 if (iters < 0) iters = prox_iters;
             }
         } else {
@@ -386,7 +392,10 @@ __global__ void __launch_bounds__(512, 1) k_local(ElemView E, Tiles T, const int
             for (int c = 0; c < 3; ++c)
                 M3(Soc, r, c) = M3(Ve, r, 0) * xs[0] * M3(Ue, c, 0) + M3(Ve, r, 1) * xs[1] * M3(Ue, c, 1) +
                                 M3(Ve, r, 2) * xs[2] * M3(Ue, c, 2);
-        red[2] += vol * NH<double>{mat.mu, mat.lambda}.psi_plain(xo[0], xo[1], xo[2]);
+        if (end.ok)
+            red[2] += vol * NH<double>{mat.mu, mat.lambda}.psi_log(xo[0], xo[1], xo[2], double(end.lf));
+        else
+            red[2] += vol * NH<double>{mat.mu, mat.lambda}.psi_plain(xo[0], xo[1], xo[2]);
         double aft = 0.0, Zm[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
@@ -402,7 +411,7 @@ __global__ void __launch_bounds__(512, 1) k_local(ElemView E, Tiles T, const int
         if (cand_mode == CAND_REST) {
             E.w2c[e] = vol * mat.wr;
         } else if (cand_mode == CAND_HESSIAN) {
-            const double lm = NH<double>{mat.mu, mat.lambda}.hess_lmax(xo);
+            const double lm = NH<double>{mat.mu, mat.lambda}.template hess_lmax<sizeof(C) == sizeof(double)>(xo);
             double c = lm;
             if (lm < mat.wmin) c = mat.wmin;
             if (lm > mat.wmax) c = mat.wmax;
@@ -415,6 +424,7 @@ __global__ void __launch_bounds__(512, 1) k_local(ElemView E, Tiles T, const int
 // initialize_dual_vars (src/TetElements.cpp:145-166): Z = (V diag(s) V^T)^T of
 // F(X) with all four slots read from X, U = 0; then polar_potential_energy
 // (src/TetElements.cpp:638-675) of the new Z.  out[0] = that energy.
+template <bool FAST>
 static __global__ void __launch_bounds__(128) k_init_dual(ElemView E, Tiles T, const int* on, const double* __restrict__ x,
                                                    const double* __restrict__ xfix, Material mat0,
                                                    double* partials, unsigned* counters, double* out, int stride) {
@@ -429,7 +439,7 @@ static __global__ void __launch_bounds__(128) k_init_dual(ElemView E, Tiles T, c
         double F[9], s[3], Us[9], Vs[9], Zm[9], Zt[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) F[i] = double(Fd[i]);
-        svd3(F, s, Us, Vs);
+        svd3_of<FAST>(F, s, Us, Vs);
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -452,7 +462,7 @@ static __global__ void __launch_bounds__(128) k_init_dual(ElemView E, Tiles T, c
                 for (int c = 0; c < 3; ++c) { const double d = M3(Zm, r, c) - (r == c ? 1.0 : 0.0); n2 += d * d; }
             red[0] = 0.5 * E.vol[e] * n2;
         } else {
-            svd3(Zt, s, Us, Vs);
+            svd3_of<FAST>(Zt, s, Us, Vs);
             red[0] = E.vol[e] * NH<double>{mat.mu, mat.lambda}.psi_plain(double(s[0]), double(s[1]), double(s[2]));
         }
     }
@@ -461,6 +471,7 @@ static __global__ void __launch_bounds__(128) k_init_dual(ElemView E, Tiles T, c
 
 // Candidate weights of midupdate_weights (src/TetElements.cpp:360-388): from
 // F(X) (from_x = 1) or from the cached singular values.
+template <bool FAST>
 static __global__ void __launch_bounds__(128) k_mid_candidates(ElemView E, Tiles T, const int* on,
                                                         const double* __restrict__ x, const double* __restrict__ xfix,
                                                         Material mat0, int from_x, int cand_mode) {
@@ -476,7 +487,7 @@ static __global__ void __launch_bounds__(128) k_mid_candidates(ElemView E, Tiles
         double F[9], st[3], Us[9], Vs[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) F[i] = double(Fd[i]);
-        svd3(F, st, Us, Vs);
+        svd3_of<FAST>(F, st, Us, Vs);
         s[0] = st[0]; s[1] = st[1]; s[2] = st[2];
     } else {
 #pragma unroll
@@ -484,7 +495,7 @@ static __global__ void __launch_bounds__(128) k_mid_candidates(ElemView E, Tiles
     }
     const double vol = E.vol[e];
     if (cand_mode == CAND_HESSIAN) {
-        const double lm = NH<double>{mat.mu, mat.lambda}.hess_lmax(s);
+        const double lm = NH<double>{mat.mu, mat.lambda}.template hess_lmax<FAST>(s);
         double c = lm;
         if (lm < mat.wmin) c = mat.wmin;
         if (lm > mat.wmax) c = mat.wmax;
@@ -1071,7 +1082,8 @@ __global__ void __launch_bounds__(128, 4) k_local_unaware(ElemView E, const doub
 #pragma unroll
             for (int c = 0; c < 3; ++c) M3(Fp, r, c) = C(F[r + 3 * c] + M3(Um, c, r));   // (F^T + U)^T
         C sg[3], Ue[9], Ve[9];
-        svd3(Fp, sg, Ue, Ve);
+        if constexpr (sizeof(C) == sizeof(double)) svd3_fast(Fp, sg, Ue, Ve);
+        else svd3(Fp, sg, Ue, Ve);
         if (mat.model == MODEL_ARAP) {
 #pragma unroll
             for (int r = 0; r < 3; ++r)
@@ -1132,7 +1144,7 @@ __global__ void __launch_bounds__(128, 4) k_local_unaware(ElemView E, const doub
             if (cand_mode == CAND_REST) {
                 E.w2c[e] = vol * mat.wr;
             } else if (cand_mode == CAND_HESSIAN) {
-                const double lm = NH<double>{mat.mu, mat.lambda}.hess_lmax(xo);
+                const double lm = NH<double>{mat.mu, mat.lambda}.template hess_lmax<sizeof(C) == sizeof(double)>(xo);
                 double cnd = lm;
                 if (lm < mat.wmin) cnd = mat.wmin;
                 if (lm > mat.wmax) cnd = mat.wmax;

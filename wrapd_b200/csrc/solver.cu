@@ -627,7 +627,7 @@ const Logs& SolverGPU::mesh_logs(int m) const {
 
 #define WRAPD_ELEM_LAUNCH(kernel, tiles, block, ...)                                        \
     do {                                                                                    \
-        kernel<<<(tiles).count, block, 0, st_>>>(view(), (tiles).view(), __VA_ARGS__);      \
+        (kernel)<<<(tiles).count, block, 0, st_>>>(view(), (tiles).view(), __VA_ARGS__);      \
         WRAPD_LAUNCH_CHECK();                                                               \
         kernel_launches++;                                                                  \
     } while (0)
@@ -641,25 +641,17 @@ const Logs& SolverGPU::mesh_logs(int m) const {
 // against 128; 3.9M bar: 5.09 -> 4.95 ms), in a batch too, so that a mesh's
 // sums are added in the same order as when it is solved alone.
 void SolverGPU::grad_at_x(bool write_gel, int mk) {
-    if (nm > 1) {
-        WRAPD_ELEM_LAUNCH(k_grad<true>, te256_, 256, mask(mk), d_x_, d_xfix_, mat_, write_gel ? 1 : 0, d_partials_,
-                          d_counters_, ds(S_GRAD), kScalStride);
-    } else if (d_uv_ && write_gel && cfg.rot_aware && !cfg.global_ls) {
-        if (uv_valid_)
-            k_grad<false, 2><<<te256_.count, 256, 0, st_>>>(view(), te256_.view(), mask(mk), d_x_, d_xfix_, mat_, 1,
-                                                             d_partials_, d_counters_, ds(S_GRAD), kScalStride, d_uv_);
-        else
-            k_grad<false, 1><<<te256_.count, 256, 0, st_>>>(view(), te256_.view(), mask(mk), d_x_, d_xfix_, mat_, 1,
-                                                             d_partials_, d_counters_, ds(S_GRAD), kScalStride, d_uv_);
-        WRAPD_LAUNCH_CHECK();
-        kernel_launches++;
-        uv_valid_ = true;
-        return;
-    } else {
-        WRAPD_ELEM_LAUNCH(k_grad<false>, te256_, 256, mask(mk), d_x_, d_xfix_, mat_, write_gel ? 1 : 0, d_partials_,
-                          d_counters_, ds(S_GRAD), kScalStride);
-    }
-    uv_valid_ = false;
+    const bool keep = nm == 1 && d_uv_ && write_gel && cfg.rot_aware && !cfg.global_ls;
+    // FP64 solves take the SVD's fast form, mixed precision the general one (see k_grad)
+    const auto fn = nm > 1 ? (fp32() ? k_grad<false, true, 0> : k_grad<true, true, 0>)
+                    : !keep ? (fp32() ? k_grad<false, false, 0> : k_grad<true, false, 0>)
+                    : uv_valid_ ? k_grad<false, false, 2>
+                                : (fp32() ? k_grad<false, false, 1> : k_grad<true, false, 1>);
+    fn<<<te256_.count, 256, 0, st_>>>(view(), te256_.view(), mask(mk), d_x_, d_xfix_, mat_, write_gel ? 1 : 0, d_partials_,
+                                      d_counters_, ds(S_GRAD), kScalStride, keep ? d_uv_ : nullptr);
+    WRAPD_LAUNCH_CHECK();
+    kernel_launches++;
+    uv_valid_ = keep;
 }
 
 void SolverGPU::gather(int mode, int mk, bool xerr, double* plain) {
@@ -767,7 +759,7 @@ void SolverGPU::set_prox_net(const float* blob) {
 }
 
 void SolverGPU::mid_candidates(bool from_x, int cand_mode) {
-    WRAPD_ELEM_LAUNCH(k_mid_candidates, te128_, 128, mask(MK_ALL), d_x_, d_xfix_, mat_, from_x ? 1 : 0, cand_mode);
+    WRAPD_ELEM_LAUNCH((fp32() ? k_mid_candidates<false> : k_mid_candidates<true>), te128_, 128, mask(MK_ALL), d_x_, d_xfix_, mat_, from_x ? 1 : 0, cand_mode);
 }
 
 void SolverGPU::apply_weights(int mk) {
@@ -930,7 +922,7 @@ void SolverGPU::begin_solve() {
     WRAPD_CUDA(cudaMemcpyAsync(d_x_, d_xinit_, 3 * (size_t)nf * sizeof(double), cudaMemcpyDeviceToDevice, st_));
     grad_at_x(false, MK_ALL);
     if (cfg.rot_aware) {
-        WRAPD_ELEM_LAUNCH(k_init_dual, te128_, 128, mask(MK_ALL), d_x_, d_xfix_, mat_, d_partials_, d_counters_,
+        WRAPD_ELEM_LAUNCH((fp32() ? k_init_dual<false> : k_init_dual<true>), te128_, 128, mask(MK_ALL), d_x_, d_xfix_, mat_, d_partials_, d_counters_,
                           ds(S_INIT), kScalStride);
     } else {
         k_init_dual_unaware<<<blocks_for(ne, 128), 128, 0, st_>>>(view(), d_x_, d_xfix_);
@@ -1002,8 +994,8 @@ double SolverGPU::line_search() {
         k_ls_trial<<<vb, 256, 0, st_>>>(n, trial, d_x_, step, alpha);
         WRAPD_LAUNCH_CHECK();
         kernel_launches++;
-        WRAPD_ELEM_LAUNCH(k_grad<false>, te256_, 256, mask(MK_ALL), trial, d_xfix_, mat_, 0, d_partials_,
-                          d_counters_, ds(S_LSV), kScalStride);   // one mesh (line search: single meshes only)
+        WRAPD_ELEM_LAUNCH((fp32() ? k_grad<false, false, 0> : k_grad<true, false, 0>), te256_, 256, mask(MK_ALL), trial, d_xfix_, mat_, 0, d_partials_,
+                          d_counters_, ds(S_LSV), kScalStride, nullptr);   // one mesh (line search: single meshes only)
         sync_read();
         const double fxa = hs(0, S_LSV);
         if (fxa <= fx0 + alpha * decrease * gtp) return alpha;
