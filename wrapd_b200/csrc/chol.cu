@@ -38,17 +38,25 @@ constexpr int GEMM_THREADS = 128;
 constexpr int kFusedPanelCtas = 4 * 148;   // panel steps up to one wave (4 CTAs per SM) run fused
 constexpr int COLS_PER_CTA = 8;    // solve / extend-add column groups (one warp each)
 
+// The list item that owns CTA b: the last i < n with prefix[i] <= b.  The lanes of a
+// warp look at 32 places at once, so a list of up to 32 items takes one round
+// trip to memory and one of 1024 two (a binary search takes five and ten, one
+// after the other, before a CTA can load anything).
 __device__ __forceinline__ int find_item(const int* prefix, int n, int b) {
-    int lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (prefix[mid] <= b) lo = mid; else hi = mid;
+    const int lane = threadIdx.x & 31;
+    int lo = 0, len = n;
+    while (len > 1) {
+        const int step = (len + 31) >> 5, o = lane * step;
+        const bool le = o < len && __ldg(prefix + lo + o) <= b;
+        const int j = 31 - __clz(__ballot_sync(0xffffffffu, le));
+        lo += j * step;
+        len = min(step, len - j * step);
     }
     return lo;
 }
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
 }
@@ -106,25 +114,28 @@ __device__ __forceinline__ void tile_store(double* C, int64_t crs, int64_t ccs, 
 }
 
 // ---- pipelined GEMM core ------------------------------------------------------
-// Operand tiles are staged by cp.async in one of two layouts, chosen by which
-// index is contiguous in global memory so that both the staging writes and the
-// DMMA fragment reads hit every shared-memory bank evenly:
-//   t-major S[t * TP + i] for sources with i contiguous (columns of F),
-//   i-major S[i * SLD + t] for sources with t contiguous (row blocks of Y).
-// Two stages: chunk c + 1 is in flight while chunk c is multiplied.
-constexpr int TP = TL + 8;            // t-major pitch: 8 mod 16 doubles
-#ifndef WRAPD_GEMM_KC
-#define WRAPD_GEMM_KC 16
-#endif
-constexpr int KC = WRAPD_GEMM_KC;     // K columns per staged chunk of the trailing-update GEMMs
-constexpr int GSLD = KC + 4;          // i-major pitch (KC + 4 = 4 mod 8 doubles: conflict-free fragment reads)
-constexpr int TILE_D = (KC * TP > TL * GSLD) ? KC * TP : TL * GSLD;   // doubles per staged operand tile
-static_assert(KC % 4 == 0 && KC <= NB, "chunks of whole DMMA k-steps");
-#ifndef WRAPD_GEMM_STAGES
-#define WRAPD_GEMM_STAGES 2
-#endif
-constexpr int GEMM_STAGES = WRAPD_GEMM_STAGES;   // cp.async pipeline depth of the trailing-update GEMMs
+// 64 x 64 tiles of FP64 DMMA, four CTAs of four warps per SM, K in chunks of KC
+// columns staged by cp.async, three stages, one barrier per chunk.  Operand tiles
+// are staged in one of two layouts, chosen by which index is contiguous in global
+// memory so that both the staging writes and the DMMA fragment reads (4 x 4 values
+// per half-warp) hit every shared-memory bank evenly:
+//   t-major S[t * TP + i] for sources with i contiguous (columns of F); a source
+//     that starts on an odd row is staged from the even row before it, shifted by
+//     one, so that its copies are 16 bytes wide too;
+//   i-major S[i * KC + (t ^ 4 (i % 4))] for sources with t contiguous (row blocks of Y).
+// The loop is bound by the DMMA pipe only if little else is issued: a thread's
+// copies differ from chunk to chunk by one pointer step, and the k-steps are
+// unrolled with constant shared-memory offsets, so a DMMA comes with about two other
+// instructions (twelve in the form before, which recomputed every copy's place and
+// ran two barriers a chunk).  Rate on the 64x64x160 bar's trailing updates and W
+// products: 27 -> 31 to 32.6 of the 37.1 TFLOP/s that the instruction reaches alone.
+// Every entry adds its products in ascending k in steps of four, whatever the chunks.
+constexpr int KC = 16;                // K columns per staged chunk
+constexpr int TP = TL + 4;            // t-major pitch (4 mod 16 doubles)
+constexpr int TILE_D = KC * TP;       // doubles per staged operand tile
+constexpr int GEMM_STAGES = 3;
 constexpr int GEMM_SMEM = GEMM_STAGES * 2 * TILE_D * (int)sizeof(double);   // stages x (A, B)
+static_assert(TL * KC <= TILE_D && KC == 16 && GEMM_THREADS == 128, "the staging maps below");
 
 __device__ __forceinline__ void cp_async8(double* s, const double* g, bool valid) {
     const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(s));
@@ -140,96 +151,125 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Element (i, t), i < rows, t < K, of a source with (TMAJOR) i contiguous:
-// base[i + t * ld], or t contiguous: base[i * ld + t]; zeros up to K4.
-// Where the source is 16-byte aligned and ld even (every front's F and Y
-// blocks have an even leading dimension; a job's row offset may still be odd),
-// element pairs move as one 16-byte copy: along i in the t-major layout, along
-// t in the i-major one.
+// One operand of a tile: element (i, t), i < rows, t < K, at base[i + t * ld]
+// (TMAJOR) or base[i * ld + t].  TMAJOR: thread copies row pair tid % 32 of columns
+// tid / 32 + 4 u; else: column pair tid % 8 of rows tid / 8 + 16 u.  ld is even, and
+// an i-major base even too.
 template <bool TMAJOR>
-__device__ __forceinline__ void stage_tile(double* S, const double* base, int64_t ld, int rows, int K, int K4) {
-    if ((reinterpret_cast<uintptr_t>(base) & 15) == 0 && (ld & 1) == 0) {
-        if constexpr (TMAJOR) {
-            const int total = (TL / 2) * K4;
-            for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-                const int i = 2 * (idx % (TL / 2)), t = idx / (TL / 2);
-                const int nbytes = (t < K && i < rows) ? (i + 1 < rows ? 16 : 8) : 0;
-                cp_async16(S + t * TP + i, nbytes ? base + i + (int64_t)t * ld : base, nbytes);
-            }
-        } else {
-            const int total = TL * (K4 / 2);
-            for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-                const int t = 2 * (idx % (K4 / 2)), i = idx / (K4 / 2);
-                const int nbytes = (i < rows && t < K) ? (t + 1 < K ? 16 : 8) : 0;
-                cp_async16(S + i * GSLD + t, nbytes ? base + (int64_t)i * ld + t : base, nbytes);
-            }
-        }
-        return;
-    }
-    const int total = TL * K4;
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        if constexpr (TMAJOR) {
-            const int i = idx % TL, t = idx / TL;
-            const bool v = i < rows && t < K;
-            cp_async8(S + t * TP + i, v ? base + i + (int64_t)t * ld : base, v);
-        } else {
-            const int t = idx % K4, i = idx / K4;
-            const bool v = i < rows && t < K;
-            cp_async8(S + i * GSLD + t, v ? base + (int64_t)i * ld + t : base, v);
-        }
-    }
-}
+struct Operand {
+    const double* base;   // a valid address, for copies of nothing
+    const double* p;      // this thread's first source of the next chunk
+    int64_t step;         // between its copies
+    int64_t chunk;        // between chunks
+    double* dst;          // within a stage
+    int t0;               // its first (TMAJOR) or only t
+    int bytes;            // TMAJOR: of the row pair that exist; else: how many of its four rows exist
+    int shift;            // TMAJOR: rows the source is shifted by
+    bool last;            // TMAJOR, shifted: this thread copies row TL - 1 of column tid
 
-template <bool AT, bool BT>
-__device__ __forceinline__ void tile_mma2(const double* As, const double* Bs, int K4, double (&acc)[4][4][2]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = warp & 1, wn = warp >> 1;
-    const int r = lane >> 2, c = lane & 3;
-    for (int kk = 0; kk < K4; kk += 4) {
-        double a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int row = wm * 32 + i * 8 + r;
-            a[i] = AT ? As[(kk + c) * TP + row] : As[row * GSLD + kk + c];
+    __device__ __forceinline__ void init(const double* b, int64_t ld, int rows, double* s) {
+        const int tid = threadIdx.x;
+        base = b;
+        if constexpr (TMAJOR) {
+            shift = (reinterpret_cast<uintptr_t>(b) >> 3) & 1;
+            const int i = 2 * (tid & 31), left = rows + shift - i;
+            t0 = tid >> 5;
+            bytes = left <= 0 ? 0 : left == 1 ? 8 : 16;
+            p = b - shift + (bytes ? i : shift) + (int64_t)t0 * ld;
+            step = 4 * ld;
+            chunk = KC * ld;
+            dst = s + t0 * TP + i;
+            last = shift && rows == TL && tid < KC;
+        } else {
+            const int i = tid >> 3;
+            t0 = 2 * (tid & 7);
+            bytes = rows <= i ? 0 : (rows - i + 15) >> 4;
+            p = b + (int64_t)i * ld + t0;
+            step = 16 * ld;
+            chunk = KC;
+            dst = s + i * KC + (t0 ^ (4 * (i & 3)));
+            shift = 0;
+            last = false;
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int col = wn * 32 + j * 8 + r;
-            b[j] = BT ? Bs[(kk + c) * TP + col] : Bs[col * GSLD + kk + c];
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
-}
+    // Copies the chunk that has `left` columns of K left into stage `st`.
+    __device__ __forceinline__ void issue(int st, int left) {
+        double* d = dst + st * (2 * TILE_D);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if constexpr (TMAJOR) {
+                const bool v = t0 + 4 * u < left;
+                cp_async16(d + 4 * u * TP, v ? p + u * step : base - shift, v ? bytes : 0);
+            } else {
+                const int n = u < bytes ? min(max(left - t0, 0), 2) : 0;
+                cp_async16(d + 16 * u * KC, n ? p + u * step : base, 8 * n);
+            }
+        }
+        if constexpr (TMAJOR) {
+            // row TL - 1 of a shifted source lies in the 33rd pair: its column is this thread's number
+            if (last) {
+                const bool v = (int)threadIdx.x < left;
+                const int64_t ld = step >> 2;
+                const double* q = p + (TL - 2 * (int)(threadIdx.x & 31)) + ((int)threadIdx.x - t0) * ld;
+                cp_async8(d - (t0 * TP + 2 * (threadIdx.x & 31)) + threadIdx.x * TP + TL, v ? q : base, v);
+            }
+        }
+        p += chunk;
+    }
+};
 
 // acc += A B'^T over t in [0, K): A(i, t) = A0[i + t * lda] (i < M), B'(j, t) =
-// B0[j + t * ldb] when BT, else B0[j * ldb + t] (j < N).
+// B0[j + t * ldb] when BT, else B0[j * ldb + t] (j < N).  4 warps in a 2 x 2 grid of 32 x 32.
 template <bool BT>
 __device__ __forceinline__ void gemm_pipelined(const double* A0, int64_t lda, int M, const double* B0, int64_t ldb,
                                                int N, int K, double* smem, double (&acc)[4][4][2]) {
     const int nch = (K + KC - 1) / KC;
-    auto issue = [&](int c) {
-        if (c < nch) {
-            const int k0 = c * KC, Kc = min(KC, K - k0), K4 = (Kc + 3) & ~3;
-            double* st = smem + (c % GEMM_STAGES) * 2 * TILE_D;
-            stage_tile<true>(st, A0 + (int64_t)k0 * lda, lda, M, Kc, K4);
-            stage_tile<BT>(st + TILE_D, BT ? B0 + (int64_t)k0 * ldb : B0 + k0, ldb, N, Kc, K4);
+    Operand<true> A;
+    Operand<BT> B;
+    A.init(A0, lda, M, smem);
+    B.init(B0, ldb, N, smem + TILE_D);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wm = warp & 1, wn = warp >> 1, r = lane >> 2, c = lane & 3;
+    const double* As = smem + c * TP + wm * 32 + r + A.shift;
+    // i-major: (t ^ 4 (i % 4)) with t = kk + c: the k-step kk is swizzled by the row's low bits
+    const double* Bs = smem + TILE_D + (BT ? c * TP + wn * 32 + r + B.shift : (wn * 32 + r) * KC + c);
+    const int sw = BT ? 0 : 4 * (r & 3);
+#pragma unroll
+    for (int s = 0; s < GEMM_STAGES - 1; ++s) {
+        if (s < nch) {
+            A.issue(s, K - s * KC);
+            B.issue(s, K - s * KC);
         }
         cp_async_commit();   // an empty group past the last chunk keeps the wait count uniform
-    };
-#pragma unroll
-    for (int c = 0; c < GEMM_STAGES - 1; ++c) issue(c);
-    for (int c = 0; c < nch; ++c) {
-        issue(c + GEMM_STAGES - 1);
-        cp_async_wait<GEMM_STAGES - 1>();
-        __syncthreads();
-        const int Kc = min(KC, K - c * KC), K4 = (Kc + 3) & ~3;
-        const double* st = smem + (c % GEMM_STAGES) * 2 * TILE_D;
-        tile_mma2<true, BT>(st, st + TILE_D, K4, acc);
-        __syncthreads();
     }
+    int rd = 0, wr = GEMM_STAGES - 1;
+    for (int k = 0; k < nch; ++k) {
+        cp_async_wait<GEMM_STAGES - 2>();
+        __syncthreads();   // chunk k is there, and stage wr, read for chunk k - 1, is free
+        const int left = K - (k + GEMM_STAGES - 1) * KC;
+        if (left > 0) {
+            A.issue(wr, left);
+            B.issue(wr, left);
+        }
+        cp_async_commit();
+        const double* a0 = As + rd * (2 * TILE_D);
+        const double* b0 = Bs + rd * (2 * TILE_D);
+#pragma unroll
+        for (int kk = 0; kk < KC; kk += 4) {
+            double a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = a0[kk * TP + i * 8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = BT ? b0[kk * TP + j * 8] : b0[j * 8 * KC + (kk ^ sw)];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+        }
+        rd = rd + 1 == GEMM_STAGES ? 0 : rd + 1;
+        wr = wr + 1 == GEMM_STAGES ? 0 : wr + 1;
+    }
+    cp_async_wait<0>();
 }
 
 // ---- assembly ----------------------------------------------------------------
@@ -602,44 +642,45 @@ __device__ __forceinline__ void tile_sub_staged(double* __restrict__ C, int64_t 
 }
 
 // Tile t of a job: kind 0 enumerates lower tiles (ti >= tj) column by column,
-// kind 1 the full rectangle.
+// kind 1 the full rectangle.  Column tj of the lower tiles starts at tile
+// tj Tr - tj (tj - 1) / 2; the root of that, corrected, gives tj.
 __device__ __forceinline__ void job_tile(const GemmJob& jb, int t, int& ti, int& tj) {
-    const int Tr = (jb.r1 - jb.r0 + TL - 1) / TL, Tc = (jb.c1 - jb.c0 + TL - 1) / TL;
-    if (jb.kind == 1) { ti = t / Tc; tj = t % Tc; return; }
-    for (tj = 0; tj < Tc; ++tj) {
-        const int cnt = Tr - tj;
-        if (t < cnt) { ti = tj + t; return; }
-        t -= cnt;
-    }
-    ti = Tr;   // not reached for valid t
+    const int Tr = (jb.rows + TL - 1) / TL, Tc = (jb.cols + TL - 1) / TL;
+    if (jb.kind == 1) { ti = t / Tc; tj = t - ti * Tc; return; }
+    const float m = 2.0f * Tr + 1.0f;
+    tj = static_cast<int>(0.5f * (m - sqrtf(fmaxf(0.0f, m * m - 8.0f * t))));
+    tj = max(0, min(tj, Tc - 1));
+    auto start = [&](int c) { return c * Tr - (c * (c - 1)) / 2; };
+    while (tj > 0 && start(tj) > t) --tj;
+    while (tj + 1 < Tc && start(tj + 1) <= t) ++tj;
+    ti = tj + t - start(tj);
 }
 
 #ifndef WRAPD_GEMM_MINB
 #define WRAPD_GEMM_MINB 4
 #endif
 __global__ void __launch_bounds__(GEMM_THREADS, WRAPD_GEMM_MINB) k_update(double* __restrict__ F, double* __restrict__ Y,
-                                                         const FrontDesc* __restrict__ desc, JobList jl) {
+                                                         JobList jl) {
     extern __shared__ __align__(16) double gemm_smem[];
     const int item = find_item(jl.d_prefix, jl.n, blockIdx.x);
     const GemmJob jb = jl.d_jobs[item];
-    const FrontDesc d = desc[jb.front];
     int ti, tj;
     job_tile(jb, blockIdx.x - jl.d_prefix[item], ti, tj);
-    const int r0 = jb.r0 + ti * TL, c0 = jb.c0 + tj * TL;
-    const int M = min(TL, jb.r1 - r0), N = min(TL, jb.c1 - c0);
+    const int r0 = ti * TL, c0 = tj * TL;
+    const int M = min(TL, jb.rows - r0), N = min(TL, jb.cols - c0);
+    double* C = (jb.kind == 0 ? F : Y) + jb.c + r0 + (int64_t)c0 * jb.ldc;
+    // the tile of C that the epilogue reads: towards L2 meanwhile (16 lines of 128 bytes
+    // per 4 columns at most; rows past M stay in the pool's next columns)
+    for (int q = threadIdx.x; q < 4 * N; q += GEMM_THREADS)
+        if (16 * (q & 3) < M) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + 16 * (q & 3) + (int64_t)(q >> 2) * jb.ldc));
     double acc[4][4][2] = {};
-    const double* A0 = F + d.f_off + r0 + (int64_t)jb.k0 * d.ld;
+    const double* A0 = F + jb.a + r0;
     if (jb.kind == 0)
-        gemm_pipelined<true>(A0, d.ld, M, F + d.f_off + c0 + (int64_t)jb.k0 * d.ld, d.ld, N, jb.k1 - jb.k0,
-                             gemm_smem, acc);
+        gemm_pipelined<true>(A0, jb.lda, M, F + jb.b + c0, jb.lda, N, jb.K, gemm_smem, acc);
     else   // B'(j, t) = Y(k0 + t, c0 + j)
-        gemm_pipelined<false>(A0, d.ld, M, Y + d.y_off + jb.k0 + (int64_t)c0 * d.ldy, d.ldy, N, jb.k1 - jb.k0,
-                              gemm_smem, acc);
+        gemm_pipelined<false>(A0, jb.lda, M, Y + jb.b + (int64_t)c0 * jb.ldc, jb.ldc, N, jb.K, gemm_smem, acc);
     // on tiles of kind 0 crossing the diagonal keep only row >= column (global indices)
-    if (jb.kind == 0)
-        tile_sub_staged(F + d.f_off + r0 + (int64_t)c0 * d.ld, d.ld, M, N, r0 - c0, acc, gemm_smem);
-    else
-        tile_sub_staged(Y + d.y_off + r0 + (int64_t)c0 * d.ldy, d.ldy, M, N, TL, acc, gemm_smem);
+    tile_sub_staged(C, jb.ldc, M, N, jb.kind == 0 ? jb.diag + r0 - c0 : TL, acc, gemm_smem);
 }
 
 // W = L_rs Y (r x k) with Y lower triangular: tile (ti, tj) of 64 x 64 sums
@@ -1170,8 +1211,8 @@ JobList CholGPU::make_jobs(const std::vector<GemmJob>& jobs, cudaStream_t st) {
     std::vector<GemmJob> keep;
     std::vector<int> pre(1, 0);
     for (const GemmJob& jb : jobs) {
-        const int Tr = ceil_div(jb.r1 - jb.r0, TL), Tc = ceil_div(jb.c1 - jb.c0, TL);
-        if (Tr <= 0 || Tc <= 0 || jb.k1 <= jb.k0) continue;
+        const int Tr = ceil_div(jb.rows, TL), Tc = ceil_div(jb.cols, TL);
+        if (Tr <= 0 || Tc <= 0 || jb.K <= 0) continue;
         int tiles = 0;
         if (jb.kind == 1) tiles = Tr * Tc;
         else for (int tj = 0; tj < Tc; ++tj) tiles += std::max(0, Tr - tj);
@@ -1334,14 +1375,26 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
                 act.push_back(f);
                 nP.push_back(ceil_div(m, TL));
                 ct.push_back(ceil_div(m, TL) + ceil_div(p0, TL));
+                // F[r0:r1, c0:c1] -= F[r0:r1, k0:k1] F[c0:c1, k0:k1]^T, and
+                // Y[r0:r1, c0:c1] -= F[r0:r1, k0:k1] Y[k0:k1, c0:c1]
+                auto f_job = [&](int r0, int r1, int c0, int c1, int k0, int k1) {
+                    jobs.push_back(GemmJob{d.f_off + r0 + (int64_t)k0 * d.ld, d.f_off + c0 + (int64_t)k0 * d.ld,
+                                           d.f_off + r0 + (int64_t)c0 * d.ld, d.ld, d.ld, r1 - r0, c1 - c0, k1 - k0, 0,
+                                           r0 - c0, 0});
+                };
+                auto y_job = [&](int r0, int r1, int c0, int c1, int k0, int k1) {
+                    jobs.push_back(GemmJob{d.f_off + r0 + (int64_t)k0 * d.ld, d.y_off + k0 + (int64_t)c0 * d.ldy,
+                                           d.y_off + r0 + (int64_t)c0 * d.ldy, d.ld, d.ldy, r1 - r0, c1 - c0, k1 - k0, 1,
+                                           0, 0});
+                };
                 if (j0 < be) {
                     // inside the outer block: only the block's remaining columns, K = this panel
-                    jobs.push_back(GemmJob{f, 0, j0, d.ld, j0, be, p0, j0});
-                    jobs.push_back(GemmJob{f, 1, j0, be, 0, j0, p0, j0});
+                    f_job(j0, d.ld, j0, be, p0, j0);
+                    y_job(j0, be, 0, j0, p0, j0);
                 } else {
                     // the block's last panel: the deferred trailing update, K = the whole block
-                    jobs.push_back(GemmJob{f, 0, be, d.ld, be, d.ld, bs, be});
-                    jobs.push_back(GemmJob{f, 1, be, d.k, 0, be, bs, be});
+                    f_job(be, d.ld, be, d.ld, bs, be);
+                    y_job(be, d.k, 0, be, bs, be);
                 }
             }
             // every active front gets at least one item (its diagonal block is factored there)
@@ -1703,7 +1756,7 @@ void CholGPU::factor_launches(const double* d_w2, const double* d_Di, int ne, cu
                 }
             }
             if (L.update[p].total) {
-                k_update<<<L.update[p].total, GEMM_THREADS, GEMM_SMEM, st>>>(d_F_, d_Y_, d_desc_, L.update[p]);
+                k_update<<<L.update[p].total, GEMM_THREADS, GEMM_SMEM, st>>>(d_F_, d_Y_, L.update[p]);
                 WRAPD_LAUNCH_CHECK();
             }
         }

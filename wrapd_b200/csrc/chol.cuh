@@ -37,8 +37,12 @@ struct FrontDesc {
 // of panel columns.  kind 0: C is F[r0:r1, c0:c1] of the front (lower part
 // where rows and columns overlap), A = F[r0:r1, k0:k1], B' = F[c0:c1, k0:k1];
 // kind 1: C is Y[r0:r1, c0:c1], A = F[r0:r1, k0:k1], B'(j, t) = Y[k0 + t, c0 + j].
-struct GemmJob {
-    int front, kind, r0, r1, c0, c1, k0, k1;
+struct __align__(16) GemmJob {
+    int64_t a, b, c;          // offsets of A, B' and C in their pools (F; F or Y; F or Y)
+    int lda, ldc;             // leading dimensions of A (and B' of kind 0) and of C (and B' of kind 1)
+    int rows, cols, K, kind;
+    int diag;                 // kind 0: the first row's index minus the first column's
+    int pad;
 };
 
 // A solve work item on the host: a 64-wide band starting at b0 (rows forward,
