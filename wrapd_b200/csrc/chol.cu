@@ -387,63 +387,83 @@ __global__ void __launch_bounds__(32 * COLS_PER_CTA) k_assemble_front(double* F,
 
 // ---- panel factorization -------------------------------------------------------
 // Cholesky of the nb x nb (nb <= NB = 32) diagonal block at Fd (column-major,
-// lower part read) and its inverse, by a CTA of 128 threads in shared memory.
+// lower part read) and its inverse, in shared memory by a CTA of CHOL_THREADS:
+// four warps run the pivots, the fifth the inverse, one row behind them.
 // Right-looking: at pivot j every thread updates a fixed slice of 8 entries
 // of row i = tid % 32 (columns tid / 32 + 4m), with all its operands loaded
 // before the first store, so one barrier per pivot is the only serial step.
+// Every thread also works out the next pivot, A'(j+1, j+1) less its update, and
+// starts its rsqrt before the barrier, whose latency then runs behind the updates
+// (the entry itself is left as it is: nobody reads it again).
 // L(i, j) = A'(i, j) rsqrt(d) goes to Lsm (pitch lp), rsqrt(d) to D.  The
-// inverse is right-looking by rows with no barrier: lane c of warp 0 owns
+// inverse is right-looking by rows: lane c of the fifth warp owns
 // column c of inv(L), its partial sums P(r, c) in registers; row s of the
 // column is (delta(s, c) - P(s, c)) / L(s, s), and the rows below add L(r, s)
-// times it (the same fma sequence per entry as a row-by-row sweep).  Row s of
-// inv(L) is written to X (pitch xp), columns < nb.  A non-positive (or NaN)
-// pivot sets *bad and continues with a unit pivot.
+// times it (the same fma sequence per entry as a row-by-row sweep; the sums of
+// rows past nb are never used and are not guarded: the 496 branches took more
+// than half of the inverse's time).  Row s of inv(L) is written to X (pitch xp),
+// columns < nb.  A non-positive (or NaN) pivot sets *bad and continues with a unit
+// pivot.  A pivot's 320 cycles are its rsqrt and the three operations between
+// two of them.  Measured, cycles for a block of 32: pivots 10.4k and inverse
+// behind them 0.3k; with the four warps alone, the inverse after the pivots,
+// 10.4k + 5.1k (12.0k with its guards).
 constexpr int LSP = NB + 1;
+constexpr int CHOL_THREADS = GEMM_THREADS + 32;
 static_assert(GEMM_THREADS == 128 && NB == 32, "cta_chol_inv maps 128 threads onto 32 rows x 4 column slices");
+// A barrier of the CTA's CHOL_THREADS that its warps reach in different loops.
+__device__ __forceinline__ void chol_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(CHOL_THREADS) : "memory"); }
 __device__ __forceinline__ void cta_chol_inv(const double* __restrict__ Fd, int64_t ld, int nb, double* S,
                                              double* Lsm, int lp, double* D, double* X, int xp, bool* bad) {
     const int tid = threadIdx.x;
-    for (int idx = tid; idx < NB * NB; idx += GEMM_THREADS) {
+    for (int idx = tid; idx < NB * NB; idx += CHOL_THREADS) {
         const int i = idx & 31, c = idx >> 5;
         S[i * LSP + c] = (i < nb && c <= i) ? Fd[i + (int64_t)c * ld] : 0.0;
     }
     __syncthreads();
-    const int i = tid & 31, q = tid >> 5;
     bool b = false;
-    for (int j = 0; j < nb; ++j) {
-        double piv = S[j * LSP + j];
-        const double sij = S[i * LSP + j];
-        double cj[8], ic[8];
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            cj[m] = S[(q + 4 * m) * LSP + j];
-            ic[m] = S[i * LSP + q + 4 * m];
-        }
+    if (tid < GEMM_THREADS) {
+        const int i = tid & 31, q = tid >> 5;
+        double piv = S[0];
         if (!(piv > 0.0)) { b = true; piv = 1.0; }
-        const double rs = rsqrt(piv);
-        if (q == 0 && i >= j && i < nb) Lsm[i * lp + j] = i == j ? piv * rs : sij * rs;
-        if (tid == 0) D[j] = rs;
-        const double t = sij * (rs * rs);
+        double rs = rsqrt(piv);
+        for (int j = 0; j < nb; ++j) {
+            const double sij = S[i * LSP + j];
+            const int n = min(j + 1, NB - 1);
+            const double nj = S[n * LSP + j], nn = S[n * LSP + n];
+            double cj[8], ic[8];
 #pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            const int c = q + 4 * m;
-            if (c > j && c <= i && i < nb) S[i * LSP + c] = fma(-t, cj[m], ic[m]);
+            for (int m = 0; m < 8; ++m) {
+                cj[m] = S[(q + 4 * m) * LSP + j];
+                ic[m] = S[i * LSP + q + 4 * m];
+            }
+            const double r2 = rs * rs;
+            double next = fma(-(nj * r2), nj, nn);
+            if (j + 1 < nb && !(next > 0.0)) { b = true; next = 1.0; }
+            if (q == 0 && i >= j && i < nb) Lsm[i * lp + j] = i == j ? piv * rs : sij * rs;
+            if (tid == 0) D[j] = rs;
+            const double t = sij * r2;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                const int c = q + 4 * m;
+                if (c > j && c <= i && i < nb && i > j + 1) S[i * LSP + c] = fma(-t, cj[m], ic[m]);
+            }
+            piv = next;
+            rs = rsqrt(next);
+            chol_barrier();
         }
-        __syncthreads();
-    }
-    if (tid < 32) {
-        const int c = tid;
+    } else {
+        const int c = tid - GEMM_THREADS;
         double P[NB];
 #pragma unroll
         for (int r = 0; r < NB; ++r) P[r] = 0.0;
 #pragma unroll
         for (int s = 0; s < NB; ++s) {
             if (s < nb) {
+                chol_barrier();   // column s of L and D[s] are there
                 const double f = (c <= s) ? ((c == s ? 1.0 : 0.0) - P[s]) * D[s] : 0.0;
                 if (c < nb) X[s * xp + c] = f;
 #pragma unroll
-                for (int r = s + 1; r < NB; ++r)
-                    if (r < nb) P[r] = fma(Lsm[r * lp + s], f, P[r]);
+                for (int r = s + 1; r < NB; ++r) P[r] = fma(Lsm[r * lp + s], f, P[r]);
             }
         }
     }
@@ -454,7 +474,7 @@ __device__ __forceinline__ void cta_chol_inv(const double* __restrict__ Fd, int6
 // Diagonal step alone, for panel steps with many CTAs (where redoing the
 // block in every CTA would cost more than a launch): one CTA per front
 // factors the block and writes Li as the diagonal block of Y.
-__global__ void __launch_bounds__(GEMM_THREADS) k_diag(const double* __restrict__ F, double* __restrict__ Y,
+__global__ void __launch_bounds__(CHOL_THREADS) k_diag(const double* __restrict__ F, double* __restrict__ Y,
                                                        const FrontDesc* __restrict__ desc, WorkList wl, int p,
                                                        int* __restrict__ status) {
     __shared__ double S[NB * LSP];
@@ -468,7 +488,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_diag(const double* __restrict_
     cta_chol_inv(F + d.f_off + p0 + (int64_t)p0 * d.ld, d.ld, nb, S, Lsm, LSP, D, X, LSP, &bad);
     if (bad && threadIdx.x == 0) atomicExch(status, WRAPD_E_NOT_SPD);
     double* Yp = Y + d.y_off + p0;   // row block p of Y (column-major, ld = ldy)
-    for (int idx = threadIdx.x; idx < NB * NB; idx += GEMM_THREADS) {
+    for (int idx = threadIdx.x; idx < NB * NB; idx += CHOL_THREADS) {
         const int i = idx & 31, c = idx >> 5;
         if (i < nb && c < nb) Yp[i + (int64_t)(p0 + c) * d.ldy] = c <= i ? X[i * LSP + c] : 0.0;
     }
@@ -520,7 +540,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_trsm(double* __restrict__ F, d
 // neither has one item that only factors.  The front's first item writes Li
 // as the diagonal block of Y.  F's diagonal block is read, never written: the
 // solve and the later steps use only Y, W and the panels below it.
-__global__ void __launch_bounds__(GEMM_THREADS) k_panel(double* __restrict__ F, double* __restrict__ Y,
+__global__ void __launch_bounds__(CHOL_THREADS) k_panel(double* __restrict__ F, double* __restrict__ Y,
                                                         const FrontDesc* __restrict__ desc, WorkList wl,
                                                         const int* __restrict__ nP_of_item, int p,
                                                         int* __restrict__ status) {
@@ -545,7 +565,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_panel(double* __restrict__ F, 
     if (ptile) {
         const int m = min(d.ld - j0 - tile * TL, TL);
         const double* A = F + d.f_off + j0 + tile * TL + (int64_t)p0 * d.ld;
-        for (int idx = tid; idx < TL * K4; idx += GEMM_THREADS) {
+        for (int idx = tid; idx < TL * K4; idx += CHOL_THREADS) {
             const int i = idx % TL, t = idx / TL;
             const bool v = i < m && t < nb;
             cp_async8(As + i * SLD + t, v ? A + i + (int64_t)t * d.ld : A, v);
@@ -553,7 +573,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_panel(double* __restrict__ F, 
     } else if (ytile) {
         const int n = min(p0 - c0, TL);
         const double* Yr = Y + d.y_off + p0 + (int64_t)c0 * d.ldy;
-        for (int idx = tid; idx < TL * K4; idx += GEMM_THREADS) {
+        for (int idx = tid; idx < TL * K4; idx += CHOL_THREADS) {
             const int t = idx % K4, j = idx / K4;
             const bool v = j < n && t < nb;
             cp_async8(Bs + j * SLD + t, v ? Yr + t + (int64_t)j * d.ldy : Yr, v);
@@ -564,22 +584,22 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_panel(double* __restrict__ F, 
     // Li(j, t)), A for inverse row-block tiles (A(i, t) = Li(i, t)); rows 32..63
     // of that slot hold L meanwhile and are cleared afterwards.
     double* Ls = ptile ? Bs : As;
-    for (int idx = tid; idx < NB * SLD; idx += GEMM_THREADS) Ls[idx] = 0.0;
+    for (int idx = tid; idx < NB * SLD; idx += CHOL_THREADS) Ls[idx] = 0.0;
     bool bad = false;
     cta_chol_inv(F + d.f_off + p0 + (int64_t)p0 * d.ld, d.ld, nb, S, Ls + NB * SLD, SLD, D, Ls, SLD, &bad);
     if (tile == 0) {
         if (bad && tid == 0) atomicExch(status, WRAPD_E_NOT_SPD);
         double* Yp = Y + d.y_off + p0;   // row block p of Y (column-major, ld = ldy)
-        for (int idx = tid; idx < NB * NB; idx += GEMM_THREADS) {
+        for (int idx = tid; idx < NB * NB; idx += CHOL_THREADS) {
             const int i = idx & 31, c = idx >> 5;
             if (i < nb && c < nb) Yp[i + (int64_t)(p0 + c) * d.ldy] = Ls[i * SLD + c];
         }
     }
     __syncthreads();
-    for (int idx = tid; idx < NB * SLD; idx += GEMM_THREADS) Ls[NB * SLD + idx] = 0.0;
+    for (int idx = tid; idx < NB * SLD; idx += CHOL_THREADS) Ls[NB * SLD + idx] = 0.0;
     cp_async_wait<0>();
     __syncthreads();
-    if (!ptile && !ytile) return;
+    if ((!ptile && !ytile) || tid >= GEMM_THREADS) return;   // the product is the first four warps'
     double acc[4][4][2] = {};
     tile_mma(As, Bs, K4, acc);
     if (ptile) {
@@ -1740,13 +1760,13 @@ void CholGPU::factor_launches(const double* d_w2, const double* d_Di, int ne, cu
         for (size_t p = 0; p < L.trsm.size(); ++p) {
             if (L.trsm[p].total <= fused_ctas_) {
                 if (L.trsm[p].total) {
-                    k_panel<<<L.trsm[p].total, GEMM_THREADS, 0, st>>>(d_F_, d_Y_, d_desc_, L.trsm[p],
+                    k_panel<<<L.trsm[p].total, CHOL_THREADS, 0, st>>>(d_F_, d_Y_, d_desc_, L.trsm[p],
                                                                       trsm_nP_[l][p], (int)p, d_status);
                     WRAPD_LAUNCH_CHECK();
                 }
             } else {
                 if (L.diag[p].n) {
-                    k_diag<<<L.diag[p].n, GEMM_THREADS, 0, st>>>(d_F_, d_Y_, d_desc_, L.diag[p], (int)p, d_status);
+                    k_diag<<<L.diag[p].n, CHOL_THREADS, 0, st>>>(d_F_, d_Y_, d_desc_, L.diag[p], (int)p, d_status);
                     WRAPD_LAUNCH_CHECK();
                 }
                 if (L.trsm[p].total) {
