@@ -744,8 +744,8 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_wgemm(const double* __restrict
 // of ten levels is a chain of ten such hand-overs, each way.  The partial sums
 // of a band's chunks are handed to the band's last item the same way and added
 // in chunk order, so results do not depend on which CTA takes which item.
-// kUnset is a signalling NaN, which no arithmetic operation returns, and every
-// value stored in these buffers is the result of one.
+// (kUnset, see common.cuh; every value stored in these buffers is the result of
+// an arithmetic operation.)
 //
 // Everything waited for comes from items earlier in the list, which were taken
 // by running CTAs, so the earliest unfinished item never waits and the list
@@ -776,43 +776,10 @@ constexpr int kSolveItems = 2 * 148;   // items wanted per level (see build and 
 constexpr int kBwdSub = 4;            // narrow backward bands per 64 columns
 constexpr size_t kBwdDeepBytes = (size_t)3 << 29;     // largest [Y; W] of the deep backward ring (see k_bwd_queue)
 constexpr size_t kGateBytes = (size_t)256 << 20;      // largest [Y; W] whose items poll their inputs directly (see k_fwd_queue)
-constexpr unsigned long long kUnset = 0x7ff45a5a5a5a5a5aull;
-
-__device__ __forceinline__ bool unset(double v) {
-    return static_cast<unsigned long long>(__double_as_longlong(v)) == kUnset;
-}
-__device__ __forceinline__ double ld_relaxed(const double* p) {
-    double v;
-    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed(double* p, double v) {
-    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
-}
 __device__ __forceinline__ void st_unset3(double* p) {
-    const double u = __longlong_as_double(static_cast<long long>(kUnset));
-    st_relaxed(p, u);
-    st_relaxed(p + 1, u);
-    st_relaxed(p + 2, u);
-}
-
-__global__ void k_unset(double* __restrict__ p, int64_t n) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = __longlong_as_double(static_cast<long long>(kUnset));
-}
-
-// After the i-th look at entries that were not all set (i from 0): whether to
-// look again.
-__device__ __forceinline__ bool look_again(int i, unsigned long long& t0, int* status) {
-    if (*reinterpret_cast<volatile int*>(status) != 0) return false;
-    const unsigned long long now = global_ns();
-    if (i == 0) t0 = now;
-    if (now - t0 > kWaitNs || i >= kWaitPolls) {
-        atomicCAS(status, 0, WRAPD_E_TIMEOUT);
-        return false;
-    }
-    __nanosleep(32);
-    return true;
+    st_relaxed(p, unset_value());
+    st_relaxed(p + 1, unset_value());
+    st_relaxed(p + 2, unset_value());
 }
 
 // The rows of three values at p[0 .. N-1] (null: zeros), looked at until all
@@ -1642,14 +1609,9 @@ void CholGPU::build_queues(cudaStream_t st) {
 // The state that a solve starts from and leaves behind: every hand-over entry
 // unset, both queue heads 0.
 void CholGPU::fill_unset(cudaStream_t st) {
-    auto fill = [&](double* p, int64_t count) {
-        if (count <= 0) return;
-        k_unset<<<ceil_div(count, 256), 256, 0, st>>>(p, count);
-        WRAPD_LAUNCH_CHECK();
-    };
-    fill(d_U_, u_pool_);
-    fill(d_Xp_, 3 * (int64_t)n);
-    fill(d_P_, 3 * TL * solve_parts_);
+    unset_fill(d_U_, u_pool_, st);
+    unset_fill(d_Xp_, 3 * (int64_t)n, st);
+    unset_fill(d_P_, 3 * TL * solve_parts_, st);
     WRAPD_CUDA(cudaMemsetAsync(d_heads_, 0, 2 * sizeof(unsigned), st));
     solve_stale_ = false;
 }

@@ -72,19 +72,12 @@ __device__ __forceinline__ T block_max(T v, T* smem) {
 }
 
 // ---- bounded waits between CTAs ----------------------------------------------
-// A wait on a counter that other CTAs raise (release: their writes, a fence,
-// then the atomic) polls it with an acquire load for at most one second of the
-// global timer and kWaitPolls polls.  One that gives up sets *status to
-// WRAPD_E_TIMEOUT (if it was 0) and returns false; a wait that finds *status
-// already set returns false at once, so every waiter of a failed launch ends.
+// A wait looks at most kWaitPolls times and for one second of the global timer
+// (look_again).  One that gives up sets *status to WRAPD_E_TIMEOUT (if it was 0)
+// and one that finds *status already set ends at once, so every waiter of a
+// failed launch ends.
 constexpr unsigned long long kWaitNs = 1000000000ull;
 constexpr int kWaitPolls = 1 << 24;
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -92,16 +85,49 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-__device__ __forceinline__ bool wait_count_geq(const unsigned* count, unsigned target, int* status) {
-    const unsigned long long t0 = global_ns();
-    for (int i = 0; i < kWaitPolls; ++i) {
-        if (ld_acquire(count) >= target) return true;
-        if (*reinterpret_cast<volatile int*>(status) != 0) return false;
-        if (global_ns() - t0 > kWaitNs) break;
-        __nanosleep(64);
+// ---- values handed from CTA to CTA by themselves -----------------------------
+// An entry that is not yet written holds kUnset; its reader polls the entry itself
+// until it holds a value, which thus crosses in one store and one load, with no
+// fence, counter or flag between them.  kUnset is a signalling NaN, which no
+// arithmetic operation returns, so no result can be mistaken for it.
+constexpr unsigned long long kUnset = 0x7ff45a5a5a5a5a5aull;
+
+__device__ __forceinline__ bool unset(double v) {
+    return static_cast<unsigned long long>(__double_as_longlong(v)) == kUnset;
+}
+__device__ __forceinline__ double unset_value() { return __longlong_as_double(static_cast<long long>(kUnset)); }
+__device__ __forceinline__ double ld_relaxed(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed(double* p, double v) {
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+// After the i-th look at entries that were not all set (i from 0): whether to
+// look again.  The status word and the timer, a round trip to memory each, are
+// looked at every sixteenth time only: a hand-over's latency is a few looks.
+__device__ __forceinline__ bool look_again(int i, unsigned long long& t0, int* status) {
+    if ((i & 15) != 15) return true;
+    if (*reinterpret_cast<volatile int*>(status) != 0) return false;
+    const unsigned long long now = global_ns();
+    if (i == 15) t0 = now;
+    if (now - t0 > kWaitNs || i >= kWaitPolls) {
+        atomicCAS(status, 0, WRAPD_E_TIMEOUT);
+        return false;
     }
-    atomicCAS(status, 0, WRAPD_E_TIMEOUT);
-    return false;
+    __nanosleep(32);
+    return true;
+}
+
+static __global__ void k_unset(double* __restrict__ p, int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = unset_value();
+}
+inline void unset_fill(double* p, int64_t n, cudaStream_t st) {
+    if (n <= 0) return;
+    k_unset<<<ceil_div(n, 256), 256, 0, st>>>(p, n);
+    WRAPD_LAUNCH_CHECK();
 }
 
 // ---- deterministic grid reduction: per-block partials, summed in block order

@@ -605,62 +605,167 @@ static __global__ void __launch_bounds__(256) k_lbfgs_second(Tiles T, const int*
     }
 }
 
-// ---- the two-loop recursion in one cooperative launch per loop (one mesh) ---------
-// For a single mesh above the one-CTA size the M + 1 steps of each loop are
-// the k_lbfgs_first / k_lbfgs_second steps above, run by one cooperative launch
-// (all CTAs resident): CTA b takes vector tiles b, b + G, ... and keeps them
-// for the whole loop, each step's inner product is the same per-tile block sum
-// in partials (two buffers, alternating by step), and after a grid barrier
-// every CTA adds the tile partials in the seg_reduce order -- the same alpha_i,
-// c_i and decrement as the per-step launches, bit for bit, in every CTA.  The
-// barrier is a counter the CTAs raise, waited on with wait_count_geq (bounded;
-// a wait that gives up leaves WRAPD_E_TIMEOUT in *status and the CTA returns).
-// REG (when the grid has a CTA per tile at the register form's occupancy):
-// a CTA's kTwoLoopPT entries per thread stay in registers for the whole loop,
-// q is stored once at the end, and the two history vectors of the next step
-// (which do not change during the loop) are loaded before the grid barrier, so
-// no step waits on a memory round trip after its barrier.  The per-entry
-// operations and the order of every sum are those of the tile loop.
+// ---- the two-loop recursion in one launch per loop -------------------------------
+// The M + 1 steps of each loop above, with the vectors' entries in registers or
+// walked in place, and the step's inner product exchanged inside the launch.  The
+// per-entry operations and the order of every sum are those of the per-step
+// launches: the same alpha_i, c_i and decrement, bit for bit, in every CTA.  The
+// second loop can end with the step x <- x - q of k_xupdate (`x` given), whose
+// restart rule needs the decrement that every CTA then holds: q never goes to memory.
+// Us per inner iteration at history 5, first + second loop (+ x step before): a
+// barrier of atomics per step or one CTA per small mesh before, now:
+//   8x8x32      10.7 + 11.7 + 3.5     7.1 +  9.6
+//   16x16x64    13.2 + 15.7 + 4.8    10.0 + 12.7
+//   24x24x48    13.7 + 17.1 + 6.1    11.1 + 17.6
+//   32x32x128   16.2 + 19.8 + 6.3    14.6 + 20.5
+//   16 bars     18 + 18 + 11 per-step launches of 10.5 + 5.5 -> 10 + 14 + 12 + 16
+struct TwoLoopArgs {
+    const MeshCtl* ctl;
+    VecPools P;
+    const double* rho;    // per mesh, kHistSlots each
+    double* q;
+    TwoLoopSlots sl;
+    double* scal;
+    int stride;
+    double* x;            // second loop: x to step, or null (q is stored instead)
+};
+
+// x and s = x_new - x_old at entry i (k_xupdate with rate 1).
+__device__ __forceinline__ void x_step(const TwoLoopArgs& a, double* s, int i, double step) {
+    const double xo = a.x[i];
+    const double xn = xo - step;
+    s[i] = xn - xo;
+    a.x[i] = xn;
+}
+
+// Meshes above kTwoLoopMaxN unknowns: a cooperative launch (all CTAs resident).
+// Step j's tile sums go to slots[j * count + tile].  In a mesh of at most
+// kDirectTiles tiles every CTA polls them (see kUnset) and adds them in
+// seg_reduce's order; with more, that many readers of the same few lines slow the
+// writers down, so the mesh's first CTA alone does, and hands the total on in
+// eight copies.  Each launch unsets the other loop's slots and totals, whose
+// launch has ended.  REG: a CTA per tile of any
+// mesh, kTwoLoopPT entries of q per thread in registers and the two history vectors
+// of the next step loaded before the exchange.  Otherwise one mesh, CTA b taking tiles
+// b, b + G, ... with q in memory.
 constexpr int kTwoLoopGridThreads = 256;
+constexpr int kDirectTiles = 64;   // (203 tiles: 26 + 38 us polled by all, 15 + 21 through the first CTA)
 constexpr int kTwoLoopPT = kVecTile / kTwoLoopGridThreads;
 static_assert(kVecTile % kTwoLoopGridThreads == 0, "whole entries per thread");
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int* status) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(bar, 1u);
-        ok = wait_count_geq(bar, target, status) ? 1 : 0;
+
+// q <- qs + cf v over a tile (v null: as it is; qd null: not stored), and the threads'
+// parts of <w, q> (w null: 0) to `sum`.  Four entries' reads go out together.
+template <typename F>
+__device__ __forceinline__ void walk_tile(const Tile& tl, const double* qs, double* qd, const double* v, double cf,
+                                          const double* w, F&& sum) {
+    double red = 0.0;
+    constexpr int U = 4;
+    for (int i = tl.first + (int)threadIdx.x; i < tl.end; i += U * kTwoLoopGridThreads) {
+        double qi[U], vi[U], wi[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = i + u * kTwoLoopGridThreads;
+            qi[u] = k < tl.end ? qs[k] : 0.0;
+            vi[u] = (v && k < tl.end) ? v[k] : 0.0;
+            wi[u] = (w && k < tl.end) ? w[k] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = i + u * kTwoLoopGridThreads;
+            if (k >= tl.end) break;
+            if (v) qi[u] = qi[u] + cf * vi[u];
+            if (qd) qd[k] = qi[u];
+            if (w) red += wi[u] * qi[u];
+        }
     }
-    __syncthreads();
-    return ok != 0;
+    sum(red);
 }
 
-// The total over the mesh's tiles of partials[] in seg_reduce's order (every thread gets it).
-__device__ __forceinline__ double grid_total(const double* partials, int ntiles) {
-    __shared__ double sm[32];
-    __shared__ double total;
-    double acc = 0.0;
-    for (int b = threadIdx.x; b < ntiles; b += blockDim.x) acc += __ldcg(partials + b);
-    const double r = block_sum(acc, sm);
-    if (threadIdx.x == 0) total = r;
-    __syncthreads();
-    return total;
-}
+constexpr int kTotalCopies = 8, kTotalPitch = 16;      // copies of a total, a 128-byte line each
+constexpr int kTotalSlots = kHistSlots * kTotalCopies * kTotalPitch;   // doubles per mesh
+struct GridExchange {
+    double* slots;
+    double* totals;       // the mesh's
+    int count, t0, t1;
+    int* status;
+    bool lead;            // the mesh's first CTA
+    // A tile's sum of the threads' v (block_sum's order), to slot j.  `again`: the
+    // second or a later tile of the step.
+    __device__ __forceinline__ void put(int j, int tile, double v, bool again = false) {
+        __shared__ double sm[kTwoLoopGridThreads / 32];
+        if (again) __syncthreads();   // thread 0 has read the tile's before
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double r = 0.0;
+            for (int w = 0; w < kTwoLoopGridThreads / 32; ++w) r += sm[w];
+            st_relaxed(slots + (size_t)j * count + tile, r);
+        }
+    }
+    // The total of slot j over the mesh's tiles, in every thread; false when a wait gave up.
+    __device__ __forceinline__ bool get(int j, double& total) {
+        __shared__ double sm[kTwoLoopGridThreads / 32];
+        double acc = 0.0;
+        bool ok = true;
+        unsigned long long since = 0;
+        const bool direct = t1 - t0 <= kDirectTiles;
+        if (!direct && !lead) {
+            if (threadIdx.x == 0) {
+                const double* p = totals + (j * kTotalCopies + blockIdx.x % kTotalCopies) * kTotalPitch;
+                double v = ld_relaxed(p);
+                for (int i = 0; unset(v) && ok; ++i) {
+                    ok = look_again(i, since, status);
+                    v = ld_relaxed(p);
+                }
+                sm[0] = v;
+            }
+            ok = __syncthreads_and(ok);
+            total = sm[0];
+            return ok;
+        }
+        for (int b = t0 + (int)threadIdx.x; b < t1; b += kTwoLoopGridThreads) {
+            double v = ld_relaxed(slots + (size_t)j * count + b);
+            for (int i = 0; unset(v) && ok; ++i) {
+                ok = look_again(i, since, status);
+                v = ld_relaxed(slots + (size_t)j * count + b);
+            }
+            acc += v;
+        }
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
+        ok = __syncthreads_and(ok);
+        double r = 0.0;
+        for (int w = 0; w < kTwoLoopGridThreads / 32; ++w) r += sm[w];
+        total = r;
+        if (!direct && ok && threadIdx.x < kTotalCopies)
+            st_relaxed(totals + (j * kTotalCopies + threadIdx.x) * kTotalPitch, r);
+        return ok;
+    }
+};
 
 template <bool SECOND, bool REG>
-static __global__ void __launch_bounds__(kTwoLoopGridThreads) k_two_loop_grid(Tiles T, const MeshCtl* __restrict__ ctl, VecPools P,
-                                                       const double* __restrict__ rho, double* __restrict__ q,
-                                                       TwoLoopSlots sl, double* partials, unsigned* bar,
-                                                       int* status, double* scal) {
-    __shared__ double sm[32];
-    const MeshCtl c = ctl[0];
-    const int ntiles = T.count, G = gridDim.x;
-    unsigned nbar = 0;
+static __global__ void __launch_bounds__(kTwoLoopGridThreads, REG ? 3 : 4) k_two_loop_grid(Tiles T, const int* on, TwoLoopArgs A,
+                                                       double* slots, double* other, int nslots, int* status) {
+    const int count = T.count, G = gridDim.x;
+    for (int s = threadIdx.x; s < nslots * ((count + G - 1) / G); s += kTwoLoopGridThreads) {
+        const int t = blockIdx.x + (s / nslots) * G;
+        if (t < count) st_relaxed(other + (size_t)(s % nslots) * count + t, unset_value());
+    }
+    const Tile tl = tile_at(T, blockIdx.x);
+    if (!mesh_on(on, tl.mesh)) return;
+    const MeshCtl c = A.ctl[tl.mesh];
+    const VecPools& P = A.P;
+    const double* rho = A.rho + (size_t)tl.mesh * kHistSlots;
+    double* scal = A.scal + (size_t)tl.mesh * A.stride;
+    const int t0 = T.t ? T.tile0[tl.mesh] : 0;
+    const bool first_cta = (int)blockIdx.x == t0;
+    const size_t totals = (size_t)kHistSlots * count + (size_t)tl.mesh * kTotalSlots;
+    GridExchange X{slots, slots + totals, count, t0, T.t ? T.tile0[tl.mesh + 1] : count, status, first_cta};
+    if (first_cta)
+        for (int s = threadIdx.x; s < nslots * kTotalCopies; s += kTwoLoopGridThreads)
+            st_relaxed(other + totals + s * kTotalPitch, unset_value());
     if constexpr (REG) {
-        // one tile per CTA (the host launches REG only with ntiles <= G), kept in registers
-        const int t = blockIdx.x;
-        const Tile tl = t < ntiles ? tile_at(T, t) : Tile{0, 0, 0};
         const int i0 = tl.first + (int)threadIdx.x;
         double qv[kTwoLoopPT], av[kTwoLoopPT], bv[kTwoLoopPT];
         auto load = [&](double (&v)[kTwoLoopPT], const double* src) {
@@ -674,7 +779,7 @@ static __global__ void __launch_bounds__(kTwoLoopGridThreads) k_two_loop_grid(Ti
 #pragma unroll
             for (int k = 0; k < kTwoLoopPT; ++k) {
                 const int i = i0 + k * kTwoLoopGridThreads;
-                if (i < tl.end) q[i] = qv[k];
+                if (i < tl.end) A.q[i] = qv[k];
             }
         };
         if constexpr (!SECOND) {
@@ -696,21 +801,19 @@ static __global__ void __launch_bounds__(kTwoLoopGridThreads) k_two_loop_grid(Ti
                     }
                 }
                 if (j < 0) break;
-                double* part = partials + (size_t)(j & 1) * ntiles;
-                const double r = block_sum(red, sm);
-                if (threadIdx.x == 0 && t < ntiles) part[t] = r;
+                X.put(j, blockIdx.x, red);
                 load(av, P.Y[hist_slot(c, j, P.M)]);
                 load(bv, j - 1 >= 0 ? P.S[hist_slot(c, j - 1, P.M)] : nullptr);
-                nbar += G;
-                if (!grid_barrier(bar, nbar, status)) return;
-                alpha_next = rho[hist_slot(c, j, P.M)] * grid_total(part, ntiles);
-                if (blockIdx.x == 0 && threadIdx.x == 0) scal[sl.alpha + j] = alpha_next;
+                double tot;
+                if (!X.get(j, tot)) return;
+                alpha_next = rho[hist_slot(c, j, P.M)] * tot;
+                if (first_cta && threadIdx.x == 0) scal[A.sl.alpha + j] = alpha_next;
             }
             store_q();
         } else {
             // av: s_{j-1} (the update), bv: y_j or g (the inner product) of step j
-            double c_prev = 0.0;
-            load(qv, q);
+            double c_prev = 0.0, dir = 0.0;
+            load(qv, A.q);
             load(bv, 0 < c.it ? P.Y[hist_slot(c, 0, P.M)] : g_cur(P, c));
             for (int j = 0; j <= c.it; ++j) {
                 const double cf = j > 0 ? c_prev : 0.0;
@@ -726,204 +829,175 @@ static __global__ void __launch_bounds__(kTwoLoopGridThreads) k_two_loop_grid(Ti
                         red += bv[k] * qi;
                     }
                 }
-                double* part = partials + (size_t)(j & 1) * ntiles;
-                const double r = block_sum(red, sm);
-                if (threadIdx.x == 0 && t < ntiles) part[t] = r;
+                X.put(j, blockIdx.x, red);
                 if (j < c.it) {
                     load(av, P.S[hist_slot(c, j, P.M)]);
                     load(bv, j + 1 < c.it ? P.Y[hist_slot(c, j + 1, P.M)] : g_cur(P, c));
                 }
-                nbar += G;
-                if (!grid_barrier(bar, nbar, status)) return;
-                const double tot = grid_total(part, ntiles);
+                double tot;
+                if (!X.get(j, tot)) return;
                 if (j < c.it) {
-                    c_prev = __ldcg(scal + sl.alpha + j) + (-rho[hist_slot(c, j, P.M)]) * tot;
-                    if (blockIdx.x == 0 && threadIdx.x == 0) scal[sl.c + j] = c_prev;
-                } else if (blockIdx.x == 0 && threadIdx.x == 0) {
-                    scal[sl.dir] = tot;
+                    c_prev = __ldcg(scal + A.sl.alpha + j) + (-rho[hist_slot(c, j, P.M)]) * tot;
+                    if (first_cta && threadIdx.x == 0) scal[A.sl.c + j] = c_prev;
+                } else {
+                    dir = tot;
+                    if (first_cta && threadIdx.x == 0) scal[A.sl.dir] = tot;
                 }
             }
-            store_q();
+            if (!A.x) { store_q(); return; }
+            const bool restart = !(dir > 0.0);   // bv holds g
+#pragma unroll
+            for (int k = 0; k < kTwoLoopPT; ++k) {
+                const int i = i0 + k * kTwoLoopGridThreads;
+                if (i < tl.end) x_step(A, P.S[c.stage], i, restart ? bv[k] : qv[k]);
+            }
         }
-        return;
     } else if constexpr (!SECOND) {
-        // first loop, j = it - 1 .. -1: q = (first ? g : q) - alpha_{j+1} y_{j+1}; alpha_j = rho_j <s_j, q>
+        // j = it - 1 .. -1: q = (first ? g : q) - alpha_{j+1} y_{j+1}; alpha_j = rho_j <s_j, q>
         double alpha_next = 0.0;
         for (int j = c.it - 1; j >= -1; --j) {
             const bool first = j == c.it - 1;
-            const double* g = g_cur(P, c);
+            const double* qs = first ? g_cur(P, c) : A.q;
             const double* yv = first ? nullptr : P.Y[hist_slot(c, j + 1, P.M)];
             const double cf = first ? 0.0 : -alpha_next;
             const double* sv = j >= 0 ? P.S[hist_slot(c, j, P.M)] : nullptr;
-            double* part = partials + (size_t)(j & 1) * ntiles;
-            for (int t = blockIdx.x; t < ntiles; t += G) {
-                const Tile tl = tile_at(T, t);
-                double red = 0.0;
-                for (int i = tl.first + (int)threadIdx.x; i < tl.end; i += blockDim.x) {
-                    double qi = first ? g[i] : q[i];
-                    if (yv) qi = qi + cf * yv[i];
-                    q[i] = qi;
-                    if (sv) red += sv[i] * qi;
-                }
-                if (j >= 0) {
-                    const double r = block_sum(red, sm);
-                    if (threadIdx.x == 0) part[t] = r;
-                }
-            }
+            for (int t = blockIdx.x; t < count; t += G)
+                walk_tile(tile_at(T, t), qs, A.q, yv, cf, sv, [&](double red) { if (j >= 0) X.put(j, t, red, t != (int)blockIdx.x); });
             if (j < 0) break;
-            nbar += G;
-            if (!grid_barrier(bar, nbar, status)) return;
-            alpha_next = rho[hist_slot(c, j, P.M)] * grid_total(part, ntiles);
-            if (blockIdx.x == 0 && threadIdx.x == 0) scal[sl.alpha + j] = alpha_next;
+            double tot;
+            if (!X.get(j, tot)) return;
+            alpha_next = rho[hist_slot(c, j, P.M)] * tot;
+            if (first_cta && threadIdx.x == 0) scal[A.sl.alpha + j] = alpha_next;
         }
     } else {
-        // second loop, j = 0 .. it: q += c_{j-1} s_{j-1}; c_j = alpha_j - rho_j <y_j, q>, dir = <g, q>
-        double c_prev = 0.0;
+        // j = 0 .. it: q += c_{j-1} s_{j-1}; c_j = alpha_j - rho_j <y_j, q>, dir = <g, q>
+        double c_prev = 0.0, dir = 0.0;
         for (int j = 0; j <= c.it; ++j) {
             const double* sv = j > 0 ? P.S[hist_slot(c, j - 1, P.M)] : nullptr;
-            const double cf = j > 0 ? c_prev : 0.0;
             const double* w = j < c.it ? P.Y[hist_slot(c, j, P.M)] : g_cur(P, c);
-            double* part = partials + (size_t)(j & 1) * ntiles;
-            for (int t = blockIdx.x; t < ntiles; t += G) {
-                const Tile tl = tile_at(T, t);
-                double red = 0.0;
-                for (int i = tl.first + (int)threadIdx.x; i < tl.end; i += blockDim.x) {
-                    double qi = q[i];
-                    if (sv) {
-                        qi = qi + cf * sv[i];
-                        q[i] = qi;
-                    }
-                    red += w[i] * qi;
-                }
-                const double r = block_sum(red, sm);
-                if (threadIdx.x == 0) part[t] = r;
-            }
-            nbar += G;
-            if (!grid_barrier(bar, nbar, status)) return;
-            const double tot = grid_total(part, ntiles);
+            for (int t = blockIdx.x; t < count; t += G)
+                walk_tile(tile_at(T, t), A.q, j > 0 ? A.q : nullptr, sv, c_prev, w, [&](double red) { X.put(j, t, red, t != (int)blockIdx.x); });
+            double tot;
+            if (!X.get(j, tot)) return;
             if (j < c.it) {
-                c_prev = __ldcg(scal + sl.alpha + j) + (-rho[hist_slot(c, j, P.M)]) * tot;
-                if (blockIdx.x == 0 && threadIdx.x == 0) scal[sl.c + j] = c_prev;
-            } else if (blockIdx.x == 0 && threadIdx.x == 0) {
-                scal[sl.dir] = tot;
+                c_prev = __ldcg(scal + A.sl.alpha + j) + (-rho[hist_slot(c, j, P.M)]) * tot;
+                if (first_cta && threadIdx.x == 0) scal[A.sl.c + j] = c_prev;
+            } else {
+                dir = tot;
+                if (first_cta && threadIdx.x == 0) scal[A.sl.dir] = tot;
             }
         }
+        if (!A.x) return;
+        const double* step = !(dir > 0.0) ? g_cur(P, c) : A.q;
+        for (int t = blockIdx.x; t < count; t += G) {
+            const Tile w = tile_at(T, t);
+            for (int i = w.first + (int)threadIdx.x; i < w.end; i += kTwoLoopGridThreads) x_step(A, P.S[c.stage], i, step[i]);
+        }
     }
 }
 
-// ---- the two-loop recursion in one CTA per mesh, for small meshes -----------------
-// With 3 x free vertices <= kTwoLoopMaxN the chain of short reductions above is
-// latency-bound: one 1024-thread CTA per mesh runs each half of the
-// recursion, q in registers (kTwoLoopPerThread entries per thread), each inner
-// product a block sum in a fixed order.  Same formulas and the same alpha_i,
-// c_i and decrement slots.  Block b serves mesh b (meshes that are off or not
-// small return).
-constexpr int kTwoLoopThreads = 1024;
+// Meshes of at most kTwoLoopMaxN unknowns: a cluster of eight CTAs per mesh, which
+// stand for one CTA of 1024 threads (thread v of it is thread v % 128 of CTA v / 128)
+// with kTwoLoopPerThread entries of q each in registers.  A step's warp sums go to
+// every CTA's shared memory, and after one cluster barrier every thread adds the
+// 32 of them in order, as block_sum does for 1024 threads.  The history vectors of
+// the next step are loaded before the exchange.  (One CTA of 1024 threads, the form
+// before, reads all vectors through one SM and exchanges behind two barriers.)
+constexpr int kTwoLoopCluster = 8;
+constexpr int kTwoLoopThreads = 128;       // per CTA
 constexpr int kTwoLoopPerThread = 16;
-constexpr int kTwoLoopMaxN = kTwoLoopThreads * kTwoLoopPerThread;
+constexpr int kTwoLoopMaxN = kTwoLoopCluster * kTwoLoopThreads * kTwoLoopPerThread;
 
-__device__ __forceinline__ double cta_sum_all(double v, double* sm) {
-    __shared__ double total;
-    const double r = block_sum(v, sm);
-    if (threadIdx.x == 0) total = r;
-    __syncthreads();
-    return total;
+__device__ __forceinline__ double cluster_total(double v, double (*sm)[32], int buf, unsigned rank) {
+    const int lane = threadIdx.x & 31, vw = rank * (kTwoLoopThreads / 32) + (threadIdx.x >> 5);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    v = __shfl_sync(0xffffffffu, v, 0);
+    if (lane < kTwoLoopCluster) {
+        const unsigned local = static_cast<unsigned>(__cvta_generic_to_shared(&sm[buf][vw]));
+        unsigned remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(lane));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    double r = 0.0;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) r += sm[buf][w];
+    return r;
 }
 
-// First loop (SplitLBFGS.hpp:152-158): q = g; for i = it-1 .. 0:
-// alpha_i = rho_i <s_i, q>, q -= alpha_i y_i.
-static __global__ void __launch_bounds__(kTwoLoopThreads) k_two_loop_first(const int* on, const MeshCtl* __restrict__ ctl,
-                                                                           VecPools P, const double* __restrict__ rho,
-                                                                           double* __restrict__ q, TwoLoopSlots sl,
-                                                                           double* scal, int stride) {
-    const int m = blockIdx.x;
-    const MeshCtl c = ctl[m];
-    if (!mesh_on(on, m) || !c.small) return;
-    __shared__ double sm[32];
-    const int n = c.v1 - c.v0;
-    const double* g = g_cur(P, c) + c.v0;
-    double* qm = q + c.v0;
-    double* alpha = scal + (size_t)m * stride + sl.alpha;
-    double qr[kTwoLoopPerThread];
+template <bool SECOND>
+static __global__ void __cluster_dims__(kTwoLoopCluster, 1, 1) __launch_bounds__(kTwoLoopThreads)
+    k_two_loop_cluster(const int* on, TwoLoopArgs A) {
+    __shared__ double sm[2][32];   // by step parity: a step's barrier ends the reads of the step before the last
+    const int m = blockIdx.x / kTwoLoopCluster;
+    const unsigned rank = blockIdx.x % kTwoLoopCluster;
+    const MeshCtl c = A.ctl[m];
+    if (!mesh_on(on, m) || !c.small) return;   // the whole cluster
+    const VecPools& P = A.P;
+    const double* rho = A.rho + (size_t)m * kHistSlots;
+    double* scal = A.scal + (size_t)m * A.stride;
+    constexpr int STEP = kTwoLoopCluster * kTwoLoopThreads, PT = kTwoLoopPerThread;
+    const int i0 = c.v0 + (int)(rank * kTwoLoopThreads + threadIdx.x), end = c.v1;
+    const bool lead = rank == 0 && threadIdx.x == 0;
+    double qv[PT], av[PT], bv[PT];
+    auto load = [&](double (&v)[PT], const double* src) {
 #pragma unroll
-    for (int k = 0; k < kTwoLoopPerThread; ++k) {
-        const int i = threadIdx.x + k * kTwoLoopThreads;
-        qr[k] = i < n ? g[i] : 0.0;
-    }
-    for (int h = c.it - 1; h >= 0; --h) {
-        const int hs = hist_slot(c, h, P.M);
-        const double* sp = P.S[hs] + c.v0;
-        const double* yp = P.Y[hs] + c.v0;
+        for (int k = 0; k < PT; ++k) v[k] = i0 + k * STEP < end ? src[i0 + k * STEP] : 0.0;
+    };
+    // every CTA of the cluster is running before any writes to another's shared memory
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if constexpr (!SECOND) {
+        // q = g; for j = it-1 .. 0: alpha_j = rho_j <s_j, q>, q -= alpha_j y_j (SplitLBFGS.hpp:152-158)
+        load(qv, g_cur(P, c));
+        if (c.it > 0) load(bv, P.S[hist_slot(c, c.it - 1, P.M)]);
+        for (int j = c.it - 1; j >= 0; --j) {
+            double d = 0.0;
+#pragma unroll
+            for (int k = 0; k < PT; ++k)
+                if (i0 + k * STEP < end) d += bv[k] * qv[k];
+            load(av, P.Y[hist_slot(c, j, P.M)]);
+            if (j > 0) load(bv, P.S[hist_slot(c, j - 1, P.M)]);
+            const double a = rho[hist_slot(c, j, P.M)] * cluster_total(d, sm, j & 1, rank);
+            if (lead) scal[A.sl.alpha + j] = a;
+#pragma unroll
+            for (int k = 0; k < PT; ++k)
+                if (i0 + k * STEP < end) qv[k] = qv[k] + (-a) * av[k];
+        }
+#pragma unroll
+        for (int k = 0; k < PT; ++k)
+            if (i0 + k * STEP < end) A.q[i0 + k * STEP] = qv[k];
+    } else {
+        // for j = 0 .. it-1: c_j = alpha_j - rho_j <y_j, q>, q += c_j s_j; then dir = <g, q> (SplitLBFGS.hpp:170-173)
+        load(qv, A.q);
+        load(bv, 0 < c.it ? P.Y[hist_slot(c, 0, P.M)] : g_cur(P, c));
+        for (int j = 0; j < c.it; ++j) {
+            double d = 0.0;
+#pragma unroll
+            for (int k = 0; k < PT; ++k)
+                if (i0 + k * STEP < end) d += bv[k] * qv[k];
+            load(av, P.S[hist_slot(c, j, P.M)]);
+            load(bv, j + 1 < c.it ? P.Y[hist_slot(c, j + 1, P.M)] : g_cur(P, c));
+            const double cc = scal[A.sl.alpha + j] + (-rho[hist_slot(c, j, P.M)]) * cluster_total(d, sm, j & 1, rank);
+            if (lead) scal[A.sl.c + j] = cc;
+#pragma unroll
+            for (int k = 0; k < PT; ++k)
+                if (i0 + k * STEP < end) qv[k] = qv[k] + cc * av[k];
+        }
         double d = 0.0;
 #pragma unroll
-        for (int k = 0; k < kTwoLoopPerThread; ++k) {
-            const int i = threadIdx.x + k * kTwoLoopThreads;
-            if (i < n) d += sp[i] * qr[k];
-        }
-        const double a = rho[(size_t)m * kHistSlots + hs] * cta_sum_all(d, sm);
-        if (threadIdx.x == 0) alpha[h] = a;
+        for (int k = 0; k < PT; ++k)
+            if (i0 + k * STEP < end) {
+                if (!A.x) A.q[i0 + k * STEP] = qv[k];
+                d += bv[k] * qv[k];
+            }
+        const double dir = cluster_total(d, sm, c.it & 1, rank);
+        if (lead) scal[A.sl.dir] = dir;
+        if (!A.x) return;
+        const bool restart = !(dir > 0.0);   // bv holds g
 #pragma unroll
-        for (int k = 0; k < kTwoLoopPerThread; ++k) {
-            const int i = threadIdx.x + k * kTwoLoopThreads;
-            if (i < n) qr[k] = qr[k] + (-a) * yp[i];
-        }
+        for (int k = 0; k < PT; ++k)
+            if (i0 + k * STEP < end) x_step(A, P.S[c.stage], i0 + k * STEP, restart ? bv[k] : qv[k]);
     }
-#pragma unroll
-    for (int k = 0; k < kTwoLoopPerThread; ++k) {
-        const int i = threadIdx.x + k * kTwoLoopThreads;
-        if (i < n) qm[i] = qr[k];
-    }
-}
-
-// Second loop (SplitLBFGS.hpp:170-173) after q = A^-1 q: for i = 0 .. it-1:
-// c_i = alpha_i - rho_i <y_i, q>, q += c_i s_i; then dir = <g, q>.
-static __global__ void __launch_bounds__(kTwoLoopThreads) k_two_loop_second(const int* on, const MeshCtl* __restrict__ ctl,
-                                                                            VecPools P, const double* __restrict__ rho,
-                                                                            double* __restrict__ q, TwoLoopSlots sl,
-                                                                            double* scal, int stride) {
-    const int m = blockIdx.x;
-    const MeshCtl c = ctl[m];
-    if (!mesh_on(on, m) || !c.small) return;
-    __shared__ double sm[32];
-    const int n = c.v1 - c.v0;
-    const double* g = g_cur(P, c) + c.v0;
-    double* qm = q + c.v0;
-    double* sc = scal + (size_t)m * stride;
-    double qr[kTwoLoopPerThread];
-#pragma unroll
-    for (int k = 0; k < kTwoLoopPerThread; ++k) {
-        const int i = threadIdx.x + k * kTwoLoopThreads;
-        qr[k] = i < n ? qm[i] : 0.0;
-    }
-    for (int h = 0; h < c.it; ++h) {
-        const int hs = hist_slot(c, h, P.M);
-        const double* sp = P.S[hs] + c.v0;
-        const double* yp = P.Y[hs] + c.v0;
-        double d = 0.0;
-#pragma unroll
-        for (int k = 0; k < kTwoLoopPerThread; ++k) {
-            const int i = threadIdx.x + k * kTwoLoopThreads;
-            if (i < n) d += yp[i] * qr[k];
-        }
-        const double cc = sc[sl.alpha + h] + (-rho[(size_t)m * kHistSlots + hs]) * cta_sum_all(d, sm);
-        if (threadIdx.x == 0) sc[sl.c + h] = cc;
-#pragma unroll
-        for (int k = 0; k < kTwoLoopPerThread; ++k) {
-            const int i = threadIdx.x + k * kTwoLoopThreads;
-            if (i < n) qr[k] = qr[k] + cc * sp[i];
-        }
-    }
-    double d = 0.0;
-#pragma unroll
-    for (int k = 0; k < kTwoLoopPerThread; ++k) {
-        const int i = threadIdx.x + k * kTwoLoopThreads;
-        if (i < n) {
-            qm[i] = qr[k];
-            d += g[i] * qr[k];
-        }
-    }
-    const double dd = cta_sum_all(d, sm);
-    if (threadIdx.x == 0) sc[sl.dir] = dd;
 }
 
 // x <- x - rate * step with step = q, or grad when the mesh's decrement

@@ -472,9 +472,10 @@ void SolverGPU::initialize() {
                                           blocks_for(8 * (int64_t)nf, 256), vec_blocks(3 * (int64_t)nf)}) + 8;
     d_partials_ = static_cast<double*>(dalloc(nblk * 5 * sizeof(double)));
     d_counters_ = static_cast<unsigned*>(dalloc(nm * sizeof(unsigned)));
-    // the cooperative two-loop recursion (one mesh above the one-CTA size):
-    // its grid is what fits on the device at once
-    d_bar_ = static_cast<unsigned*>(dalloc(sizeof(unsigned)));
+    // the cooperative two-loop recursion (meshes above the one-cluster size): the
+    // register form when every vector tile gets its own resident CTA; otherwise a
+    // single mesh walks its tiles with what fits on the device at once, and a batch
+    // takes the per-step launches
     coop_grid_ = 0;
     {
         int dev = 0, coop = 0, sms = 0;
@@ -490,9 +491,10 @@ void SolverGPU::initialize() {
                                  fits((const void*)k_two_loop_grid<true, false>));
         const int cap_reg = std::min(fits((const void*)k_two_loop_grid<false, true>),
                                      fits((const void*)k_two_loop_grid<true, true>));
-        // the register form when every vector tile gets its own resident CTA
         coop_reg_ = tvec_.count <= cap_reg;
-        if (coop && nm == 1) coop_grid_ = std::min(tvec_.count, coop_reg_ ? cap_reg : cap);
+        if (coop && coop_reg_) coop_grid_ = tvec_.count;
+        else if (coop && nm == 1) coop_grid_ = std::min(tvec_.count, cap);
+        if (coop_grid_ > 0) d_slots_ = static_cast<double*>(dalloc(2 * slot_set() * sizeof(double)));
     }
     d_scal_ = static_cast<double*>(dalloc((size_t)nm * kScalStride * sizeof(double)));
     WRAPD_CUDA(cudaMemsetAsync(d_counters_, 0, nm * sizeof(unsigned), st_));
@@ -819,6 +821,7 @@ void SolverGPU::sync_read() {
         const int status = *h_status_;
         *h_status_ = 0;
         chol.reset_solve();
+        slots_stale_ = true;
         WRAPD_CUDA(cudaMemsetAsync(chol.d_status, 0, sizeof(int), st_));
         throw_status(status);
     }
@@ -831,6 +834,7 @@ void SolverGPU::check_status() {
     ctl_pending_ = false;
     if (status != 0) {
         chol.reset_solve();
+        slots_stale_ = true;
         WRAPD_CUDA(cudaMemsetAsync(chol.d_status, 0, sizeof(int), st_));
         throw_status(status);
     }
@@ -1004,26 +1008,30 @@ double SolverGPU::line_search() {
     return -1.0;
 }
 
-// One loop of the two-loop recursion of a single mesh as one cooperative
-// launch (k_two_loop_grid); its barrier counter starts from 0.
-void SolverGPU::two_loop_grid(bool second, const VecPools& P, const TwoLoopSlots& sl) {
-    WRAPD_CUDA(cudaMemsetAsync(d_bar_, 0, sizeof(unsigned), st_));
+// Doubles of one loop's tile sums and totals.
+size_t SolverGPU::slot_set() const { return (size_t)kHistSlots * tvec_.count + (size_t)nm * kTotalSlots; }
+
+// One loop of the two-loop recursion of the meshes of MK_LARGE as one cooperative
+// launch (k_two_loop_grid).
+void SolverGPU::two_loop_grid(bool second, const TwoLoopArgs& args) {
+    if (slots_stale_) {   // the first launch, or a failed one before
+        unset_fill(d_slots_, 2 * (int64_t)slot_set(), st_);
+        slots_stale_ = false;
+    }
     Tiles T = tvec_.view();
-    VecPools Pc = P;
-    TwoLoopSlots slc = sl;
-    const MeshCtl* ctl = d_ctl_;
-    const double* rho = d_rho_;
-    double* q = d_q_;
-    double* partials = d_partials_;
-    unsigned* bar = d_bar_;
+    const int* on = mask(MK_LARGE);
+    TwoLoopArgs a = args;
+    const size_t set = slot_set();
+    double* mine = d_slots_ + (second ? set : 0);
+    double* other = d_slots_ + (second ? 0 : set);
+    int nslots = cfg.lbfgs_m + 1;
     int* status = chol.d_status;
-    double* scal = d_scal_;
-    void* args[] = {&T, &ctl, &Pc, &rho, &q, &slc, &partials, &bar, &status, &scal};
+    void* p[] = {&T, &on, &a, &mine, &other, &nslots, &status};
     const void* fn = coop_reg_ ? (second ? reinterpret_cast<const void*>(&k_two_loop_grid<true, true>)
                                          : reinterpret_cast<const void*>(&k_two_loop_grid<false, true>))
                                : (second ? reinterpret_cast<const void*>(&k_two_loop_grid<true, false>)
                                          : reinterpret_cast<const void*>(&k_two_loop_grid<false, false>));
-    WRAPD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(coop_grid_), dim3(kTwoLoopGridThreads), args, 0, st_));
+    WRAPD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(coop_grid_), dim3(kTwoLoopGridThreads), p, 0, st_));
     kernel_launches++;
 }
 
@@ -1062,14 +1070,17 @@ int SolverGPU::lbfgs_minimize() {
         push_ctl();
         const bool small = any_mask(MK_SMALL), large = any_mask(MK_LARGE);
         const VecPools P = pools();
+        // the second loop's launches step x themselves where each mesh has one and
+        // no line search chooses the rate
+        const bool fused = !cfg.global_ls && !(large && coop_grid_ == 0);
+        const TwoLoopArgs A{d_ctl_, P, d_rho_, d_q_, sl, d_scal_, kScalStride, fused ? d_x_ : nullptr};
         // first loop (newest to oldest): alpha_i = rho_i <s_i, q>, q -= alpha_i y_i
         if (small) {
-            k_two_loop_first<<<nm, kTwoLoopThreads, 0, st_>>>(mask(MK_SMALL), d_ctl_, P, d_rho_, d_q_, sl, d_scal_,
-                                                              kScalStride);
+            k_two_loop_cluster<false><<<nm * kTwoLoopCluster, kTwoLoopThreads, 0, st_>>>(mask(MK_SMALL), A);
             kernel_launches++;
         }
         if (large && coop_grid_ > 0) {
-            two_loop_grid(false, P, sl);
+            two_loop_grid(false, A);
         } else if (large) {
             for (int j = jmax - 1; j >= -1; --j) {
                 k_lbfgs_first<<<tvec_.count, 256, 0, st_>>>(tvec_.view(), mask(MK_LARGE), d_ctl_, P, d_rho_, d_q_, j, sl,
@@ -1084,14 +1095,14 @@ int SolverGPU::lbfgs_minimize() {
         kernel_launches += chol.launches_solve;
         n_solve++;
         mark(3);
+        uv_valid_ = false;   // x moves
         // second loop (oldest to newest): c_i = alpha_i - rho_i <y_i, q>, q += c_i s_i; then dir = <grad, q>
         if (small) {
-            k_two_loop_second<<<nm, kTwoLoopThreads, 0, st_>>>(mask(MK_SMALL), d_ctl_, P, d_rho_, d_q_, sl, d_scal_,
-                                                               kScalStride);
+            k_two_loop_cluster<true><<<nm * kTwoLoopCluster, kTwoLoopThreads, 0, st_>>>(mask(MK_SMALL), A);
             kernel_launches++;
         }
         if (large && coop_grid_ > 0) {
-            two_loop_grid(true, P, sl);
+            two_loop_grid(true, A);
         } else if (large) {
             for (int j = 0; j <= jmax; ++j) {
                 k_lbfgs_second<<<tvec_.count, 256, 0, st_>>>(tvec_.view(), mask(MK_LARGE), d_ctl_, P, d_rho_, d_q_, j,
@@ -1112,11 +1123,13 @@ int SolverGPU::lbfgs_minimize() {
             }
         }
         // x -= rate q (or rate grad on a non-descent direction); s = x_new - x_old
-        uv_valid_ = false;   // x moves
-        k_xupdate<<<tvec_.count, 256, 0, st_>>>(tvec_.view(), mask(MK_LBFGS), d_ctl_, P, d_x_, d_q_, d_scal_, S_DIR,
-                                                kScalStride, rate);
-        WRAPD_LAUNCH_CHECK();
-        kernel_launches++;
+        if (!fused) {
+            uv_valid_ = false;   // (a line search's trials set it)
+            k_xupdate<<<tvec_.count, 256, 0, st_>>>(tvec_.view(), mask(MK_LBFGS), d_ctl_, P, d_x_, d_q_, d_scal_, S_DIR,
+                                                    kScalStride, rate);
+            WRAPD_LAUNCH_CHECK();
+            kernel_launches++;
+        }
         mark(2);
         // gradient at the new x; y = grad_new - grad
         grad_at_x(true, MK_LBFGS);

@@ -167,10 +167,12 @@ private:
     double* d_scal_ = nullptr;             // kScalStride scalars per mesh
     double* h_scal_ = nullptr;
     int* h_status_ = nullptr;    // pinned: the device status word, read with the scalars
-    unsigned* d_bar_ = nullptr;  // grid-barrier counter of the cooperative two-loop recursion
-    int coop_grid_ = 0;          // its CTAs (0: not used -- a batch, or no cooperative launch)
+    double* d_slots_ = nullptr;  // the cooperative two-loop recursion's tile sums, first and second loop
+    size_t slot_set() const;
+    bool slots_stale_ = true;    // they are to be refilled before the next launch
+    int coop_grid_ = 0;          // its CTAs (0: not used)
     bool coop_reg_ = false;      // its register form (one vector tile per CTA)
-    void two_loop_grid(bool second, const VecPools& P, const TwoLoopSlots& sl);
+    void two_loop_grid(bool second, const struct TwoLoopArgs& args);
     // ---- the meshes of the batch: each its own ADMM and L-BFGS state ----
     int nm = 0;
     struct MeshRun {
