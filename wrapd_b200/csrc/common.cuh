@@ -41,34 +41,37 @@ constexpr int kNumSMs = 148;
 
 inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
 
-// Deterministic block sum of one value per thread (blockDim.x a multiple of 32,
-// at most 1024).  Returns the total in thread 0.
-template <typename T>
-__device__ __forceinline__ T block_sum(T v, T* smem) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+// Deterministic block sum (MAX: maximum) of NV values per thread (blockDim.x a
+// multiple of 32, at most 1024): a shuffle tree per warp, then the warps in order.
+// Returns the totals in thread 0.  One pair of barriers for all the values: with
+// one pair for each, the five sums of the local step took ten barriers, a chain
+// that a launch of few CTAs has nothing else to hide behind.
+template <int NV, bool MAX = false>
+__device__ __forceinline__ void block_reduce(double (&v)[NV]) {
+    __shared__ double sm[NV][32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const double w = __shfl_down_sync(0xffffffffu, v[k], o);
+            v[k] = MAX ? fmax(v[k], w) : v[k] + w;
+        }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();   // the previous call's readers of sm are done
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) sm[k][warp] = v[k];
     __syncthreads();
-    if (lane == 0) smem[warp] = v;
-    __syncthreads();
-    T r = 0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r += smem[w];
-    return r;
-}
-
-template <typename T>
-__device__ __forceinline__ T block_max(T v, T* smem) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) smem[warp] = v;
-    __syncthreads();
-    T r = 0;
     if (threadIdx.x == 0) {
-        r = smem[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, smem[w]);
+        double r[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) r[k] = MAX ? sm[k][0] : 0.0 + sm[k][0];
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) r[k] = MAX ? fmax(r[k], sm[k][w]) : r[k] + sm[k][w];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] = r[k];
     }
-    return r;
 }
 
 // ---- bounded waits between CTAs ----------------------------------------------
@@ -130,36 +133,56 @@ inline void unset_fill(double* p, int64_t n, cudaStream_t st) {
     WRAPD_LAUNCH_CHECK();
 }
 
+// One block more has written its partials: returns how many had before it.  The
+// release orders thread 0's own stores only, and the partials are all that the last
+// block reads: the other threads' stores (a gradient's rows) need not be waited for
+// (a fence by every thread before the count: 166 -> 160 us for the gradient's
+// value alone, 786k elements).
+__device__ __forceinline__ unsigned arrive(unsigned* counter) {
+    unsigned n;
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(n) : "l"(counter) : "memory");
+    return n;
+}
+
 // ---- deterministic grid reduction: per-block partials, summed in block order
 // by whichever block finishes last. -------------------------------------------
-// out[k] = total_k, or for k = 0 with an affine epilogue: (base ? *base : 0) + scale * total_0.
-template <int NV, bool MAX = false>
-__device__ __forceinline__ void grid_reduce(const double (&v)[NV], double* partials, unsigned* counter, double* out,
-                                            const double* base = nullptr, double scale = 1.0) {
-    __shared__ double sm[32];
-    __shared__ bool last;
+// The sum of the partials of blocks [b0, b1): thread i takes blocks b0 + i,
+// b0 + i + blockDim.x, ..., then a block sum.
+template <int NV, bool MAX>
+__device__ __forceinline__ void sum_partials(double (&acc)[NV], const double* partials, int b0, int b1) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        const double r = MAX ? block_max(v[k], sm) : block_sum(v[k], sm);
-        if (threadIdx.x == 0) partials[(size_t)blockIdx.x * NV + k] = r;
+    for (int k = 0; k < NV; ++k) acc[k] = MAX ? -1.0e308 : 0.0;
+    for (int b = b0 + (int)threadIdx.x; b < b1; b += blockDim.x)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const double p = __ldcg(partials + (size_t)b * NV + k);
+            acc[k] = MAX ? fmax(acc[k], p) : acc[k] + p;
+        }
+    block_reduce<NV, MAX>(acc);
+}
+
+// out[k] = total_k.
+template <int NV, bool MAX = false>
+__device__ __forceinline__ void grid_reduce(const double (&v)[NV], double* partials, unsigned* counter, double* out) {
+    __shared__ bool last;
+    double acc[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) acc[k] = v[k];
+    block_reduce<NV, MAX>(acc);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) partials[(size_t)blockIdx.x * NV + k] = acc[k];
+        last = arrive(counter) == gridDim.x - 1;
     }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
+    sum_partials<NV, MAX>(acc, partials, 0, (int)gridDim.x);
+    if (threadIdx.x == 0) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double acc = MAX ? -1.0e308 : 0.0;
-        for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-            const double p = __ldcg(partials + (size_t)b * NV + k);
-            acc = MAX ? fmax(acc, p) : acc + p;
-        }
-        const double r = MAX ? block_max(acc, sm) : block_sum(acc, sm);
-        if (threadIdx.x == 0) out[k] = (k == 0 && (base || scale != 1.0)) ? (base ? *base : 0.0) + scale * r : r;
+        for (int k = 0; k < NV; ++k) out[k] = acc[k];
+        *counter = 0u;
     }
-    if (threadIdx.x == 0) *counter = 0u;
 }
 
 // ---- launches over a batch of meshes ----------------------------------------
@@ -200,13 +223,14 @@ __device__ __forceinline__ bool mesh_on(const int* on, int mesh) { return !on ||
 template <int NV, bool MAX = false>
 __device__ __forceinline__ bool seg_reduce(const double (&v)[NV], const Tiles& T, int mesh, double* partials,
                                            unsigned* counters, double (&tot)[NV]) {
-    __shared__ double sm[32];
     __shared__ bool last;
+    double acc[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        const double r = MAX ? block_max(v[k], sm) : block_sum(v[k], sm);
-        if (threadIdx.x == 0) partials[(size_t)blockIdx.x * NV + k] = r;
-    }
+    for (int k = 0; k < NV; ++k) acc[k] = v[k];
+    block_reduce<NV, MAX>(acc);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) partials[(size_t)blockIdx.x * NV + k] = acc[k];
     const int t0 = T.t ? T.tile0[mesh] : 0, t1 = T.t ? T.tile0[mesh + 1] : (int)gridDim.x;
     __threadfence();
     __syncthreads();
@@ -214,15 +238,7 @@ __device__ __forceinline__ bool seg_reduce(const double (&v)[NV], const Tiles& T
     __syncthreads();
     if (!last) return false;
     __threadfence();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double acc = MAX ? -1.0e308 : 0.0;
-        for (int b = t0 + (int)threadIdx.x; b < t1; b += blockDim.x) {
-            const double p = __ldcg(partials + (size_t)b * NV + k);
-            acc = MAX ? fmax(acc, p) : acc + p;
-        }
-        tot[k] = MAX ? block_max(acc, sm) : block_sum(acc, sm);
-    }
+    sum_partials<NV, MAX>(tot, partials, t0, t1);
     if (threadIdx.x == 0) counters[mesh] = 0u;
     return true;
 }

@@ -14,6 +14,10 @@ struct Material {
     int pad;
 };
 
+// Doubles of a gradient row: three and a pad, so that a row is one 32-byte sector,
+// written and read by one instruction.
+constexpr int kRow = 4;
+
 struct ElemView {
     int ne;
     const int4* idx;     // per vertex slot: free vertex (dissection order) or -(pin + 1)
@@ -26,7 +30,8 @@ struct ElemView {
     double* symF;        // 9 x ne, cached V diag(sigma) V^T at the last gradient point
     double* sig;         // 3 x ne, cached singular values at the last gradient point
     double* slast;       // 3 x ne, prox warm start (m_last_sigma)
-    double* gel;         // 12 x ne, per-element gradient rows g(a, r) at [(r + 3a) * ne + e]
+    const int4* row;     // per vertex slot: its row of gel (negative: pinned, no row)
+    double* gel;         // the elements' gradient rows g(a, :), four doubles each (kRow), a vertex's rows together
     const int* mid;      // per element: index into mats (a batch of meshes of several materials), or null
     const Material* mats;
 };

@@ -65,6 +65,15 @@ __device__ __forceinline__ void deformation(const ElemView& E, int e, const doub
     }
 }
 
+// A gradient row (kRow doubles, 32-byte aligned) in one 256-bit access.
+__device__ __forceinline__ void store_row(double* p, double a, double b, double c) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(0.0) : "memory");
+}
+__device__ __forceinline__ void load_row(const double* p, double (&v)[3]) {
+    double pad;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(pad) : "l"(p));
+}
+
 // potential_energy_x per element (src/TetElements.cpp:598-635) from the
 // sign-fixed singular values: NH psi(sigma); ARAP |F - R|^2 / 2 with
 // R = U V^T, i.e. sum (sigma_i - 1)^2 / 2 (k = 1).
@@ -81,9 +90,9 @@ __device__ __forceinline__ double elastic_energy(const Material& m, const double
 // value 0.5 w^2 |symF - P|^2, the potential energy and the inversion count at
 // x (src/TetElements.cpp:444-468, 598-635).  Outputs out[0..2] = value, pe, flips.
 // SEG: a batch (per-mesh sums); a single mesh takes grid_reduce, the same
-// arithmetic.  Register budgets: the single-mesh form compiles to 128 with no
-// occupancy hint; the segmented one and the UV forms below are held to 128
-// (16 warps per SM) by the hint, without which they took 164-168.  Launched
+// arithmetic.  Register budget: all forms are held to 128 (16 warps per SM) by the
+// hint, without which they took 164-168 (the form without U and V, 786k elements:
+// 245 -> 160 us).  Launched
 // on 256-element tiles (two CTAs per SM).
 // UV (single mesh only): 0 = SVD as usual; 1 = also keep U and V of the SVD
 // in uv (U then V, 9 SoA components each); 2 = x is the point of the last
@@ -93,7 +102,7 @@ __device__ __forceinline__ double elastic_energy(const Material& m, const double
 // general form's operations: there the FP32 local step turns a last bit of the
 // gradient into 1e-8 of the positions within twenty iterations.
 template <bool FAST, bool SEG, int UV = 0>
-static __global__ void __launch_bounds__(256, (SEG || UV != 0) ? 2 : 0) k_grad(ElemView E, Tiles T, const int* on, const double* __restrict__ x,
+static __global__ void __launch_bounds__(256, 2) k_grad(ElemView E, Tiles T, const int* on, const double* __restrict__ x,
                                               const double* __restrict__ xfix, Material mat0, int write_gel,
                                               double* partials, unsigned* counters, double* out, int stride,
                                               double* __restrict__ uv = nullptr) {
@@ -178,15 +187,20 @@ static __global__ void __launch_bounds__(256, (SEG || UV != 0) ? 2 : 0) k_grad(E
                     M3(Mm, r, c) = F[r + 3 * c] - v;
                 }
             const double w2t = double(w2);
+            const int4 row = E.row[e];
+            const int rows[4] = {row.x, row.y, row.z, row.w};
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < 4; ++a) {
+                double g[3];
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
                     double v = double(0);
 #pragma unroll
                     for (int c = 0; c < 3; ++c) v += double(E.Di[(size_t)(c + 3 * a) * E.ne + e]) * (w2t * M3(Mm, r, c));
-                    E.gel[(size_t)(r + 3 * a) * E.ne + e] = v;
+                    g[r] = v;
                 }
+                if (rows[a] >= 0) store_row(E.gel + (size_t)kRow * rows[a], g[0], g[1], g[2]);
+            }
         }
     }
     if constexpr (SEG)
@@ -210,18 +224,38 @@ enum { GATHER_START = 0, GATHER_LBFGS = 1, GATHER_PLAIN = 2 };
 // Free-vertex gather of the element gradients (atomic-free; each vertex's
 // incidences, in element order, are added by eight lanes in a fixed order, so
 // the sum is deterministic):
-//   grad[i] = sum over (e, a) incident to i of gel(a, :)[e].
+//   grad[i] = sum over (e, a) incident to i of g_e(a, :).
 // Tiles of 32 free vertices (eight lanes each).  Per mesh: out[0] = |d|^2 with
 // d = grad - gold, out[1] = <s_stage, d> (GATHER_LBFGS), out[2] = |x - xs|^2
 // (the x error of AlgorithmData, at the point the gradient was taken; x may be
 // null).
-static __global__ void __launch_bounds__(256) k_gather(Tiles T, const int* on, int mode, const MeshCtl* __restrict__ ctl,
+// Bound by the rows' traffic on a large mesh and by the chain of loads on a small
+// one.  The rows lie in the order in which they are added here, each a sector of
+// its own: eight lanes read 256 contiguous bytes, no index is read on the way and
+// every byte that is fetched is used.  (With the rows in element order, component
+// by component, each of a vertex's incidences cost three sectors for 24 bytes.)
+// A lane has its first three rows in flight at once (a vertex of the bars' meshes
+// has 24 incidences at most): five CTAs of 48 registers on an SM; two rows and six
+// or eight CTAs, or four and four, are 1 to 15 % slower.  Per launch: 8x8x32
+// 8.1 -> 5.4 us, 16x16x64 11.2 -> 7.8, 32x32x128 57 -> 40, a batch of 16 bars
+// 18.9 -> 14.6.
+constexpr int kGatherAhead = 3;
+static __global__ void __launch_bounds__(256, 5) k_gather(Tiles T, const int* on, int mode, const MeshCtl* __restrict__ ctl,
                                                 VecPools P, double* __restrict__ plain, const int* __restrict__ inc_ptr,
-                                                const int* __restrict__ inc, const double* __restrict__ gel, int ne,
-                                                const double* __restrict__ x, const double* __restrict__ xs,
-                                                double* partials, unsigned* counters, double* out, int stride) {
+                                                const double* __restrict__ gel, const double* __restrict__ x,
+                                                const double* __restrict__ xs, double* partials, unsigned* counters,
+                                                double* out, int stride) {
     const Tile tl = tile_at(T, blockIdx.x);
     if (!mesh_on(on, tl.mesh)) return;
+    // eight lanes per vertex: lane s of the group adds incidences s, s + 8, ...
+    // of the vertex, then the group adds its lanes in a fixed xor tree
+    const int i = tl.first + (threadIdx.x >> 3), sub = threadIdx.x & 7;
+    const bool lead = i < tl.end && sub == 0;
+    int t = 0, t1 = 0;
+    if (i < tl.end) {
+        t = inc_ptr[i] + sub;
+        t1 = inc_ptr[i + 1];
+    }
     double *grad = plain, *ystage = nullptr;
     const double *gold = nullptr, *sstage = nullptr;
     if (mode != GATHER_PLAIN) {
@@ -236,19 +270,24 @@ static __global__ void __launch_bounds__(256) k_gather(Tiles T, const int* on, i
             sstage = P.S[c.stage];
         }
     }
-    // eight lanes per vertex: lane s of the group adds incidences s, s + 8, ...
-    // of the vertex, then the group adds its lanes in a fixed xor tree
-    const int i = tl.first + (threadIdx.x >> 3), sub = threadIdx.x & 7;
-    double red[3] = {0.0, 0.0, 0.0};
+    // the lane's first rows and what the vertex's sum is compared with, all on
+    // their way before the first is used; lane c < 3 of a group has component c
+    double r[kGatherAhead][3];
+#pragma unroll
+    for (int j = 0; j < kGatherAhead; ++j)
+        if (t + 8 * j < t1) load_row(gel + (size_t)kRow * (t + 8 * j), r[j]);
+    const size_t at = 3 * (size_t)i + sub;
+    const bool comp = i < tl.end && sub < 3;
+    const double go = comp && gold ? gold[at] : 0.0;
+    const double ss = comp && sstage ? sstage[at] : 0.0;
+    const double dx = comp && x ? x[at] - xs[at] : 0.0;
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    if (i < tl.end) {
-        for (int t = inc_ptr[i] + sub; t < inc_ptr[i + 1]; t += 8) {
-            const int c = inc[t];
-            const int e = c >> 2, a = c & 3;
-            g0 += gel[(size_t)(0 + 3 * a) * ne + e];
-            g1 += gel[(size_t)(1 + 3 * a) * ne + e];
-            g2 += gel[(size_t)(2 + 3 * a) * ne + e];
-        }
+#pragma unroll
+    for (int j = 0; j < kGatherAhead; ++j)
+        if (t + 8 * j < t1) { g0 += r[j][0]; g1 += r[j][1]; g2 += r[j][2]; }
+    for (t += 8 * kGatherAhead; t < t1; t += 8) {
+        load_row(gel + (size_t)kRow * t, r[0]);
+        g0 += r[0][0]; g1 += r[0][1]; g2 += r[0][2];
     }
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
@@ -256,19 +295,24 @@ static __global__ void __launch_bounds__(256) k_gather(Tiles T, const int* on, i
         g1 += __shfl_xor_sync(0xffffffffu, g1, o);
         g2 += __shfl_xor_sync(0xffffffffu, g2, o);
     }
-    if (i < tl.end && sub == 0) {
-        grad[3 * (size_t)i] = g0; grad[3 * (size_t)i + 1] = g1; grad[3 * (size_t)i + 2] = g2;
-        if (gold) {
-            const double d0 = g0 - gold[3 * (size_t)i], d1 = g1 - gold[3 * (size_t)i + 1], d2 = g2 - gold[3 * (size_t)i + 2];
-            if (ystage) { ystage[3 * (size_t)i] = d0; ystage[3 * (size_t)i + 1] = d1; ystage[3 * (size_t)i + 2] = d2; }
-            red[0] = d0 * d0 + d1 * d1 + d2 * d2;
-            if (sstage) red[1] = sstage[3 * (size_t)i] * d0 + sstage[3 * (size_t)i + 1] * d1 + sstage[3 * (size_t)i + 2] * d2;
+    const double g = sub == 0 ? g0 : sub == 1 ? g1 : g2;   // every lane of the group has the sums
+    const double d = g - go;
+    if (comp) {
+        grad[at] = g;
+        if (ystage) ystage[at] = d;
+    }
+    double red[3] = {0.0, 0.0, 0.0};
+    if (gold) {
+        const double d1 = __shfl_down_sync(0xffffffffu, d, 1), d2 = __shfl_down_sync(0xffffffffu, d, 2);
+        if (lead) red[0] = d * d + d1 * d1 + d2 * d2;
+        if (sstage) {
+            const double s1 = __shfl_down_sync(0xffffffffu, ss, 1), s2 = __shfl_down_sync(0xffffffffu, ss, 2);
+            if (lead) red[1] = ss * d + s1 * d1 + s2 * d2;
         }
-        if (x) {
-            const double e0 = x[3 * (size_t)i] - xs[3 * (size_t)i], e1 = x[3 * (size_t)i + 1] - xs[3 * (size_t)i + 1],
-                         e2 = x[3 * (size_t)i + 2] - xs[3 * (size_t)i + 2];
-            red[2] = e0 * e0 + e1 * e1 + e2 * e2;
-        }
+    }
+    if (x) {
+        const double e1 = __shfl_down_sync(0xffffffffu, dx, 1), e2 = __shfl_down_sync(0xffffffffu, dx, 2);
+        if (lead) red[2] = dx * dx + e1 * e1 + e2 * e2;
     }
     seg_reduce_out<3>(red, T, tl.mesh, partials, counters, out, stride);
 }
@@ -1258,16 +1302,22 @@ static __global__ void __launch_bounds__(128) k_rhs_unaware(ElemView E, const do
         }
     }
     const double w2 = E.w2[e];
+    const int4 row = E.row[e];
+    const int rows[4] = {row.x, row.y, row.z, row.w};
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 4; ++a) {
+        if (rows[a] < 0) continue;
+        double b[3];
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
             double v = 0.0;
 #pragma unroll
             for (int c = 0; c < 3; ++c)
                 v += E.Di[(size_t)(c + 3 * a) * E.ne + e] * (M3(Zm, c, r) - M3(Um, c, r) - Ffix[c + 3 * r]);
-            E.gel[(size_t)(r + 3 * a) * E.ne + e] = w2 * v;
+            b[r] = w2 * v;
         }
+        store_row(E.gel + (size_t)kRow * rows[a], b[0], b[1], b[2]);
+    }
 }
 
 }  // namespace wrapd

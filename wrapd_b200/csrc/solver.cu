@@ -207,6 +207,7 @@ ElemView SolverGPU::view() {
     v.symF = d_symF_;
     v.sig = d_sig_;
     v.slast = d_slast_;
+    v.row = d_row_;
     v.gel = d_gel_;
     v.mid = d_mid_;
     v.mats = d_mats_;
@@ -378,19 +379,21 @@ void SolverGPU::initialize() {
     std::vector<int> A_ptr, A_con;
     assembly_map(S, vinc_ptr, vinc, ptr, adj, A_pos, A_ptr, A_con);
     lap("A pattern (scatter map)");
-    // gather incidences, element order per free vertex
-    std::vector<int> inc_ptr(nf + 1, 0), inc;
+    // gradient rows: a free vertex's incidences together, in element order
+    std::vector<int> inc_ptr(nf + 1, 0);
+    std::vector<int4> row(ne);
     for (int e = 0; e < ne; ++e) {
         const int s[4] = {idx[e].x, idx[e].y, idx[e].z, idx[e].w};
         for (int a = 0; a < 4; ++a) if (s[a] >= 0) inc_ptr[s[a] + 1]++;
     }
     for (int i = 0; i < nf; ++i) inc_ptr[i + 1] += inc_ptr[i];
-    inc.resize(inc_ptr[nf]);
     {
         std::vector<int> fill(inc_ptr.begin(), inc_ptr.end() - 1);
         for (int e = 0; e < ne; ++e) {
             const int s[4] = {idx[e].x, idx[e].y, idx[e].z, idx[e].w};
-            for (int a = 0; a < 4; ++a) if (s[a] >= 0) inc[fill[s[a]]++] = e * 4 + a;
+            int r[4];
+            for (int a = 0; a < 4; ++a) r[a] = s[a] >= 0 ? fill[s[a]]++ : -1;
+            row[e] = make_int4(r[0], r[1], r[2], r[3]);
         }
     }
     lap("gather incidences");
@@ -407,14 +410,14 @@ void SolverGPU::initialize() {
     d_symF_ = static_cast<double*>(dalloc(9 * (size_t)ne * TS));
     d_sig_ = static_cast<double*>(dalloc(3 * (size_t)ne * TS));
     d_slast_ = static_cast<double*>(dalloc(3 * (size_t)ne * TS));
-    d_gel_ = static_cast<double*>(dalloc(12 * (size_t)ne * TS));
+    d_gel_ = static_cast<double*>(dalloc(kRow * (size_t)inc_ptr[nf] * TS));
     WRAPD_CUDA(cudaMemsetAsync(d_U_, 0, 9 * (size_t)ne * TS, st_));
     WRAPD_CUDA(cudaMemsetAsync(d_Z_, 0, 9 * (size_t)ne * TS, st_));
     // m_last_sigma = (1, 1, 1)
     k_fill<<<blocks_for(3 * (int64_t)ne, 256), 256, 0, st_>>>(d_slast_, 3 * (int64_t)ne, 1.0);
     WRAPD_LAUNCH_CHECK();
     d_inc_ptr_ = dupload(inc_ptr);
-    d_inc_ = dupload(inc);
+    d_row_ = dupload(row);
     std::vector<double> xp(3 * (size_t)nf), xs(3 * (size_t)nf), xfix(3 * (size_t)std::max(np, 1));
     for (int i = 0; i < nv; ++i) {
         if (free_of_vert_[i] >= 0) {
@@ -657,8 +660,8 @@ void SolverGPU::grad_at_x(bool write_gel, int mk) {
 }
 
 void SolverGPU::gather(int mode, int mk, bool xerr, double* plain) {
-    k_gather<<<tv32_.count, 256, 0, st_>>>(tv32_.view(), mask(mk), mode, d_ctl_, pools(), plain, d_inc_ptr_, d_inc_,
-                                           d_gel_, ne, xerr ? d_x_ : nullptr, d_xsoln_, d_partials_, d_counters_,
+    k_gather<<<tv32_.count, 256, 0, st_>>>(tv32_.view(), mask(mk), mode, d_ctl_, pools(), plain, d_inc_ptr_,
+                                           d_gel_, xerr ? d_x_ : nullptr, d_xsoln_, d_partials_, d_counters_,
                                            ds(S_GATHER), kScalStride);
     WRAPD_LAUNCH_CHECK();
     kernel_launches++;

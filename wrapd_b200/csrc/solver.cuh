@@ -156,7 +156,8 @@ private:
     double* d_uv_ = nullptr;     // U, V of the last gradient's SVD (one mesh), valid at x while uv_valid_
     bool uv_valid_ = false;
     double *d_Z_ = nullptr, *d_U_ = nullptr, *d_symF_ = nullptr, *d_sig_ = nullptr, *d_slast_ = nullptr, *d_gel_ = nullptr;
-    int *d_inc_ptr_ = nullptr, *d_inc_ = nullptr;
+    int* d_inc_ptr_ = nullptr;
+    int4* d_row_ = nullptr;
     double *d_x_ = nullptr, *d_xfix_ = nullptr, *d_xsoln_ = nullptr, *d_xinit_ = nullptr;
     double* d_q_ = nullptr;
     double* d_G_[3] = {};                  // gradient ring (see VecPools)
