@@ -94,10 +94,10 @@ __device__ __forceinline__ double elastic_energy(const Material& m, const double
 // hint, without which they took 164-168 (the form without U and V, 786k elements:
 // 245 -> 160 us).  Launched
 // on 256-element tiles (two CTAs per SM).
-// UV (single mesh only): 0 = SVD as usual; 1 = also keep U and V of the SVD
-// in uv (U then V, 9 SoA components each); 2 = x is the point of the last
-// UV = 1 launch, so F's SVD is that launch's: sig, U, V and symF are read
-// back instead of recomputed (the same values, so the same results).
+// UV: 0 = SVD as usual; 1 = also keep U and V of the SVD in uv (U then V, 9 SoA
+// components each); 2 = x is the point of the meshes' last UV = 1 launch, so F's
+// SVD is that launch's: sig, U, V and symF are read back instead of recomputed
+// (the same values, so the same results).
 // FAST: the SVD's rotations from rsqrt (svd3_fast).  Mixed precision keeps the
 // general form's operations: there the FP32 local step turns a last bit of the
 // gradient into 1e-8 of the positions within twenty iterations.
@@ -1059,7 +1059,7 @@ static __global__ void __launch_bounds__(256) k_xupdate(Tiles T, const int* on, 
     double* s = P.S[c.stage];
     for (int i = tl.first + (int)threadIdx.x; i < tl.end; i += blockDim.x) {
         const double xo = x[i];
-        const double xn = xo - rate * (restart ? grad[i] : q[i]);
+        const double xn = fma(-rate, restart ? grad[i] : q[i], xo);
         s[i] = xn - xo;
         x[i] = xn;
     }
@@ -1111,11 +1111,12 @@ static __global__ void __launch_bounds__(256) k_ls_gmax(int n, const double* __r
     grid_reduce<1, true>(red, partials, counter, out);
 }
 
-// Trial point of the line search: xt = x + alpha * p with p = -step.
+// Trial point of the line search: xt = x + alpha * p with p = -step; the same
+// operation as k_xupdate's, so that an accepted step arrives at the trial's bits.
 static __global__ void __launch_bounds__(256) k_ls_trial(int n, double* __restrict__ xt, const double* __restrict__ x,
                                                   const double* __restrict__ step, double alpha) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        xt[i] = x[i] + alpha * -step[i];
+        xt[i] = fma(-alpha, step[i], x[i]);
 }
 
 // ---- ARAP local step (rotation-aware) ------------------------------------------

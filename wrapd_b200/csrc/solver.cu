@@ -402,9 +402,6 @@ void SolverGPU::initialize() {
     const size_t TS = sizeof(double);
     d_idx_ = dupload(idx);
     d_w2c_ = static_cast<double*>(dalloc(ne * sizeof(double)));
-    // U and V of the last gradient's SVD (single mesh): 18 doubles per element
-    d_uv_ = meshes_.size() == 1 ? static_cast<double*>(dalloc((size_t)18 * ne * sizeof(double))) : nullptr;
-    uv_valid_ = false;
     d_Z_ = static_cast<double*>(dalloc(9 * (size_t)ne * TS));
     d_U_ = static_cast<double*>(dalloc(9 * (size_t)ne * TS));
     d_symF_ = static_cast<double*>(dalloc(9 * (size_t)ne * TS));
@@ -554,6 +551,16 @@ void SolverGPU::initialize() {
     factor();
     for (MeshRun& R : runs_) R.ctl.k = 0;
     check_status();
+    // U and V of the last gradient's SVD: 18 doubles per element, allocated last, and
+    // done without where they would not leave autotune_local's copy of the state room
+    uv_ok_.assign(nm, 0);
+    d_uv_ = nullptr;
+    if (cfg.rot_aware) {
+        size_t room = 0, total = 0;
+        WRAPD_CUDA(cudaMemGetInfo(&room, &total));
+        if (room > (size_t)(18 + 24) * ne * sizeof(double))
+            d_uv_ = static_cast<double*>(dalloc((size_t)18 * ne * sizeof(double)));
+    }
     lap("first factorization (graph capture + run)");
     initialized_ = true;
     runtime_ms[0] += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -637,27 +644,41 @@ const Logs& SolverGPU::mesh_logs(int m) const {
         kernel_launches++;                                                                  \
     } while (0)
 
-// The global gradient at x.  A single mesh in the rotation-aware global step
-// without line search keeps the SVD factors of its last gradient (k_grad
-// UV = 1); the first gradient of the next ADMM iteration is taken at the same
-// x (the local step changes only Z and U), so it reads them back (UV = 2)
-// instead of redoing the per-element SVD.  uv_valid_ is cleared wherever x
-// changes.  256-element tiles (786k bar: 1.095 -> 1.077 ms per global step
-// against 128; 3.9M bar: 5.09 -> 4.95 ms), in a batch too, so that a mesh's
-// sums are added in the same order as when it is solved alone.
-void SolverGPU::grad_at_x(bool write_gel, int mk) {
-    const bool keep = nm == 1 && d_uv_ && write_gel && cfg.rot_aware && !cfg.global_ls;
+// One launch of the gradient kernel at x for the meshes of a mask: the gradient of
+// the solve (slot S_GRAD, x = d_x_) or a line-search trial's value (S_LSV).  In the
+// rotation-aware global step both keep the SVD's factors (k_grad UV = 1), and a
+// gradient at a point whose factors are held reads them back (UV = 2) instead of
+// redoing the SVD of every element: the first gradient of an ADMM iteration (the
+// local step changes only Z and U) and the one at an accepted trial.  uv_ok_ says
+// which meshes' factors are those of their x; it is cleared wherever x moves.
+// Per launch, 16 bars in a mixed-precision batch: 101 us with the SVD, 51 without; per
+// solve of 16x16x64 with the line search, 57 of 96 launches read back: 17.6 -> 16.5 ms.
+// 256-element tiles (786k bar: 1.095 -> 1.077 ms per global step against 128; 3.9M
+// bar: 5.09 -> 4.95 ms), in a batch too, so that a mesh's sums are added in the same
+// order as when it is solved alone.
+void SolverGPU::grad_at(const double* x, bool write_gel, int mk, int slot) {
+    const bool keep = d_uv_ && (write_gel || slot == S_LSV);
+    bool held = keep && slot == S_GRAD;
+    for (int m = 0; m < nm; ++m)
+        if (h_masks_[(size_t)mk * nm + m]) {
+            held = held && uv_ok_[m];
+            uv_ok_[m] = keep && slot == S_GRAD;
+        }
     // FP64 solves take the SVD's fast form, mixed precision the general one (see k_grad)
-    const auto fn = nm > 1 ? (fp32() ? k_grad<false, true, 0> : k_grad<true, true, 0>)
-                    : !keep ? (fp32() ? k_grad<false, false, 0> : k_grad<true, false, 0>)
-                    : uv_valid_ ? k_grad<false, false, 2>
-                                : (fp32() ? k_grad<false, false, 1> : k_grad<true, false, 1>);
-    fn<<<te256_.count, 256, 0, st_>>>(view(), te256_.view(), mask(mk), d_x_, d_xfix_, mat_, write_gel ? 1 : 0, d_partials_,
-                                      d_counters_, ds(S_GRAD), kScalStride, keep ? d_uv_ : nullptr);
+    const bool f = !fp32();
+    const auto fn = nm > 1 ? (held ? k_grad<false, true, 2>
+                              : keep ? (f ? k_grad<true, true, 1> : k_grad<false, true, 1>)
+                                     : (f ? k_grad<true, true, 0> : k_grad<false, true, 0>))
+                           : (held ? k_grad<false, false, 2>
+                              : keep ? (f ? k_grad<true, false, 1> : k_grad<false, false, 1>)
+                                     : (f ? k_grad<true, false, 0> : k_grad<false, false, 0>));
+    fn<<<te256_.count, 256, 0, st_>>>(view(), te256_.view(), mask(mk), x, d_xfix_, mat_, write_gel ? 1 : 0, d_partials_,
+                                      d_counters_, ds(slot), kScalStride, d_uv_);
     WRAPD_LAUNCH_CHECK();
     kernel_launches++;
-    uv_valid_ = keep;
 }
+
+void SolverGPU::grad_at_x(bool write_gel, int mk) { grad_at(d_x_, write_gel, mk, S_GRAD); }
 
 void SolverGPU::gather(int mode, int mk, bool xerr, double* plain) {
     k_gather<<<tv32_.count, 256, 0, st_>>>(tv32_.view(), mask(mk), mode, d_ctl_, pools(), plain, d_inc_ptr_,
@@ -743,7 +764,6 @@ void SolverGPU::global_step_unaware() {
     kernel_launches += chol.launches_solve;
     n_solve++;
     mark(3);
-    uv_valid_ = false;
     WRAPD_CUDA(cudaMemcpyAsync(d_x_, d_q_, 3 * (size_t)nf * sizeof(double), cudaMemcpyDeviceToDevice, st_));
     // update_defo_cache(x, true): singular values for the energy and flips
     grad_at_x(false, MK_ALL);
@@ -925,7 +945,7 @@ void SolverGPU::begin_solve() {
     }
     push_ctl();
     // setup_solve (src/ADMM.cpp:89-107): X = X_init, defo cache, dual variables
-    uv_valid_ = false;
+    std::fill(uv_ok_.begin(), uv_ok_.end(), 0);
     WRAPD_CUDA(cudaMemcpyAsync(d_x_, d_xinit_, 3 * (size_t)nf * sizeof(double), cudaMemcpyDeviceToDevice, st_));
     grad_at_x(false, MK_ALL);
     if (cfg.rot_aware) {
@@ -972,8 +992,8 @@ void SolverGPU::begin_solve() {
 // Armijo decrease 1e-4, step factor 0.7; a direction of norm <= machine
 // epsilon returns 1e-4.  fx0 is the AL value of the last gradient evaluation,
 // which was at x.  Each trial value is one gradient-kernel pass (no gradient
-// rows) at x + alpha p into the stage vector; the element cache it leaves is
-// refreshed by the gradient at the accepted x.  On a non-descent restart the
+// rows) at x + alpha p into the stage vector; the element cache and the SVD's
+// factors it leaves are the accepted point's.  On a non-descent restart the
 // history reset of SplitLBFGS.hpp:189-194 is applied here, before the search.
 double SolverGPU::line_search() {
     const int n = 3 * nf, vb = vec_blocks(n);
@@ -1001,11 +1021,13 @@ double SolverGPU::line_search() {
         k_ls_trial<<<vb, 256, 0, st_>>>(n, trial, d_x_, step, alpha);
         WRAPD_LAUNCH_CHECK();
         kernel_launches++;
-        WRAPD_ELEM_LAUNCH((fp32() ? k_grad<false, false, 0> : k_grad<true, false, 0>), te256_, 256, mask(MK_ALL), trial, d_xfix_, mat_, 0, d_partials_,
-                          d_counters_, ds(S_LSV), kScalStride, nullptr);   // one mesh (line search: single meshes only)
+        grad_at(trial, false, MK_ALL, S_LSV);   // one mesh (line search: single meshes only)
         sync_read();
         const double fxa = hs(0, S_LSV);
-        if (fxa <= fx0 + alpha * decrease * gtp) return alpha;
+        if (fxa <= fx0 + alpha * decrease * gtp) {
+            uv_ok_[0] = d_uv_ != nullptr;   // the step goes to the trial point, bit for bit
+            return alpha;
+        }
         alpha *= tau;
     }
     return -1.0;
@@ -1098,7 +1120,8 @@ int SolverGPU::lbfgs_minimize() {
         kernel_launches += chol.launches_solve;
         n_solve++;
         mark(3);
-        uv_valid_ = false;   // x moves
+        for (int m = 0; m < nm; ++m)
+            if (runs_[m].in_loop) uv_ok_[m] = 0;   // x moves
         // second loop (oldest to newest): c_i = alpha_i - rho_i <y_i, q>, q += c_i s_i; then dir = <grad, q>
         if (small) {
             k_two_loop_cluster<true><<<nm * kTwoLoopCluster, kTwoLoopThreads, 0, st_>>>(mask(MK_SMALL), A);
@@ -1127,7 +1150,6 @@ int SolverGPU::lbfgs_minimize() {
         }
         // x -= rate q (or rate grad on a non-descent direction); s = x_new - x_old
         if (!fused) {
-            uv_valid_ = false;   // (a line search's trials set it)
             k_xupdate<<<tvec_.count, 256, 0, st_>>>(tvec_.view(), mask(MK_LBFGS), d_ctl_, P, d_x_, d_q_, d_scal_, S_DIR,
                                                     kScalStride, rate);
             WRAPD_LAUNCH_CHECK();
@@ -1473,7 +1495,7 @@ void SolverGPU::set_state(const std::string& name, const double* in, int64_t n) 
         std::vector<double> xp(3 * (size_t)nf);
         for (int i = 0; i < nf; ++i)
             for (int c = 0; c < 3; ++c) xp[3 * (size_t)iperm_[i] + c] = in[3 * (size_t)i + c];
-        uv_valid_ = false;
+        std::fill(uv_ok_.begin(), uv_ok_.end(), 0);
         WRAPD_CUDA(cudaMemcpyAsync(d_x_, xp.data(), xp.size() * 8, cudaMemcpyHostToDevice, st_));
         WRAPD_CUDA(cudaStreamSynchronize(st_));
         ctl_pending_ = false;

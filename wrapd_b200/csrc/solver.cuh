@@ -101,6 +101,7 @@ private:
     std::vector<cudaEvent_t> event_pool_;
     size_t event_next_ = 0;
     void check_status();
+    void grad_at(const double* x, bool write_gel, int mask, int slot);
     void grad_at_x(bool write_gel, int mask);
     void gather(int mode, int mask, bool xerr, double* plain = nullptr);
     void local_step_unaware(int cand_mode, bool fp32_compute);
@@ -153,8 +154,8 @@ private:
     std::vector<void*> allocs_;
     int4* d_idx_ = nullptr;
     double *d_Di_ = nullptr, *d_vol_ = nullptr, *d_w2_ = nullptr, *d_w2c_ = nullptr;
-    double* d_uv_ = nullptr;     // U, V of the last gradient's SVD (one mesh), valid at x while uv_valid_
-    bool uv_valid_ = false;
+    double* d_uv_ = nullptr;     // U, V of the last gradient's SVD, or null
+    std::vector<char> uv_ok_;    // per mesh: d_uv_, symF and sig are those at its x
     double *d_Z_ = nullptr, *d_U_ = nullptr, *d_symF_ = nullptr, *d_sig_ = nullptr, *d_slast_ = nullptr, *d_gel_ = nullptr;
     int* d_inc_ptr_ = nullptr;
     int4* d_row_ = nullptr;
