@@ -57,6 +57,13 @@ struct MeshCtl {
     int small;     // the two-loop runs in one CTA (3 x free vertices <= kTwoLoopMaxN)
     int v0, v1;    // the mesh's range in the n x 3 vectors, in doubles
 };
+// Where a launch hands a mesh's scalars to the host (publish_mesh).
+struct HostWords {
+    const double* scal;        // the meshes' scalar blocks
+    const int* status;
+    unsigned long long* host;  // kHostSlots + 1 words per mesh in pinned memory, or null
+    int stride;                // doubles of a scalar block
+};
 // Slots of the two-loop recursion's scalars in a mesh's scalar block.
 struct TwoLoopSlots {
     int alpha, c, dir;    // offsets in a mesh's scalar block

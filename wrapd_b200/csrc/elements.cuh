@@ -215,6 +215,17 @@ __device__ __forceinline__ double* g_cur(const VecPools& P, const MeshCtl& c) { 
 __device__ __forceinline__ double* g_new(const VecPools& P, const MeshCtl& c) { return P.G[(c.grot + 1) % 3]; }
 __device__ __forceinline__ double* g_old(const VecPools& P, const MeshCtl& c) { return P.G[(c.grot + 2) % 3]; }
 
+// A mesh's scalars and the status word to pinned host memory, a store each, with no
+// order among them: the host polls every word.
+constexpr int kHostLow = 20, kHostHigh = 85, kHostSlots = 26;   // slots [0, 20) and from 85 on
+__device__ __forceinline__ void publish_mesh(const HostWords& P, int mesh) {
+    volatile unsigned long long* w = P.host + (size_t)mesh * (kHostSlots + 1);
+    const double* s = P.scal + (size_t)mesh * P.stride;
+    for (int k = threadIdx.x; k <= kHostSlots; k += blockDim.x)
+        w[k] = k == kHostSlots ? (unsigned long long)*reinterpret_cast<const volatile unsigned*>(P.status)
+                               : (unsigned long long)__double_as_longlong(__ldcg(s + (k < kHostLow ? k : k - kHostLow + kHostHigh)));
+}
+
 // Gather modes: at the start of an ADMM iteration the gradient goes to the
 // mesh's cur buffer and is compared with old (|grad - grad_old|^2, the early
 // return of SplitLBFGS.hpp:138-142); inside the L-BFGS loop it goes to new,
@@ -228,7 +239,8 @@ enum { GATHER_START = 0, GATHER_LBFGS = 1, GATHER_PLAIN = 2 };
 // Tiles of 32 free vertices (eight lanes each).  Per mesh: out[0] = |d|^2 with
 // d = grad - gold, out[1] = <s_stage, d> (GATHER_LBFGS), out[2] = |x - xs|^2
 // (the x error of AlgorithmData, at the point the gradient was taken; x may be
-// null).
+// null).  The last block of a mesh then hands the mesh's scalars to the host (pub):
+// this is the last launch before the host decides.
 // Bound by the rows' traffic on a large mesh and by the chain of loads on a small
 // one.  The rows lie in the order in which they are added here, each a sector of
 // its own: eight lanes read 256 contiguous bytes, no index is read on the way and
@@ -244,7 +256,7 @@ static __global__ void __launch_bounds__(256, 5) k_gather(Tiles T, const int* on
                                                 VecPools P, double* __restrict__ plain, const int* __restrict__ inc_ptr,
                                                 const double* __restrict__ gel, const double* __restrict__ x,
                                                 const double* __restrict__ xs, double* partials, unsigned* counters,
-                                                double* out, int stride) {
+                                                double* out, int stride, HostWords pub) {
     const Tile tl = tile_at(T, blockIdx.x);
     if (!mesh_on(on, tl.mesh)) return;
     // eight lanes per vertex: lane s of the group adds incidences s, s + 8, ...
@@ -314,7 +326,14 @@ static __global__ void __launch_bounds__(256, 5) k_gather(Tiles T, const int* on
         const double e1 = __shfl_down_sync(0xffffffffu, dx, 1), e2 = __shfl_down_sync(0xffffffffu, dx, 2);
         if (lead) red[2] = dx * dx + e1 * e1 + e2 * e2;
     }
-    seg_reduce_out<3>(red, T, tl.mesh, partials, counters, out, stride);
+    double tot[3];
+    if (!seg_reduce<3>(red, T, tl.mesh, partials, counters, tot)) return;
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) out[(size_t)tl.mesh * stride + k] = tot[k];
+    if (!pub.host) return;
+    __syncthreads();
+    publish_mesh(pub, tl.mesh);
 }
 
 // ---- local step ---------------------------------------------------------------

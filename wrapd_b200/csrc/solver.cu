@@ -16,7 +16,7 @@ namespace wrapd {
 
 namespace {
 
-// Slots of the device scalar block (one pinned download per sync point).
+// Slots of the device scalar block (k_publish hands them to the host).
 enum : int {
     S_GRAD = 0,      // value, pe, flips
     S_GATHER = 4,    // |grad - gold|^2, <s, y>, |x - x_soln|^2
@@ -26,7 +26,7 @@ enum : int {
     S_DIR = 16,      // L-BFGS decrement
     S_XERR = 18,     // |x - x_soln|^2
     S_DUMMY = 19,
-    S_ALPHA = 20,    // alpha_i, up to 32 entries
+    S_ALPHA = 20,    // alpha_i, up to 32 entries (these two: on the device only)
     S_C = 52,        // alpha_i - beta_i, up to 32 entries
     S_ONE = 84,      // constant 1 (a device-side coefficient)
     S_LSN = 85,      // line search: <q, q>, <grad, grad>
@@ -60,6 +60,13 @@ int blocks_for(int64_t n, int threads) { return std::max(1, ceil_div(n, threads)
 
 // Vector kernels use a fixed grid of 2 CTAs per SM (grid-stride loops).
 int vec_blocks(int64_t n) { return std::max(1, std::min(2 * kNumSMs, ceil_div(n, 256))); }
+
+// The slots of a mesh that the host reads, [0, kHostLow) and [kHostHigh, S_COUNT)
+// (elements.cuh), are all but S_ALPHA, S_C and S_ONE.
+static_assert(kHostLow == S_ALPHA && kHostHigh == S_LSN && kHostSlots == kHostLow + S_COUNT - kHostHigh, "published slots");
+
+// Every mesh's scalars to the host, where no gather has taken them along.
+__global__ void __launch_bounds__(32) k_publish(HostWords P) { publish_mesh(P, blockIdx.x); }
 
 __global__ void k_fill(double* __restrict__ p, int64_t n, double v) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -171,8 +178,7 @@ SolverGPU::~SolverGPU() {
     if (d_net_img_) cudaFree(d_net_img_);
     for (auto& set : evs_)
         for (auto& e : set) if (e) cudaEventDestroy(e);
-    if (h_scal_) cudaFreeHost(h_scal_);
-    if (h_status_) cudaFreeHost(h_status_);
+    if (h_words_) cudaFreeHost(h_words_);
     if (h_ctl_block_) cudaFreeHost(h_ctl_block_);
     if (st_) cudaStreamDestroy(st_);
 }
@@ -499,10 +505,9 @@ void SolverGPU::initialize() {
     d_scal_ = static_cast<double*>(dalloc((size_t)nm * kScalStride * sizeof(double)));
     WRAPD_CUDA(cudaMemsetAsync(d_counters_, 0, nm * sizeof(unsigned), st_));
     WRAPD_CUDA(cudaMemsetAsync(d_scal_, 0, (size_t)nm * kScalStride * sizeof(double), st_));
-    WRAPD_CUDA(cudaMallocHost(&h_scal_, (size_t)nm * kScalStride * sizeof(double)));
-    std::memset(h_scal_, 0, (size_t)nm * kScalStride * sizeof(double));
-    WRAPD_CUDA(cudaMallocHost(&h_status_, sizeof(int)));
-    *h_status_ = 0;
+    WRAPD_CUDA(cudaMallocHost(&h_words_, (size_t)nm * (kHostSlots + 1) * sizeof(*h_words_)));
+    h_scal_.assign((size_t)nm * kScalStride, 0.0);
+    publishing_.assign(nm, 0);
     {
         static const double one = 1.0;
         WRAPD_CUDA(cudaMemcpyAsync(d_scal_ + S_ONE, &one, sizeof(double), cudaMemcpyHostToDevice, st_));
@@ -681,9 +686,12 @@ void SolverGPU::grad_at(const double* x, bool write_gel, int mk, int slot) {
 void SolverGPU::grad_at_x(bool write_gel, int mk) { grad_at(d_x_, write_gel, mk, S_GRAD); }
 
 void SolverGPU::gather(int mode, int mk, bool xerr, double* plain) {
+    // a rotation-aware gather is the last launch before a synchronisation
+    HostWords P{};
+    if (mode != GATHER_PLAIN) P = prepare_publish(mk);
     k_gather<<<tv32_.count, 256, 0, st_>>>(tv32_.view(), mask(mk), mode, d_ctl_, pools(), plain, d_inc_ptr_,
                                            d_gel_, xerr ? d_x_ : nullptr, d_xsoln_, d_partials_, d_counters_,
-                                           ds(S_GATHER), kScalStride);
+                                           ds(S_GATHER), kScalStride, P);
     WRAPD_LAUNCH_CHECK();
     kernel_launches++;
 }
@@ -833,34 +841,92 @@ static void throw_status(int status) {
     throw CudaError(status, "factorization of D^T W D hit a non-positive pivot");
 }
 
-void SolverGPU::sync_read() {
-    WRAPD_CUDA(cudaMemcpyAsync(h_scal_, d_scal_, (size_t)nm * kScalStride * sizeof(double), cudaMemcpyDeviceToHost, st_));
-    WRAPD_CUDA(cudaMemcpyAsync(h_status_, chol.d_status, sizeof(int), cudaMemcpyDeviceToHost, st_));
-    WRAPD_CUDA(cudaStreamSynchronize(st_));
+// Hand-over of the scalars and the status word to the host.  A launch writes them to
+// words in pinned memory that the host has unset (kUnset, which no result equals) and
+// polls: no download, no flag, no fence, and no wait for the end of the stream's
+// work.  prepare_publish unsets the words of the meshes of a mask for the launch that
+// follows; await_publish waits for them.
+HostWords SolverGPU::prepare_publish(int mk) {
+    // (a hand-over that an error kept from being awaited)
+    if (publish_pending_) WRAPD_CUDA(cudaStreamSynchronize(st_));
+    publish_pending_ = true;
+    for (int m = 0; m < nm; ++m) {
+        publishing_[m] = h_masks_[(size_t)mk * nm + m] != 0;
+        if (publishing_[m]) std::fill_n(h_words_ + (size_t)m * (kHostSlots + 1), kHostSlots + 1, kUnset);
+    }
+    unsigned long long* d = nullptr;
+    WRAPD_CUDA(cudaHostGetDevicePointer(&d, h_words_, 0));
+    return HostWords{d_scal_, chol.d_status, d, kScalStride};
+}
+
+// The host looks at the words for a millisecond and then waits for the stream as any
+// caller would; an error of the stream ends the wait at once.  The stream's work up
+// to the publishing launch is done when this returns.  (Per synchronisation, two
+// downloads and a stream synchronisation before: 3 us each for the downloads and
+// some 5 us to notice the end.  8x8x32, a solve of 121 of them: 10.4 ms; handed over
+// by a launch of its own with a flag behind a fence, the ratio read along, 9.1; by the
+// gather, 8.6.)
+void SolverGPU::await_publish() {
+    const auto t0 = std::chrono::steady_clock::now();
+    const volatile unsigned long long* words = h_words_;
+    bool done = false;   // the stream's work has ended: every word is there
+    status_ = 0;
+    for (int m = 0; m < nm; ++m) {
+        if (!publishing_[m]) continue;
+        for (int k = 0; k <= kHostSlots; ++k) {
+            const size_t at = (size_t)m * (kHostSlots + 1) + k;
+            for (int i = 1; !done && words[at] == kUnset; ++i) {
+                if (i % 4096) continue;
+                const cudaError_t e = cudaStreamQuery(st_);
+                if (e != cudaErrorNotReady) WRAPD_CUDA(e);
+                if (e == cudaSuccess || std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(1)) {
+                    WRAPD_CUDA(cudaStreamSynchronize(st_));
+                    done = true;
+                }
+            }
+            const unsigned long long w = words[at];
+            if (k == kHostSlots) {
+                if (w != 0) status_ = static_cast<int>(w);
+            } else {
+                std::memcpy(&hs(m, k < kHostLow ? k : k - kHostLow + kHostHigh), &w, sizeof(w));
+            }
+        }
+    }
+    publish_pending_ = false;
     ctl_pending_ = false;
+}
+
+// Waits for the scalars that the last gather hands over, or hands all over now.
+void SolverGPU::publish() {
+    if (!publish_pending_) {
+        const HostWords P = prepare_publish(MK_ALL);
+        k_publish<<<nm, 32, 0, st_>>>(P);
+        WRAPD_LAUNCH_CHECK();
+        kernel_launches++;
+    }
+    await_publish();
+}
+
+void SolverGPU::sync_read() {
+    publish();
     n_sync++;
     mark(5);
-    if (*h_status_ != 0) {
-        const int status = *h_status_;
-        *h_status_ = 0;
-        chol.reset_solve();
-        slots_stale_ = true;
-        WRAPD_CUDA(cudaMemsetAsync(chol.d_status, 0, sizeof(int), st_));
-        throw_status(status);
-    }
+    raise_status();
 }
 
 void SolverGPU::check_status() {
-    int status = 0;
-    WRAPD_CUDA(cudaMemcpyAsync(&status, chol.d_status, sizeof(int), cudaMemcpyDeviceToHost, st_));
-    WRAPD_CUDA(cudaStreamSynchronize(st_));
-    ctl_pending_ = false;
-    if (status != 0) {
-        chol.reset_solve();
-        slots_stale_ = true;
-        WRAPD_CUDA(cudaMemsetAsync(chol.d_status, 0, sizeof(int), st_));
-        throw_status(status);
-    }
+    publish();
+    raise_status();
+}
+
+void SolverGPU::raise_status() {
+    const int status = status_;
+    if (status == 0) return;
+    status_ = 0;
+    chol.reset_solve();
+    slots_stale_ = true;
+    WRAPD_CUDA(cudaMemsetAsync(chol.d_status, 0, sizeof(int), st_));
+    throw_status(status);
 }
 
 // |x - x_soln|^2 per mesh (AlgorithmData::update_per_iter_data,
@@ -1227,6 +1293,15 @@ void SolverGPU::union_logs(int k) {
     }
 }
 
+// The largest change of weight of the gamma rule, per mesh.  The local step has
+// written the candidate weights and the global step touches neither they nor the
+// weights, so this follows the local step at once and the host reads the result
+// with the global step's scalars instead of waiting for it by itself.
+void SolverGPU::ratio() {
+    if (!cfg.reweighting || cfg.rw_every > 0) return;
+    WRAPD_ELEM_LAUNCH(k_ratio, te256_, 256, mask(MK_ADMM), d_partials_, d_counters_, ds(S_RATIO), kScalStride);
+}
+
 int SolverGPU::iterate(int n, bool* conv) {
     if (!solving_) throw CudaError(WRAPD_E_STATE, "iterate before begin_solve");
     int done = 0;
@@ -1265,6 +1340,7 @@ int SolverGPU::iterate(int n, bool* conv) {
             // ---- local step: polar_update (src/TetElements.cpp:256-356) ----
             local_step(cand);
             if (cfg.reweighting) count_++;
+            ratio();
             mark(0);
             WRAPD_CUDA(cudaEventRecord(ev_[1], st_));
             // ---- global step: RotAwareGS::global_step (src/GlobalStepBehavior.hpp:246-258) ----
@@ -1277,7 +1353,7 @@ int SolverGPU::iterate(int n, bool* conv) {
             gather(GATHER_START, MK_ADMM, true);
             mark(1);
             sync_read();
-            settle_timing(false);   // the previous iteration's events are behind this synchronisation
+            settle_timing();   // the previous iteration's events are behind this synchronisation
             for (int m = 0; m < nm; ++m) {
                 MeshRun& R = runs_[m];
                 R.in_loop = false;
@@ -1300,6 +1376,7 @@ int SolverGPU::iterate(int n, bool* conv) {
             // ---- local_update: TetElements::update (src/TetElements.cpp:193-254), single mesh ----
             local_step_unaware(cand, fp32() && !runs_[0].fp64_phase);
             if (cfg.reweighting) count_++;
+            ratio();
             mark(0);
             WRAPD_CUDA(cudaEventRecord(ev_[1], st_));
             // ---- UnawareGS::global_step (src/GlobalStepBehavior.hpp:162-180): x = A^-1 b ----
@@ -1319,9 +1396,6 @@ int SolverGPU::iterate(int n, bool* conv) {
             if (cfg.rw_every > 0) {
                 for (int m = 0; m < nm; ++m) rw[m] = act[m] && ((k + 1) % cfg.rw_every) == 0;
             } else {
-                WRAPD_ELEM_LAUNCH(k_ratio, te256_, 256, mask(MK_ADMM), d_partials_, d_counters_, ds(S_RATIO),
-                                  kScalStride);
-                sync_read();
                 for (int m = 0; m < nm; ++m) rw[m] = act[m] && hs(m, S_RATIO) > cfg.gamma;
             }
             for (int m = 0; m < nm; ++m) {
@@ -1378,24 +1452,23 @@ int SolverGPU::iterate(int n, bool* conv) {
         if (nm > 1) union_logs(k + 1);
         // phase times: read once a later synchronisation has passed the events
         pend_ = PendingTiming{true, k, ev_};
-        if (profiling || any_rw) settle_timing(false);          // a synchronisation passed ev_[3]
-        else if (!cfg.rot_aware) settle_timing(true);          // its last one came before ev_[2]
+        if (profiling || any_rw || !cfg.rot_aware) settle_timing();
         iter = k + 1;
         done++;
         converged_ = true;
         for (const MeshRun& R : runs_) converged_ = converged_ && R.converged;
     }
-    settle_timing(true);
+    settle_timing();
     *conv = converged_;
     return done;
 }
 
 // Adds a finished iteration's phase times (CUDA events) to the runtime and its
-// accumulated-time log entries.  wait = false: a host synchronisation of the
-// stream has already passed the events.
-void SolverGPU::settle_timing(bool wait) {
+// accumulated-time log entries; waits for them where no synchronisation of the
+// stream has passed them yet.
+void SolverGPU::settle_timing() {
     if (!pend_.on) return;
-    if (wait) WRAPD_CUDA(cudaEventSynchronize(pend_.ev[3]));
+    WRAPD_CUDA(cudaEventSynchronize(pend_.ev[3]));
     float ml = 0.f, mg = 0.f, mr = 0.f;
     WRAPD_CUDA(cudaEventElapsedTime(&ml, pend_.ev[0], pend_.ev[1]));
     WRAPD_CUDA(cudaEventElapsedTime(&mg, pend_.ev[1], pend_.ev[2]));

@@ -100,7 +100,12 @@ private:
     std::vector<std::pair<cudaEvent_t, int>> marks_;
     std::vector<cudaEvent_t> event_pool_;
     size_t event_next_ = 0;
+    HostWords prepare_publish(int mask);
+    void await_publish();
+    void publish();
     void check_status();
+    void raise_status();
+    void ratio();
     void grad_at(const double* x, bool write_gel, int mask, int slot);
     void grad_at_x(bool write_gel, int mask);
     void gather(int mode, int mask, bool xerr, double* plain = nullptr);
@@ -150,7 +155,7 @@ private:
     cudaEvent_t evs_[2][4] = {};
     struct PendingTiming { bool on = false; int k = 0; cudaEvent_t* ev = nullptr; };
     PendingTiming pend_;
-    void settle_timing(bool wait);
+    void settle_timing();
     std::vector<void*> allocs_;
     int4* d_idx_ = nullptr;
     double *d_Di_ = nullptr, *d_vol_ = nullptr, *d_w2_ = nullptr, *d_w2c_ = nullptr;
@@ -167,8 +172,11 @@ private:
     unsigned char* d_net_img_ = nullptr;   // prox network image + FP32 blob staging
     unsigned* d_counters_ = nullptr;       // one grid-reduction counter per mesh
     double* d_scal_ = nullptr;             // kScalStride scalars per mesh
-    double* h_scal_ = nullptr;
-    int* h_status_ = nullptr;    // pinned: the device status word, read with the scalars
+    unsigned long long* h_words_ = nullptr;   // pinned: per mesh its published scalars and the status word
+    std::vector<char> publishing_;            // meshes whose words are awaited
+    bool publish_pending_ = false;
+    int status_ = 0;                          // the device status word of the last hand-over
+    std::vector<double> h_scal_;              // the scalar blocks as of the last hand-over
     double* d_slots_ = nullptr;  // the cooperative two-loop recursion's tile sums, first and second loop
     size_t slot_set() const;
     bool slots_stale_ = true;    // they are to be refilled before the next launch
