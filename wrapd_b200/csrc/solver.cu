@@ -68,6 +68,15 @@ static_assert(kHostLow == S_ALPHA && kHostHigh == S_LSN && kHostSlots == kHostLo
 // Every mesh's scalars to the host, where no gather has taken them along.
 __global__ void __launch_bounds__(32) k_publish(HostWords P) { publish_mesh(P, blockIdx.x); }
 
+// A control block that fits travels as a launch's argument.
+struct CtlWords {
+    static constexpr int kMax = 32;
+    uint4 w[kMax];
+};
+__global__ void __launch_bounds__(CtlWords::kMax) k_put_ctl(const CtlWords c, int n, uint4* __restrict__ to) {
+    if ((int)threadIdx.x < n) to[threadIdx.x] = c.w[threadIdx.x];
+}
+
 __global__ void k_fill(double* __restrict__ p, int64_t n, double v) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = v;
@@ -517,7 +526,7 @@ void SolverGPU::initialize() {
         const size_t mb = (size_t)MK_COUNT * nm * sizeof(int), cb = (size_t)nm * sizeof(MeshCtl),
                      rb = (size_t)nm * kHistSlots * sizeof(double);
         const size_t mo = 0, co = (mb + 15) / 16 * 16, ro = (co + cb + 15) / 16 * 16;
-        ctl_bytes_ = ro + rb;
+        ctl_bytes_ = (ro + rb + 15) / 16 * 16;
         d_ctl_block_ = dalloc(ctl_bytes_);
         WRAPD_CUDA(cudaMallocHost(&h_ctl_block_, ctl_bytes_));
         std::memset(h_ctl_block_, 0, ctl_bytes_);
@@ -615,12 +624,24 @@ void SolverGPU::ctl_writable() {
     ctl_pending_ = false;
 }
 
-// Uploads the masks, MeshCtl and rho of every mesh.
+// Uploads the masks, MeshCtl and rho of every mesh.  A single mesh's fit in the
+// arguments of a launch, which starts the stream's next work some 4 us sooner than a
+// copy does (8x8x32, 90 uploads a solve, and the phase times read while the device
+// works: 8.57 -> 8.36 ms); a batch's are copied.
 void SolverGPU::push_ctl() {
     ctl_writable();
     for (int m = 0; m < nm; ++m) {
         h_ctl_[m] = runs_[m].ctl;
         std::memcpy(h_rho_ + (size_t)m * kHistSlots, runs_[m].rho, sizeof(runs_[m].rho));
+    }
+    if (ctl_bytes_ <= sizeof(CtlWords)) {
+        CtlWords c;
+        std::memcpy(&c, h_ctl_block_, ctl_bytes_);
+        k_put_ctl<<<1, CtlWords::kMax, 0, st_>>>(c, static_cast<int>(ctl_bytes_ / sizeof(uint4)),
+                                                 static_cast<uint4*>(d_ctl_block_));
+        WRAPD_LAUNCH_CHECK();
+        kernel_launches++;
+        return;
     }
     WRAPD_CUDA(cudaMemcpyAsync(d_ctl_block_, h_ctl_block_, ctl_bytes_, cudaMemcpyHostToDevice, st_));
     ctl_pending_ = true;
@@ -1352,8 +1373,8 @@ int SolverGPU::iterate(int n, bool* conv) {
             grad_at_x(true, MK_ADMM);
             gather(GATHER_START, MK_ADMM, true);
             mark(1);
+            settle_timing();   // the previous iteration's events; this iteration's work is on its way
             sync_read();
-            settle_timing();   // the previous iteration's events are behind this synchronisation
             for (int m = 0; m < nm; ++m) {
                 MeshRun& R = runs_[m];
                 R.in_loop = false;
@@ -1382,6 +1403,7 @@ int SolverGPU::iterate(int n, bool* conv) {
             // ---- UnawareGS::global_step (src/GlobalStepBehavior.hpp:162-180): x = A^-1 b ----
             global_step_unaware();
             x_error_launch(MK_ALL);
+            settle_timing();
             sync_read();
             prox_it[0] = hs(0, S_LOCAL + 4);
             if (hs(0, S_LOCAL + 3) > 0.0) throw CudaError(WRAPD_E_PROX_NEG, "negative singular value in a prox solution");
@@ -1450,9 +1472,8 @@ int SolverGPU::iterate(int n, bool* conv) {
         }
         runtime_ms[5] += its_sum;
         if (nm > 1) union_logs(k + 1);
-        // phase times: read once a later synchronisation has passed the events
+        // phase times: read in the next iteration, while the device works
         pend_ = PendingTiming{true, k, ev_};
-        if (profiling || any_rw || !cfg.rot_aware) settle_timing();
         iter = k + 1;
         done++;
         converged_ = true;
