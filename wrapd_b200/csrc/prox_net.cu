@@ -1,9 +1,10 @@
 // Training and batched inference of the prox-stretch network (prox_net.cuh).
 //
 // Training step over a batch: k_train_tile runs forward and backward for 128
-// samples per CTA (4 warps x 32) on the tensor cores and writes that CTA's
+// samples per CTA (8 warps x 16) on the tensor cores and writes that CTA's
 // gradient to a partial buffer; k_reduce_adam adds the partials in CTA order
-// (deterministic) and applies Adam to the FP32 blob.  Loss: mean squared error
+// (deterministic) and applies Adam to the FP32 blob and to the BF16 image of it
+// that the next step's CTAs copy.  Loss: mean squared error
 // of the normalised outputs, t = (sigma* - sigma_in) / oscale.
 //
 // Backward, per warp (rows = its samples; BF16 operands, FP32 accumulation):
@@ -28,6 +29,9 @@ namespace net {
 namespace {
 
 constexpr int TILE = 128;          // samples per CTA
+constexpr int TRAIN_THREADS = 256;
+constexpr int TRAIN_WARPS = TRAIN_THREADS / 32;
+constexpr int MT = TILE / (16 * TRAIN_WARPS);   // 16-row blocks of a warp
 constexpr int LDT = TILE + 8;      // transposed rows: [feature][sample]
 constexpr int LDZ = HID + 4;       // FP32 activations [sample][LDZ]
 
@@ -35,7 +39,8 @@ constexpr int LDZ = HID + 4;       // FP32 activations [sample][LDZ]
 constexpr int T_IMG = 0;
 constexpr int T_W2T = T_IMG + IMAGE_BYTES;          // [64][LD2] BF16, W2T[in][out]
 constexpr int T_W3T = T_W2T + HID * LD2 * 2;        // [64][LD1] BF16, W3T[in][out], out 3..23 zero
-constexpr int T_XS = T_W3T + HID * LD1 * 2;         // [128][LD1] BF16 normalised inputs
+constexpr int T_BYTES_IMAGE = T_W3T + HID * LD1 * 2;   // the image and the transposes: kept in device memory
+constexpr int T_XS = T_BYTES_IMAGE;                 // [128][LD1] BF16 normalised inputs
 constexpr int T_XT = T_XS + TILE * LD1 * 2;         // [16][LDT] BF16
 constexpr int T_TN = T_XT + 16 * LDT * 2;           // [128][4] FP32 normalised targets
 constexpr int T_Z1 = T_TN + TILE * 4 * 4;           // [128][LDZ] FP32: Z1, then dZ1
@@ -46,30 +51,83 @@ constexpr int T_DYT = T_H2T + HID * LDT * 2;        // [16][LDT] BF16, rows 3..1
 constexpr int T_DYF = T_DYT + 16 * LDT * 2;         // [128][4] FP32 dY
 constexpr int T_DZ1T = T_DYF + TILE * 4 * 4;        // [64][LDT] BF16
 constexpr int T_DZ2T = T_DZ1T + HID * LDT * 2;      // [64][LDT] BF16
-constexpr int T_RED = T_DZ2T + HID * LDT * 2;       // double[4]
-constexpr int TRAIN_SMEM = T_RED + 4 * 8;
+constexpr int T_RED = T_DZ2T + HID * LDT * 2;       // double[TRAIN_WARPS]
+constexpr int TRAIN_SMEM = T_RED + TRAIN_WARPS * 8;
+static_assert(T_BYTES_IMAGE % 16 == 0, "copied in 16-byte words");
 static_assert(TRAIN_SMEM <= 227 * 1024, "training tile exceeds shared memory");
 
 __device__ __forceinline__ void st_bf16(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// The training image of a blob: build_image's, then W2 and W3 transposed.
+__global__ void k_train_image(const float* __restrict__ blob, unsigned char* __restrict__ img) {
+    build_image(blob, img + T_IMG, threadIdx.x, blockDim.x);
+    __nv_bfloat16* W2T = reinterpret_cast<__nv_bfloat16*>(img + T_W2T);
+    __nv_bfloat16* W3T = reinterpret_cast<__nv_bfloat16*>(img + T_W3T);
+    for (int i = threadIdx.x; i < HID * LD2; i += blockDim.x) {
+        const int in = i / LD2, o = i % LD2;
+        W2T[i] = __float2bfloat16_rn(o < HID ? blob[B_W2 + o * HID + in] : 0.0f);
+    }
+    for (int i = threadIdx.x; i < HID * LD1; i += blockDim.x) {
+        const int in = i / LD1, o = i % LD1;
+        W3T[i] = __float2bfloat16_rn(o < OUT ? blob[B_W3 + o * HID + in] : 0.0f);
+    }
+}
+
+// Trained value p (from B_W1) to its places in the training image.
+__device__ __forceinline__ void to_train_image(int p, float v, unsigned char* img) {
+    __nv_bfloat16* b16 = reinterpret_cast<__nv_bfloat16*>(img);
+    float* f32 = reinterpret_cast<float*>(img);
+    const int at = B_W1 + p;
+    if (at < B_B1) {
+        st_bf16(b16 + I_W1 / 2 + p / IN * LD1 + p % IN, v);
+    } else if (at < B_W2) {
+        f32[I_B1 / 4 + at - B_B1] = v;
+    } else if (at < B_B2) {
+        const int o = (at - B_W2) / HID, c = (at - B_W2) % HID;
+        st_bf16(b16 + I_W2 / 2 + o * LD2 + c, v);
+        st_bf16(b16 + T_W2T / 2 + c * LD2 + o, v);
+    } else if (at < B_W3) {
+        f32[I_B2 / 4 + at - B_B2] = v;
+    } else if (at < B_B3) {
+        const int o = (at - B_W3) / HID, c = (at - B_W3) % HID;
+        st_bf16(b16 + I_W3 / 2 + o * LD2 + c, v);
+        st_bf16(b16 + T_W3T / 2 + c * LD1 + o, v);
+    } else {
+        f32[I_B3 / 4 + at - B_B3] = v;
+    }
+}
+
 // One CTA: samples [first + 128 * blockIdx.x, ...) of the batch (through perm
 // when given), B = batch size for the loss scale.  part: N_TRAIN floats per CTA.
-__global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ blob, const float* __restrict__ X,
+// A batch of 4096 is 32 CTAs, one step waits for the one before, and nothing of it
+// is bound by a rate: what a step takes is one CTA's chain.
+// Its weights come as the finished shared-memory image, 26 KB copied in one go with all
+// its loads in flight, where every CTA used to convert and transpose the blob anew, and
+// eight warps of 16 rows share what four of 32 did.  A step of both kernels at batch
+// 4096: 36.6 -> 21.9 us (this one 13.6).
+__global__ void __launch_bounds__(TRAIN_THREADS) k_train_tile(const unsigned char* __restrict__ image, const float* __restrict__ X,
                                                     const float* __restrict__ T, const int64_t* __restrict__ perm,
                                                     int64_t first, int64_t last, float inv_b, float* __restrict__ part,
                                                     double* __restrict__ loss_part) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    build_image(blob, sm + T_IMG, tid, blockDim.x);
+    // the samples' reads, two in a chain, are on their way while the image is copied
+    const int64_t pos = first + (int64_t)blockIdx.x * TILE + tid;
+    const bool valid = tid < TILE && pos < last;
+    float f[IN] = {0.f, 0.f, 0.f, 0.f, 0.f}, tg[3] = {0.f, 0.f, 0.f};
+    if (valid) {
+        const int64_t s = perm ? perm[pos] : pos;
+#pragma unroll
+        for (int c = 0; c < IN; ++c) f[c] = X[IN * s + c];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) tg[c] = T[3 * s + c];
+    }
     __nv_bfloat16* W2T = reinterpret_cast<__nv_bfloat16*>(sm + T_W2T);
     __nv_bfloat16* W3T = reinterpret_cast<__nv_bfloat16*>(sm + T_W3T);
-    for (int i = tid; i < HID * LD2; i += blockDim.x) {
-        const int in = i / LD2, o = i % LD2;
-        W2T[i] = __float2bfloat16_rn(o < HID ? blob[B_W2 + o * HID + in] : 0.0f);
-    }
-    for (int i = tid; i < HID * LD1; i += blockDim.x) {
-        const int in = i / LD1, o = i % LD1;
-        W3T[i] = __float2bfloat16_rn(o < OUT ? blob[B_W3 + o * HID + in] : 0.0f);
+#pragma unroll
+    for (int i = 0; i < (T_BYTES_IMAGE / 16 + TRAIN_THREADS - 1) / TRAIN_THREADS; ++i) {
+        const int k = i * TRAIN_THREADS + tid;
+        if (k < T_BYTES_IMAGE / 16) reinterpret_cast<uint4*>(sm)[k] = reinterpret_cast<const uint4*>(image)[k];
     }
     __nv_bfloat16* DYT = reinterpret_cast<__nv_bfloat16*>(sm + T_DYT);
     for (int i = tid; i < 16 * LDT; i += blockDim.x) DYT[i] = __float2bfloat16_rn(0.0f);
@@ -95,19 +153,11 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
     __nv_bfloat16* DZ2T = reinterpret_cast<__nv_bfloat16*>(sm + T_DZ2T);
     double* RED = reinterpret_cast<double*>(sm + T_RED);
 
-    // ---- stage this lane's sample ----
-    const int row = warp * 32 + lane;
-    const int64_t pos = first + (int64_t)blockIdx.x * TILE + row;
-    const bool valid = pos < last;
-    {
-        float f[IN] = {0.f, 0.f, 0.f, 0.f, 0.f}, tg[3] = {0.f, 0.f, 0.f};
-        if (valid) {
-            const int64_t s = perm ? perm[pos] : pos;
+    // ---- stage the samples, one a thread ----
+    if (tid < TILE) {
+        const int row = tid;
 #pragma unroll
-            for (int c = 0; c < IN; ++c) f[c] = X[IN * s + c];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) tg[c] = (T[3 * s + c] - f[c]) / nrm[B_OSCALE + c];
-        }
+        for (int c = 0; c < 3; ++c) tg[c] = valid ? (tg[c] - f[c]) / nrm[B_OSCALE + c] : 0.0f;
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
             const float v = (valid && c < IN) ? (f[c] - nrm[B_MEAN + c]) * nrm[B_ISTD + c] : 0.0f;
@@ -118,15 +168,15 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
         for (int c = 0; c < 3; ++c) TN[row * 4 + c] = tg[c];
         TN[row * 4 + 3] = 0.0f;
     }
-    __syncwarp();
+    __syncthreads();
 
     // ---- forward ----
-    uint32_t a2[2][4][4];
+    uint32_t a2[MT][4][4];
     {
-        uint32_t a1[2][4];
+        uint32_t a1[MT][4];
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int r = warp * 32 + m * 16 + g;
+        for (int m = 0; m < MT; ++m) {
+            const int r = warp * (16 * MT) + m * 16 + g;
             a1[m][0] = ld32(XS + r * LD1 + 2 * t);
             a1[m][1] = ld32(XS + (r + 8) * LD1 + 2 * t);
             a1[m][2] = ld32(XS + r * LD1 + 2 * t + 8);
@@ -137,8 +187,8 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
             const int n = 8 * j + g, col = 8 * j + 2 * t;
             const uint32_t w0 = ld32(W1s + n * LD1 + 2 * t), w1 = ld32(W1s + n * LD1 + 2 * t + 8);
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const int r = warp * 32 + m * 16 + g;
+            for (int m = 0; m < MT; ++m) {
+                const int r = warp * (16 * MT) + m * 16 + g;
                 float d[4] = {b1[col], b1[col + 1], b1[col], b1[col + 1]};
                 mma_bf16(d, a1[m], w0, w1);
                 Z1[r * LDZ + col] = d[0]; Z1[r * LDZ + col + 1] = d[1];
@@ -151,15 +201,15 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
             }
         }
     }
-    float acc[2][4];
+    float acc[MT][4];
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
+    for (int m = 0; m < MT; ++m) {
         acc[m][0] = acc[m][2] = b3[2 * t];
         acc[m][1] = acc[m][3] = b3[2 * t + 1];
     }
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
-        uint32_t a3[2][4];
+        uint32_t a3[MT][4];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int j = 2 * s + h, n = 8 * j + g, col = 8 * j + 2 * t;
@@ -170,8 +220,8 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
                 w1[kt] = ld32(W2s + n * LD2 + 16 * kt + 2 * t + 8);
             }
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const int r = warp * 32 + m * 16 + g;
+            for (int m = 0; m < MT; ++m) {
+                const int r = warp * (16 * MT) + m * 16 + g;
                 float d[4] = {b2[col], b2[col + 1], b2[col], b2[col + 1]};
 #pragma unroll
                 for (int kt = 0; kt < 4; ++kt) mma_bf16(d, a2[m][kt], w0[kt], w1[kt]);
@@ -186,18 +236,18 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
         }
         const uint32_t v0 = ld32(W3s + g * LD2 + 16 * s + 2 * t), v1 = ld32(W3s + g * LD2 + 16 * s + 2 * t + 8);
 #pragma unroll
-        for (int m = 0; m < 2; ++m) mma_bf16(acc[m], a3[m], v0, v1);
+        for (int m = 0; m < MT; ++m) mma_bf16(acc[m], a3[m], v0, v1);
     }
 
     // ---- loss and dY ----
     double lsum = 0.0;
-    uint32_t ady[2][4];
+    uint32_t ady[MT][4];
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
+    for (int m = 0; m < MT; ++m) {
         float dy[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int r = warp * 32 + m * 16 + g + (q >> 1) * 8, col = 2 * t + (q & 1);
+            const int r = warp * (16 * MT) + m * 16 + g + (q >> 1) * 8, col = 2 * t + (q & 1);
             const int64_t p = first + (int64_t)blockIdx.x * TILE + r;
             float v = 0.0f;
             if (col < OUT && p < last) {
@@ -215,14 +265,14 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
         ady[m][3] = 0u;
     }
     // ---- dH2 = dY W3 -> dZ2 ----
-    uint32_t adz[2][4][4];
+    uint32_t adz[MT][4][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int n = 8 * j + g, col = 8 * j + 2 * t;
         const uint32_t w0 = ld32(W3T + n * LD1 + 2 * t), w1 = ld32(W3T + n * LD1 + 2 * t + 8);
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int r = warp * 32 + m * 16 + g;
+        for (int m = 0; m < MT; ++m) {
+            const int r = warp * (16 * MT) + m * 16 + g;
             float d[4] = {0.f, 0.f, 0.f, 0.f};
             mma_bf16(d, ady[m], w0, w1);
             d[0] *= gelu_grad(Z2[r * LDZ + col]);
@@ -248,8 +298,8 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
             w1[kt] = ld32(W2T + n * LD2 + 16 * kt + 2 * t + 8);
         }
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int r = warp * 32 + m * 16 + g;
+        for (int m = 0; m < MT; ++m) {
+            const int r = warp * (16 * MT) + m * 16 + g;
             float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int kt = 0; kt < 4; ++kt) mma_bf16(d, adz[m][kt], w0[kt], w1[kt]);
@@ -270,7 +320,7 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
     // ---- weight gradients over the CTA's samples (K = 128) ----
     // tiles 0..3: dW1 (m = out/16, n = in 0..7); 4..35: dW2 (4 x 8); 36..43: dW3 (n = in/8)
     float* P = part + (size_t)blockIdx.x * N_TRAIN;
-    for (int tile = warp; tile < 44; tile += 4) {
+    for (int tile = warp; tile < 44; tile += TRAIN_WARPS) {
         const __nv_bfloat16 *A, *B;
         int m0, n0, kind;
         if (tile < 4) { kind = 0; A = DZ1T; B = XT; m0 = 16 * tile; n0 = 0; }
@@ -293,42 +343,65 @@ __global__ void __launch_bounds__(128) k_train_tile(const float* __restrict__ bl
             else if (o < OUT) P[B_W3 - B_W1 + o * HID + in] = d[q];
         }
     }
-    {
-        const int j = tid & 63;
-        const float* Z = tid < 64 ? Z1 : Z2;
+    // the biases, by the upper half of the threads (whose warps have one weight tile less)
+    if (tid >= TRAIN_THREADS / 2) {
+        const int u = tid - TRAIN_THREADS / 2, j = u & 63;
+        const float* Z = u < 64 ? Z1 : Z2;
         float s = 0.0f;
+#pragma unroll 16
         for (int r = 0; r < TILE; ++r) s += Z[r * LDZ + j];
-        P[(tid < 64 ? B_B1 : B_B2) - B_W1 + j] = s;
-        if (tid < OUT) {
-            float s3 = 0.0f;
-            for (int r = 0; r < TILE; ++r) s3 += DYF[r * 4 + tid];
-            P[B_B3 - B_W1 + tid] = s3;
-        }
-        if (tid == 0) loss_part[blockIdx.x] = ((RED[0] + RED[1]) + RED[2]) + RED[3];
+        P[(u < 64 ? B_B1 : B_B2) - B_W1 + j] = s;
+    } else if (tid < OUT) {
+        float s3 = 0.0f;
+#pragma unroll 16
+        for (int r = 0; r < TILE; ++r) s3 += DYF[r * 4 + tid];
+        P[B_B3 - B_W1 + tid] = s3;
+    }
+    if (tid == 0) {
+        double s = RED[0];
+        for (int w = 1; w < TRAIN_WARPS; ++w) s += RED[w];
+        loss_part[blockIdx.x] = s;
     }
 }
 
-// Adds the CTA partials in order; mode 0: write the gradient, mode 1: Adam.
-__global__ void k_reduce_adam(int nparts, const float* __restrict__ part, const double* __restrict__ loss_part,
-                              float* __restrict__ blob, float* __restrict__ m1, float* __restrict__ m2,
+// Adds the CTA partials in order; mode 0: write the gradient, mode 1: Adam, on the
+// blob and its training image.  Eight partials' reads are on their way at a time, over
+// small CTAs on half of the SMs: 4.3 us for 32 partials.  The two moments' products are
+// rounded as written, explicitly: a weight's last bit decides BF16 roundings later on.
+constexpr int ADAM_THREADS = 64;
+__global__ void __launch_bounds__(ADAM_THREADS) k_reduce_adam(int nparts, const float* __restrict__ part, const double* __restrict__ loss_part,
+                              float* __restrict__ blob, unsigned char* __restrict__ image, float* __restrict__ m1, float* __restrict__ m2,
                               float* __restrict__ grad_out, double* __restrict__ loss_out, int mode, float lr_t,
                               float beta1, float beta2, float eps) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < N_TRAIN) {
+        float a = 0.0f, b = 0.0f, w = 0.0f;
+        if (mode != 0) { a = m1[p]; b = m2[p]; w = blob[B_W1 + p]; }
         float gsum = 0.0f;
-        for (int c = 0; c < nparts; ++c) gsum += part[(size_t)c * N_TRAIN + p];
+        constexpr int U = 8;
+        for (int c = 0; c < nparts; c += U) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = c + u < nparts ? part[(size_t)(c + u) * N_TRAIN + p] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c + u < nparts) gsum += v[u];
+        }
         if (mode == 0) {
             grad_out[p] = gsum;
         } else {
-            const float a = beta1 * m1[p] + (1.0f - beta1) * gsum;
-            const float b = beta2 * m2[p] + (1.0f - beta2) * gsum * gsum;
+            a = fmaf(1.0f - beta1, gsum, beta1 * a);
+            b = fmaf((1.0f - beta2) * gsum, gsum, beta2 * b);
             m1[p] = a;
             m2[p] = b;
-            blob[B_W1 + p] -= lr_t * a / (sqrtf(b) + eps);
+            w -= lr_t * a / (sqrtf(b) + eps);
+            blob[B_W1 + p] = w;
+            to_train_image(p, w, image);
         }
     }
     if (p == 0 && loss_out) {
         double s = 0.0;
+#pragma unroll 8
         for (int c = 0; c < nparts; ++c) s += loss_part[c];
         *loss_out = s;
     }
@@ -425,6 +498,7 @@ using namespace wrapd::net;
 
 struct wrapd_prox_net {
     float* d_blob = nullptr;
+    unsigned char* d_image = nullptr;   // the blob as k_train_tile keeps it in shared memory
     float* d_m1 = nullptr;
     float* d_m2 = nullptr;
     float* d_part = nullptr;
@@ -497,10 +571,10 @@ void launch_step(wrapd_prox_net* h, int64_t first, int64_t last, const int64_t* 
                  double* loss_out) {
     const int parts = static_cast<int>((last - first + TILE - 1) / TILE);
     ensure_parts(h, parts);
-    k_train_tile<<<parts, 128, TRAIN_SMEM, h->st>>>(h->d_blob, h->d_X, h->d_T, perm, first, last,
+    k_train_tile<<<parts, TRAIN_THREADS, TRAIN_SMEM, h->st>>>(h->d_image, h->d_X, h->d_T, perm, first, last,
                                                      1.0f / (3.0f * float(last - first)), h->d_part, h->d_loss);
     WRAPD_LAUNCH_CHECK();
-    k_reduce_adam<<<(N_TRAIN + 255) / 256, 256, 0, h->st>>>(parts, h->d_part, h->d_loss, h->d_blob, h->d_m1,
+    k_reduce_adam<<<(N_TRAIN + ADAM_THREADS - 1) / ADAM_THREADS, ADAM_THREADS, 0, h->st>>>(parts, h->d_part, h->d_loss, h->d_blob, h->d_image, h->d_m1,
                                                             h->d_m2, h->d_grad, loss_out, mode, lr_t, 0.9f, 0.999f,
                                                             1e-8f);
     WRAPD_LAUNCH_CHECK();
@@ -529,11 +603,14 @@ WRAPD_API int wrapd_net_create(const float* blob, int n_blob, wrapd_prox_net** o
             WRAPD_CUDA(cudaFuncSetAttribute(k_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, TRAIN_SMEM));
             WRAPD_CUDA(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
             h->d_blob = static_cast<float*>(h->alloc(N_BLOB * sizeof(float)));
+            h->d_image = static_cast<unsigned char*>(h->alloc(T_BYTES_IMAGE));
             h->d_m1 = static_cast<float*>(h->alloc(N_TRAIN * sizeof(float)));
             h->d_m2 = static_cast<float*>(h->alloc(N_TRAIN * sizeof(float)));
             h->d_grad = static_cast<float*>(h->alloc(N_TRAIN * sizeof(float)));
             h->d_losses = static_cast<double*>(h->alloc(sizeof(double)));
             WRAPD_CUDA(cudaMemcpyAsync(h->d_blob, blob, N_BLOB * sizeof(float), cudaMemcpyHostToDevice, h->st));
+            k_train_image<<<1, 256, 0, h->st>>>(h->d_blob, h->d_image);
+            WRAPD_LAUNCH_CHECK();
             WRAPD_CUDA(cudaMemsetAsync(h->d_m1, 0, N_TRAIN * sizeof(float), h->st));
             WRAPD_CUDA(cudaMemsetAsync(h->d_m2, 0, N_TRAIN * sizeof(float), h->st));
             WRAPD_CUDA(cudaStreamSynchronize(h->st));
