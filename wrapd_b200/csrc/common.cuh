@@ -41,12 +41,13 @@ constexpr int kNumSMs = 148;
 
 inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
 
-// Deterministic block sum (MAX: maximum) of NV values per thread (blockDim.x a
-// multiple of 32, at most 1024): a shuffle tree per warp, then the warps in order.
+// Deterministic block reduction of NV values per thread, sums before M0 and maxima
+// from M0 on (blockDim.x a multiple of 32, at most 1024): a shuffle tree per warp, then
+// the warps in order.
 // Returns the totals in thread 0.  One pair of barriers for all the values: with
 // one pair for each, the five sums of the local step took ten barriers, a chain
 // that a launch of few CTAs has nothing else to hide behind.
-template <int NV, bool MAX = false>
+template <int NV, int M0 = NV>
 __device__ __forceinline__ void block_reduce(double (&v)[NV]) {
     __shared__ double sm[NV][32];
 #pragma unroll
@@ -54,7 +55,7 @@ __device__ __forceinline__ void block_reduce(double (&v)[NV]) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             const double w = __shfl_down_sync(0xffffffffu, v[k], o);
-            v[k] = MAX ? fmax(v[k], w) : v[k] + w;
+            v[k] = k >= M0 ? fmax(v[k], w) : v[k] + w;
         }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __syncthreads();   // the previous call's readers of sm are done
@@ -65,10 +66,10 @@ __device__ __forceinline__ void block_reduce(double (&v)[NV]) {
     if (threadIdx.x == 0) {
         double r[NV];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) r[k] = MAX ? sm[k][0] : 0.0 + sm[k][0];
+        for (int k = 0; k < NV; ++k) r[k] = k >= M0 ? sm[k][0] : 0.0 + sm[k][0];
         for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
 #pragma unroll
-            for (int k = 0; k < NV; ++k) r[k] = MAX ? fmax(r[k], sm[k][w]) : r[k] + sm[k][w];
+            for (int k = 0; k < NV; ++k) r[k] = k >= M0 ? fmax(r[k], sm[k][w]) : r[k] + sm[k][w];
 #pragma unroll
         for (int k = 0; k < NV; ++k) v[k] = r[k];
     }
@@ -148,27 +149,27 @@ __device__ __forceinline__ unsigned arrive(unsigned* counter) {
 // by whichever block finishes last. -------------------------------------------
 // The sum of the partials of blocks [b0, b1): thread i takes blocks b0 + i,
 // b0 + i + blockDim.x, ..., then a block sum.
-template <int NV, bool MAX>
+template <int NV, int M0>
 __device__ __forceinline__ void sum_partials(double (&acc)[NV], const double* partials, int b0, int b1) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = MAX ? -1.0e308 : 0.0;
+    for (int k = 0; k < NV; ++k) acc[k] = k >= M0 ? -1.0e308 : 0.0;
     for (int b = b0 + (int)threadIdx.x; b < b1; b += blockDim.x)
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             const double p = __ldcg(partials + (size_t)b * NV + k);
-            acc[k] = MAX ? fmax(acc[k], p) : acc[k] + p;
+            acc[k] = k >= M0 ? fmax(acc[k], p) : acc[k] + p;
         }
-    block_reduce<NV, MAX>(acc);
+    block_reduce<NV, M0>(acc);
 }
 
 // out[k] = total_k.
-template <int NV, bool MAX = false>
+template <int NV, int M0 = NV>
 __device__ __forceinline__ void grid_reduce(const double (&v)[NV], double* partials, unsigned* counter, double* out) {
     __shared__ bool last;
     double acc[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] = v[k];
-    block_reduce<NV, MAX>(acc);
+    block_reduce<NV, M0>(acc);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) partials[(size_t)blockIdx.x * NV + k] = acc[k];
@@ -177,7 +178,7 @@ __device__ __forceinline__ void grid_reduce(const double (&v)[NV], double* parti
     __syncthreads();
     if (!last) return;
     __threadfence();
-    sum_partials<NV, MAX>(acc, partials, 0, (int)gridDim.x);
+    sum_partials<NV, M0>(acc, partials, 0, (int)gridDim.x);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) out[k] = acc[k];
@@ -220,14 +221,14 @@ __device__ __forceinline__ bool mesh_on(const int* on, int mesh) { return !on ||
 // the last tile of the mesh, with the totals in tot[] of thread 0.  With one
 // mesh and no table this is grid_reduce's arithmetic.  counters: one per
 // mesh, zero between launches (the last tile resets its mesh's).
-template <int NV, bool MAX = false>
+template <int NV, int M0 = NV>
 __device__ __forceinline__ bool seg_reduce(const double (&v)[NV], const Tiles& T, int mesh, double* partials,
                                            unsigned* counters, double (&tot)[NV]) {
     __shared__ bool last;
     double acc[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] = v[k];
-    block_reduce<NV, MAX>(acc);
+    block_reduce<NV, M0>(acc);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int k = 0; k < NV; ++k) partials[(size_t)blockIdx.x * NV + k] = acc[k];
@@ -238,17 +239,17 @@ __device__ __forceinline__ bool seg_reduce(const double (&v)[NV], const Tiles& T
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    sum_partials<NV, MAX>(tot, partials, t0, t1);
+    sum_partials<NV, M0>(tot, partials, t0, t1);
     if (threadIdx.x == 0) counters[mesh] = 0u;
     return true;
 }
 
 // seg_reduce writing the totals to out[mesh * stride + k].
-template <int NV, bool MAX = false>
+template <int NV, int M0 = NV>
 __device__ __forceinline__ void seg_reduce_out(const double (&v)[NV], const Tiles& T, int mesh, double* partials,
                                                unsigned* counters, double* out, int stride) {
     double tot[NV];
-    if (seg_reduce<NV, MAX>(v, T, mesh, partials, counters, tot) && threadIdx.x == 0)
+    if (seg_reduce<NV, M0>(v, T, mesh, partials, counters, tot) && threadIdx.x == 0)
 #pragma unroll
         for (int k = 0; k < NV; ++k) out[(size_t)mesh * stride + k] = tot[k];
 }

@@ -336,25 +336,34 @@ static __global__ void __launch_bounds__(256, 5) k_gather(Tiles T, const int* on
     publish_mesh(pub, tl.mesh);
 }
 
+// max_wsq_ratio (src/Elements.hpp:56-69) of one element: max(w2/w2c, w2c/w2).  Per mesh
+// the gamma rule (System::possibly_update_weights) takes the max over its own elements.
+__device__ __forceinline__ double weight_ratio(double w2, double w2c) {
+    const double a = w2 / w2c, b = 1.0 / a;
+    return fmax(a, b);
+}
+
 // ---- local step ---------------------------------------------------------------
 // TetElements::polar_update, NH branch (src/TetElements.cpp:284-346), fused
 // per element: S_in = (symF + U)^T, SVD, prox from the last stretches, Z and
 // U update, and the candidate weight (src/TetElements.cpp:391-432).  C is the
 // arithmetic of the SVD and the prox (double, or float in mixed mode); loads,
 // stores, the dual update and every sum are FP64.
-// out[0..4] = bef_penalty, aft_penalty, curr_pe, negative-stretch count, prox
-// iterations.
+// out[0..5] = bef_penalty, aft_penalty, curr_pe, negative-stretch count, prox
+// iterations and, with `ratio` (the gamma rule; the candidates are then written), the
+// largest weight_ratio.  (8x8x32, per iteration a launch of 4.5 us less for it: 8.36 ->
+// 8.06 ms per solve; without the rule the sixth value would cost the step 1 to 5 %.)
 // prox_mode 0: the reference's L-BFGS prox; 1: Newton (prox_newton); 2 (NET):
 // Newton from the better (lower prox objective) of the last stretches and the
 // prox network's prediction.  The FP32 instantiation always uses Newton.
 // NET needs dynamic shared memory: the network image plus one scratch per warp.
 template <typename C, bool NET>
 __global__ void __launch_bounds__(512, 1) k_local(ElemView E, Tiles T, const int* on, Material mat0, int prox_iters,
-                                               int cand_mode, int prox_mode, const unsigned char* __restrict__ net_img,
+                                               int cand_mode, int ratio, int prox_mode, const unsigned char* __restrict__ net_img,
                                                double* partials, unsigned* counters, double* out, int stride) {
     const Tile tl = tile_at(T, blockIdx.x);
     if (!mesh_on(on, tl.mesh)) return;
-    double red[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    double red[6] = {};
     extern __shared__ __align__(16) unsigned char local_smem[];
     if constexpr (NET) {
         net::load_image(net_img, local_smem);
@@ -471,17 +480,25 @@ __global__ void __launch_bounds__(512, 1) k_local(ElemView E, Tiles T, const int
         red[1] += 0.5 * w2 * aft;
         store9(E.Z, E.ne, e, Zm);
         store9(E.U, E.ne, e, Um);
+        double cand = 0.0;
         if (cand_mode == CAND_REST) {
-            E.w2c[e] = vol * mat.wr;
+            cand = vol * mat.wr;
         } else if (cand_mode == CAND_HESSIAN) {
             const double lm = NH<double>{mat.mu, mat.lambda}.template hess_lmax<sizeof(C) == sizeof(double)>(xo);
             double c = lm;
             if (lm < mat.wmin) c = mat.wmin;
             if (lm > mat.wmax) c = mat.wmax;
-            E.w2c[e] = vol * c;
+            cand = vol * c;
         }
+        if (cand_mode != CAND_NONE) E.w2c[e] = cand;
+        if (ratio) red[5] = weight_ratio(w2, cand);
     }
-    seg_reduce_out<5>(red, T, tl.mesh, partials, counters, out, stride);
+    if (ratio) {
+        seg_reduce_out<6, 5>(red, T, tl.mesh, partials, counters, out, stride);
+    } else {
+        const double sums[5] = {red[0], red[1], red[2], red[3], red[4]};
+        seg_reduce_out<5>(sums, T, tl.mesh, partials, counters, out, stride);
+    }
 }
 
 // initialize_dual_vars (src/TetElements.cpp:145-166): Z = (V diag(s) V^T)^T of
@@ -566,21 +583,6 @@ static __global__ void __launch_bounds__(128) k_mid_candidates(ElemView E, Tiles
     } else {
         E.w2c[e] = vol * mat.wr;
     }
-}
-
-// max_wsq_ratio (src/Elements.hpp:56-69): out[0] = max_e max(w2/w2c, w2c/w2).
-// Per mesh (System::possibly_update_weights takes the max over its own elements).
-static __global__ void __launch_bounds__(256) k_ratio(ElemView E, Tiles T, const int* on, double* partials,
-                                               unsigned* counters, double* out, int stride) {
-    const Tile tl = tile_at(T, blockIdx.x);
-    if (!mesh_on(on, tl.mesh)) return;
-    const int e = tl.first + threadIdx.x;
-    double red[1] = {0.0};
-    if (e < tl.end) {
-        const double a = E.w2[e] / E.w2c[e], b = 1.0 / a;
-        red[0] = fmax(a, b);
-    }
-    seg_reduce_out<1, true>(red, T, tl.mesh, partials, counters, out, stride);
 }
 
 // update_actual_weights (src/TetElements.cpp:435-442), on the meshes that reweight.
@@ -1127,7 +1129,7 @@ static __global__ void __launch_bounds__(256) k_ls_gmax(int n, const double* __r
     double red[1] = {0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         red[0] = fmax(red[0], fabs(grad[i]));
-    grid_reduce<1, true>(red, partials, counter, out);
+    grid_reduce<1, 0>(red, partials, counter, out);
 }
 
 // Trial point of the line search: xt = x + alpha * p with p = -step; the same
@@ -1205,10 +1207,10 @@ static __global__ void __launch_bounds__(128) k_init_dual_unaware(ElemView E, co
 template <typename C>
 __global__ void __launch_bounds__(128, 4) k_local_unaware(ElemView E, const double* __restrict__ x,
                                                        const double* __restrict__ xfix, Material mat0, int prox_iters,
-                                                       int cand_mode, int prox_mode, double* partials,
+                                                       int cand_mode, int ratio, int prox_mode, double* partials,
                                                        unsigned* counter, double* out) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    double red[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    double red[6] = {};
     if (e < E.ne) {
         const Material mat = elem_material(E, mat0, e);
         double F[9], Um[9], Zn[9];
@@ -1279,15 +1281,18 @@ __global__ void __launch_bounds__(128, 4) k_local_unaware(ElemView E, const doub
                 for (int c = 0; c < 3; ++c)
                     M3(Zn, r, c) = double(M3(Ve, r, 0) * xs[0] * M3(Ue, c, 0) + M3(Ve, r, 1) * xs[1] * M3(Ue, c, 1) +
                                           M3(Ve, r, 2) * xs[2] * M3(Ue, c, 2));
+            double cand = 0.0;
             if (cand_mode == CAND_REST) {
-                E.w2c[e] = vol * mat.wr;
+                cand = vol * mat.wr;
             } else if (cand_mode == CAND_HESSIAN) {
                 const double lm = NH<double>{mat.mu, mat.lambda}.template hess_lmax<sizeof(C) == sizeof(double)>(xo);
                 double cnd = lm;
                 if (lm < mat.wmin) cnd = mat.wmin;
                 if (lm > mat.wmax) cnd = mat.wmax;
-                E.w2c[e] = vol * cnd;
+                cand = vol * cnd;
             }
+            if (cand_mode != CAND_NONE) E.w2c[e] = cand;
+            if (ratio) red[5] = weight_ratio(w2, cand);
         }
 #pragma unroll
         for (int r = 0; r < 3; ++r)
@@ -1296,7 +1301,12 @@ __global__ void __launch_bounds__(128, 4) k_local_unaware(ElemView E, const doub
         store9(E.Z, E.ne, e, Zn);
         store9(E.U, E.ne, e, Um);
     }
-    grid_reduce<5>(red, partials, counter, out);
+    if (ratio) {
+        grid_reduce<6, 5>(red, partials, counter, out);
+    } else {
+        const double sums[5] = {red[0], red[1], red[2], red[3], red[4]};
+        grid_reduce<5>(sums, partials, counter, out);
+    }
 }
 
 // UnawareGS right-hand side per element (TetElements::add_to_b,

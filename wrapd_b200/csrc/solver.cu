@@ -21,8 +21,8 @@ enum : int {
     S_GRAD = 0,      // value, pe, flips
     S_GATHER = 4,    // |grad - gold|^2, <s, y>, |x - x_soln|^2
     S_LOCAL = 8,     // bef, aft, pe, negative stretches, prox iterations
-    S_INIT = 13,     // polar potential energy after initialize_dual_vars
-    S_RATIO = 14,    // max weight ratio
+    S_RATIO = 13,    // max weight ratio: the local step's sixth value
+    S_INIT = 14,     // polar potential energy after initialize_dual_vars
     S_DIR = 16,      // L-BFGS decrement
     S_XERR = 18,     // |x - x_soln|^2
     S_DUMMY = 19,
@@ -63,6 +63,7 @@ int vec_blocks(int64_t n) { return std::max(1, std::min(2 * kNumSMs, ceil_div(n,
 
 // The slots of a mesh that the host reads, [0, kHostLow) and [kHostHigh, S_COUNT)
 // (elements.cuh), are all but S_ALPHA, S_C and S_ONE.
+static_assert(S_RATIO == S_LOCAL + 5, "the local step's sixth value");
 static_assert(kHostLow == S_ALPHA && kHostHigh == S_LSN && kHostSlots == kHostLow + S_COUNT - kHostHigh, "published slots");
 
 // Every mesh's scalars to the host, where no gather has taken them along.
@@ -485,7 +486,7 @@ void SolverGPU::initialize() {
     }
     const size_t nblk = (size_t)std::max({te128_.count, te256_.count, tv32_.count, tvec_.count, finest_local,
                                           blocks_for(8 * (int64_t)nf, 256), vec_blocks(3 * (int64_t)nf)}) + 8;
-    d_partials_ = static_cast<double*>(dalloc(nblk * 5 * sizeof(double)));
+    d_partials_ = static_cast<double*>(dalloc(nblk * 6 * sizeof(double)));
     d_counters_ = static_cast<unsigned*>(dalloc(nm * sizeof(unsigned)));
     // the cooperative two-loop recursion (meshes above the one-cluster size): the
     // register form when every vector tile gets its own resident CTA; otherwise a
@@ -724,29 +725,30 @@ void SolverGPU::local_step(int cand_mode) {
         WRAPD_ELEM_LAUNCH(k_local_arap, te128_, 128, mask(MK_ADMM), d_partials_, d_counters_, ds(S_LOCAL), kScalStride);
         return;
     }
+    const int ratio = gamma_rule() && cand_mode != CAND_NONE;
     const int net_smem = local_net_bytes(te_local_.per);
     if ((any_mask(MK_L32N) || any_mask(MK_L64N)) && !d_net_img_)
         throw CudaError(WRAPD_E_STATE, "prox_mode 2 needs a network (wrapd_set_prox_net)");
     const Tiles T = te_local_.view();
     const int nb = te_local_.count, bt = te_local_.per;
     if (any_mask(MK_L32N)) {
-        k_local<float, true><<<nb, bt, net_smem, st_>>>(view(), T, mask(MK_L32N), mat_, cfg.prox_iters, cand_mode, 2,
+        k_local<float, true><<<nb, bt, net_smem, st_>>>(view(), T, mask(MK_L32N), mat_, cfg.prox_iters, cand_mode, ratio, 2,
                                                          d_net_img_, d_partials_, d_counters_, ds(S_LOCAL), kScalStride);
         kernel_launches++;
     }
     if (any_mask(MK_L32)) {
-        k_local<float, false><<<nb, bt, 0, st_>>>(view(), T, mask(MK_L32), mat_, cfg.prox_iters, cand_mode, 1,
+        k_local<float, false><<<nb, bt, 0, st_>>>(view(), T, mask(MK_L32), mat_, cfg.prox_iters, cand_mode, ratio, 1,
                                                    nullptr, d_partials_, d_counters_, ds(S_LOCAL), kScalStride);
         kernel_launches++;
     }
     if (any_mask(MK_L64N)) {
-        k_local<double, true><<<nb, bt, net_smem, st_>>>(view(), T, mask(MK_L64N), mat_, cfg.prox_iters, cand_mode, 2,
+        k_local<double, true><<<nb, bt, net_smem, st_>>>(view(), T, mask(MK_L64N), mat_, cfg.prox_iters, cand_mode, ratio, 2,
                                                           d_net_img_, d_partials_, d_counters_, ds(S_LOCAL), kScalStride);
         kernel_launches++;
     }
     if (any_mask(MK_L64)) {
         k_local<double, false><<<nb, bt, local_hist_bytes(bt), st_>>>(view(), T, mask(MK_L64), mat_, cfg.prox_iters,
-                                                                  cand_mode,
+                                                                  cand_mode, ratio,
                                                                   (fp32() || cfg.prox_mode == 2) ? 1 : cfg.prox_mode,
                                                                   nullptr, d_partials_, d_counters_, ds(S_LOCAL),
                                                                   kScalStride);
@@ -772,12 +774,13 @@ static void set_local_masks(int nm, int* masks, const std::vector<bool>& act, co
 
 void SolverGPU::local_step_unaware(int cand_mode, bool fp32_compute) {
     const int nb = blocks_for(ne, 128);
+    const int ratio = gamma_rule() && cand_mode != CAND_NONE;
     if (fp32_compute && cfg.model == MODEL_NH)
-        k_local_unaware<float><<<nb, 128, 0, st_>>>(view(), d_x_, d_xfix_, mat_, cfg.prox_iters, cand_mode, 1,
+        k_local_unaware<float><<<nb, 128, 0, st_>>>(view(), d_x_, d_xfix_, mat_, cfg.prox_iters, cand_mode, ratio, 1,
                                                     d_partials_, d_counters_, ds(S_LOCAL));
     else
         k_local_unaware<double><<<nb, 128, kLocalHistBytes, st_>>>(view(), d_x_, d_xfix_, mat_, cfg.prox_iters,
-                                                                   cand_mode, (fp32() || cfg.prox_mode != 0) ? 1 : 0,
+                                                                   cand_mode, ratio, (fp32() || cfg.prox_mode != 0) ? 1 : 0,
                                                                    d_partials_, d_counters_, ds(S_LOCAL));
     WRAPD_LAUNCH_CHECK();
     kernel_launches++;
@@ -1314,15 +1317,6 @@ void SolverGPU::union_logs(int k) {
     }
 }
 
-// The largest change of weight of the gamma rule, per mesh.  The local step has
-// written the candidate weights and the global step touches neither they nor the
-// weights, so this follows the local step at once and the host reads the result
-// with the global step's scalars instead of waiting for it by itself.
-void SolverGPU::ratio() {
-    if (!cfg.reweighting || cfg.rw_every > 0) return;
-    WRAPD_ELEM_LAUNCH(k_ratio, te256_, 256, mask(MK_ADMM), d_partials_, d_counters_, ds(S_RATIO), kScalStride);
-}
-
 int SolverGPU::iterate(int n, bool* conv) {
     if (!solving_) throw CudaError(WRAPD_E_STATE, "iterate before begin_solve");
     int done = 0;
@@ -1361,7 +1355,6 @@ int SolverGPU::iterate(int n, bool* conv) {
             // ---- local step: polar_update (src/TetElements.cpp:256-356) ----
             local_step(cand);
             if (cfg.reweighting) count_++;
-            ratio();
             mark(0);
             WRAPD_CUDA(cudaEventRecord(ev_[1], st_));
             // ---- global step: RotAwareGS::global_step (src/GlobalStepBehavior.hpp:246-258) ----
@@ -1397,7 +1390,6 @@ int SolverGPU::iterate(int n, bool* conv) {
             // ---- local_update: TetElements::update (src/TetElements.cpp:193-254), single mesh ----
             local_step_unaware(cand, fp32() && !runs_[0].fp64_phase);
             if (cfg.reweighting) count_++;
-            ratio();
             mark(0);
             WRAPD_CUDA(cudaEventRecord(ev_[1], st_));
             // ---- UnawareGS::global_step (src/GlobalStepBehavior.hpp:162-180): x = A^-1 b ----

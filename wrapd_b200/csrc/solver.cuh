@@ -105,7 +105,7 @@ private:
     void publish();
     void check_status();
     void raise_status();
-    void ratio();
+    bool gamma_rule() const { return cfg.reweighting && cfg.rw_every <= 0; }
     void grad_at(const double* x, bool write_gel, int mask, int slot);
     void grad_at_x(bool write_gel, int mask);
     void gather(int mode, int mask, bool xerr, double* plain = nullptr);
