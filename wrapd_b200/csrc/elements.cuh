@@ -1112,24 +1112,17 @@ static __global__ void __launch_bounds__(256) k_xerr(Tiles T, const int* on, con
 
 // Inputs of the global line search (Backtracking::search,
 // deps/mcloptlib/include/MCL/Backtracking.hpp:71-98): out[0] = <q, q>,
-// out[1] = <grad, grad> (sums); then, in k_ls_gmax, out[0] = max |grad|.
+// out[1] = <grad, grad> (sums), out[2] = max |grad|.
 static __global__ void __launch_bounds__(256) k_ls_norms(int n, const double* __restrict__ q,
                                                   const double* __restrict__ grad, double* partials,
                                                   unsigned* counter, double* out) {
-    double red[2] = {0.0, 0.0};
+    double red[3] = {0.0, 0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         red[0] += q[i] * q[i];
         red[1] += grad[i] * grad[i];
+        red[2] = fmax(red[2], fabs(grad[i]));
     }
-    grid_reduce<2>(red, partials, counter, out);
-}
-
-static __global__ void __launch_bounds__(256) k_ls_gmax(int n, const double* __restrict__ grad, double* partials,
-                                                 unsigned* counter, double* out) {
-    double red[1] = {0.0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        red[0] = fmax(red[0], fabs(grad[i]));
-    grid_reduce<1, 0>(red, partials, counter, out);
+    grid_reduce<3, 2>(red, partials, counter, out);
 }
 
 // Trial point of the line search: xt = x + alpha * p with p = -step; the same

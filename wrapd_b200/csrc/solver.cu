@@ -63,6 +63,7 @@ int vec_blocks(int64_t n) { return std::max(1, std::min(2 * kNumSMs, ceil_div(n,
 
 // The slots of a mesh that the host reads, [0, kHostLow) and [kHostHigh, S_COUNT)
 // (elements.cuh), are all but S_ALPHA, S_C and S_ONE.
+static_assert(S_LSM == S_LSN + 2, "k_ls_norms' third value");
 static_assert(S_RATIO == S_LOCAL + 5, "the local step's sixth value");
 static_assert(kHostLow == S_ALPHA && kHostHigh == S_LSN && kHostSlots == kHostLow + S_COUNT - kHostHigh, "published slots");
 
@@ -1091,9 +1092,8 @@ double SolverGPU::line_search() {
     double* gcur = d_G_[c.grot % 3];
     double* trial = d_S_[c.stage];
     k_ls_norms<<<vb, 256, 0, st_>>>(n, d_q_, gcur, d_partials_, d_counters_, ds(S_LSN));
-    k_ls_gmax<<<vb, 256, 0, st_>>>(n, gcur, d_partials_, d_counters_, ds(S_LSM));
     WRAPD_LAUNCH_CHECK();
-    kernel_launches += 2;
+    kernel_launches++;
     sync_read();
     const double dir = hs(0, S_DIR);
     if (std::isnan(dir)) throw CudaError(WRAPD_E_NAN, "L-BFGS decrement is NaN");
