@@ -3,9 +3,9 @@
 // Factorization, per level of the assembly tree (leaves first):
 //   assemble     the fronts' entries from A and the children's update matrices;
 //   then per panel of NB = 32 columns (right-looking partial Cholesky):
-//   panel        every CTA factors the NB x NB diagonal block in registers
-//                (one warp) and forms its inverse Li (also stored as a diagonal
-//                block of Y), then applies it to one tile: the panel rows
+//   panel        every CTA factors the NB x NB diagonal block (four warps; a
+//                fifth forms its inverse Li behind the pivots, also stored as a
+//                diagonal block of Y), then applies Li to one tile: the panel rows
 //                below the block, P <- P Li^T, or the inverse row block
 //                Y[p, 0:p0] <- Li Y[p, 0:p0] (FP64 DMMA tiles);
 //   update       blocked right-looking: inside the current OB-column block,
@@ -36,7 +36,7 @@ constexpr int TL = 64;        // output tile of the DMMA kernels
 constexpr int SLD = NB + 4;   // smem row pitch (doubles) for [row][k] operand tiles
 constexpr int GEMM_THREADS = 128;
 constexpr int kFusedPanelCtas = 4 * 148;   // panel steps up to one wave (4 CTAs per SM) run fused
-constexpr int COLS_PER_CTA = 8;    // solve / extend-add column groups (one warp each)
+constexpr int COLS_PER_CTA = 8;    // assembly column groups (one warp each)
 
 // The list item that owns CTA b: the last i < n with prefix[i] <= b.  The lanes of a
 // warp look at 32 places at once, so a list of up to 32 items takes one round
@@ -1029,7 +1029,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, MINB)
     k_bwd_queue(double* __restrict__ x, const double* __restrict__ Zb, double* Xp, double* __restrict__ U,
                 const double* __restrict__ YW, const int* __restrict__ rows, SolveQueue Q, double* P,
                 const int* __restrict__ mesh_on) {
-    constexpr int NT = SOLVE_THREADS, TPT = SCH / NT, WC = ST_C / SOLVE_WARPS, NG = TL / ST_C;
+    constexpr int NT = SOLVE_THREADS, TPT = SCH / NT, WC = ST_C / SOLVE_WARPS;
     __shared__ __align__(16) ItemSlot slots[2];
     extern __shared__ __align__(16) double ssm[];
     double* in = ssm + BRING * SOLVE_WARPS * WC * FR;   // [SCH][3], zero past the chunk
