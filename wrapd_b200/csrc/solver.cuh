@@ -150,6 +150,8 @@ private:
     Material* d_mats_ = nullptr;
     // device
     cudaStream_t st_ = nullptr;
+    cudaStream_t side_ = nullptr;    // two_loop_both's clusters; joined to st_ before anything else runs
+    cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
     // phase events of two consecutive iterations (local, global, reweight): an
     // iteration's times are read once a later host synchronisation has passed them
     cudaEvent_t evs_[2][4] = {};
@@ -183,6 +185,8 @@ private:
     int coop_grid_ = 0;          // its CTAs (0: not used)
     bool coop_reg_ = false;      // its register form (one vector tile per CTA)
     void two_loop_grid(bool second, const struct TwoLoopArgs& args);
+    void two_loop_cluster(bool second, const TwoLoopArgs& args, cudaStream_t st);
+    void two_loop_both(bool second, const TwoLoopArgs& args);
     // ---- the meshes of the batch: each its own ADMM and L-BFGS state ----
     int nm = 0;
     struct MeshRun {
