@@ -754,7 +754,7 @@ struct GridExchange {
     int count, t0, t1;
     int* status;
     bool lead;            // the mesh's first CTA
-    // A tile's sum of the threads' v (block_sum's order), to slot j.  `again`: the
+    // A tile's sum of the threads' v (block_reduce's order), to slot j.  `again`: the
     // second or a later tile of the step.
     __device__ __forceinline__ void put(int j, int tile, double v, bool again = false) {
         __shared__ double sm[kTwoLoopGridThreads / 32];
@@ -965,7 +965,7 @@ static __global__ void __launch_bounds__(kTwoLoopGridThreads, REG ? 3 : 4) k_two
 // stand for one CTA of 1024 threads (thread v of it is thread v % 128 of CTA v / 128)
 // with kTwoLoopPerThread entries of q each in registers.  A step's warp sums go to
 // every CTA's shared memory, and after one cluster barrier every thread adds the
-// 32 of them in order, as block_sum does for 1024 threads.  The history vectors of
+// 32 of them in order, as block_reduce does for 1024 threads.  The history vectors of
 // the next step are loaded before the exchange.  (One CTA of 1024 threads, the form
 // before, reads all vectors through one SM and exchanges behind two barriers.)
 constexpr int kTwoLoopCluster = 8;

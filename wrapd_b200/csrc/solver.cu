@@ -582,9 +582,15 @@ void SolverGPU::initialize() {
     d_uv_ = nullptr;
     if (cfg.rot_aware) {
         size_t room = 0, total = 0;
+        void* p = nullptr;
         WRAPD_CUDA(cudaMemGetInfo(&room, &total));
-        if (room > (size_t)(18 + 24) * ne * sizeof(double))
-            d_uv_ = static_cast<double*>(dalloc((size_t)18 * ne * sizeof(double)));
+        if (room > (size_t)(18 + 24) * ne * sizeof(double) &&
+            cudaMalloc(&p, (size_t)18 * ne * sizeof(double)) == cudaSuccess) {
+            allocs_.push_back(p);
+            d_uv_ = static_cast<double*>(p);
+        } else {
+            cudaGetLastError();   // (another handle took the room meanwhile)
+        }
     }
     lap("first factorization (graph capture + run)");
     initialized_ = true;
