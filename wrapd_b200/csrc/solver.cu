@@ -803,9 +803,6 @@ void SolverGPU::local_step_unaware(int cand_mode, bool fp32_compute) {
 }
 
 void SolverGPU::global_step_unaware() {
-    k_rhs_unaware<<<blocks_for(ne, 128), 128, 0, st_>>>(view(), d_xfix_);
-    WRAPD_LAUNCH_CHECK();
-    kernel_launches++;
     gather(GATHER_PLAIN, MK_ALL, false, d_q_);
     mark(1);
     chol.solve(d_q_, st_);
