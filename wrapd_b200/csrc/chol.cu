@@ -1607,8 +1607,9 @@ void CholGPU::build_queues(cudaStream_t st) {
 }
 
 // The state that a solve starts from and leaves behind: every hand-over entry
-// unset, both queue heads 0.
-void CholGPU::fill_unset(cudaStream_t st) {
+// unset, both queue heads 0.  Every launch of the queues goes through here first.
+void CholGPU::ready_solve(cudaStream_t st) {
+    if (!solve_stale_) return;
     unset_fill(d_U_, u_pool_, st);
     unset_fill(d_Xp_, 3 * (int64_t)n, st);
     unset_fill(d_P_, 3 * TL * solve_parts_, st);
@@ -1692,7 +1693,10 @@ void CholGPU::autotune(const double* d_w2, const double* d_Di, int ne, cudaStrea
                 for (int c = 0; c < (int)L.cand.size(); ++c) {
                     *choice = c;
                     build_queues(st);
-                    const float t = timed(3, [&] { solve_launches(s.x, st, nullptr); });
+                    const float t = timed(3, [&] {   // (the untimed launch finds the buffers unset)
+                        ready_solve(st);
+                        solve_launches(s.x, st, nullptr);
+                    });
                     if (t < best_t) { best_t = t; best_c = c; }
                 }
                 *choice = best_c;
@@ -1768,6 +1772,8 @@ void CholGPU::factor(const double* d_w2, const double* d_Di, int ne, cudaStream_
 }
 
 void CholGPU::solve_launches(double* d_x, cudaStream_t st, const int* mesh_on, int hold) {
+    // on buffers that are not unset the waits would take what they hold for values
+    if (solve_stale_) throw CudaError(WRAPD_E_STATE, "triangular solve on hand-over buffers that are not unset");
     const int hold_col = hold < 0 ? -1 : h_desc_[hold].first;
     if (nqf_ > 0) {
         const SolveQueue Q{d_qf_, nqf_, d_heads_, d_heads_ + 1, d_status, hold_col, solve_gate_};
@@ -1785,13 +1791,13 @@ void CholGPU::solve_launches(double* d_x, cudaStream_t st, const int* mesh_on, i
 
 void CholGPU::solve_holding(double* d_x, int hold, cudaStream_t st) {
     if (hold < 0 || hold >= nfronts) throw CudaError(WRAPD_E_INPUT, "front index out of range");
-    if (solve_stale_) fill_unset(st);
+    ready_solve(st);
     solve_launches(d_x, st, nullptr, hold);
     solve_stale_ = true;
 }
 
 void CholGPU::solve(double* d_x, cudaStream_t st, const int* mesh_on) {
-    if (solve_stale_) fill_unset(st);
+    ready_solve(st);
     if (!use_graphs) { solve_launches(d_x, st, mesh_on); return; }
     if (!solve_graph_ || solve_graph_x_ != d_x || solve_graph_mask_ != mesh_on) {
         if (solve_graph_) { cudaGraphExecDestroy(solve_graph_); solve_graph_ = nullptr; }

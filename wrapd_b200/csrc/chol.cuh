@@ -204,7 +204,7 @@ private:
     void solve_launches(double* d_x, cudaStream_t st, const int* mesh_on, int hold = -1);
     // the work queues of the chosen per-level candidates (after build and autotune)
     void build_queues(cudaStream_t st);
-    void fill_unset(cudaStream_t st);
+    void ready_solve(cudaStream_t st);
     void release(void* p);
     SolveWork* d_qf_ = nullptr;   // forward items, leaves first
     SolveWork* d_qb_ = nullptr;   // backward items, root first
