@@ -2,6 +2,7 @@
 #include "solver.cuh"
 
 #include "elements.cuh"
+#include "hand_over.hpp"
 
 #include <algorithm>
 #include <atomic>
@@ -884,7 +885,7 @@ static void throw_status(int status) {
 // work.  prepare_publish unsets the words of the meshes of a mask for the launch that
 // follows; await_publish waits for them.
 HostWords SolverGPU::prepare_publish(int mk) {
-    // (a hand-over that an error kept from being awaited)
+    // a hand-over that an error kept from being awaited: its launch may still write
     if (publish_pending_) WRAPD_CUDA(cudaStreamSynchronize(st_));
     publish_pending_ = true;
     for (int m = 0; m < nm; ++m) {
@@ -905,47 +906,52 @@ HostWords SolverGPU::prepare_publish(int mk) {
 // gather, 8.6.)
 void SolverGPU::await_publish() {
     const auto t0 = std::chrono::steady_clock::now();
-    const volatile unsigned long long* words = h_words_;
     bool done = false;   // the stream's work has ended: every word is there
+    auto ended = [&] {
+        if (done) return true;
+        const cudaError_t e = cudaStreamQuery(st_);
+        if (e != cudaErrorNotReady) WRAPD_CUDA(e);
+        if (e == cudaSuccess || std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(1)) {
+            WRAPD_CUDA(cudaStreamSynchronize(st_));
+            done = true;
+        }
+        return done;
+    };
     status_ = 0;
     for (int m = 0; m < nm; ++m) {
         if (!publishing_[m]) continue;
-        for (int k = 0; k <= kHostSlots; ++k) {
-            const size_t at = (size_t)m * (kHostSlots + 1) + k;
-            for (int i = 1; !done && words[at] == kUnset; ++i) {
-                if (i % 4096) continue;
-                const cudaError_t e = cudaStreamQuery(st_);
-                if (e != cudaErrorNotReady) WRAPD_CUDA(e);
-                if (e == cudaSuccess || std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(1)) {
-                    WRAPD_CUDA(cudaStreamSynchronize(st_));
-                    done = true;
-                }
-            }
-            const unsigned long long w = words[at];
-            if (k == kHostSlots) {
-                if (w != 0) status_ = static_cast<int>(w);
-            } else {
-                std::memcpy(&hs(m, k < kHostLow ? k : k - kHostLow + kHostHigh), &w, sizeof(w));
-            }
-        }
+        unsigned long long w[kHostSlots + 1];
+        if (!take_words(h_words_ + (size_t)m * (kHostSlots + 1), kHostSlots + 1, kUnset, w, ended))
+            throw CudaError(WRAPD_E_CUDA, "internal error: a launch did not hand over all of its scalars");
+        for (int k = 0; k < kHostSlots; ++k)
+            std::memcpy(&hs(m, k < kHostLow ? k : k - kHostLow + kHostHigh), &w[k], sizeof(w[k]));
+        if (w[kHostSlots] != 0) status_ = static_cast<int>(w[kHostSlots]);
     }
     publish_pending_ = false;
     ctl_pending_ = false;
 }
 
-// Waits for the scalars that the last gather hands over, or hands all over now.
+// Hands every mesh's scalars over now and waits for them.
 void SolverGPU::publish() {
-    if (!publish_pending_) {
-        const HostWords P = prepare_publish(MK_ALL);
-        k_publish<<<nm, 32, 0, st_>>>(P);
-        WRAPD_LAUNCH_CHECK();
-        kernel_launches++;
-    }
+    const HostWords P = prepare_publish(MK_ALL);
+    k_publish<<<nm, 32, 0, st_>>>(P);
+    WRAPD_LAUNCH_CHECK();
+    kernel_launches++;
     await_publish();
 }
 
 void SolverGPU::sync_read() {
     publish();
+    synced();
+}
+
+// The scalars that the gather just launched hands over.
+void SolverGPU::sync_gathered() {
+    await_publish();
+    synced();
+}
+
+void SolverGPU::synced() {
     n_sync++;
     mark(5);
     raise_status();
@@ -1286,7 +1292,7 @@ int SolverGPU::lbfgs_minimize() {
         grad_at_x(true, MK_LBFGS);
         gather(GATHER_LBFGS, MK_LBFGS, true);
         mark(1);
-        sync_read();
+        sync_gathered();
         for (int m = 0; m < nm; ++m) {
             MeshRun& R = runs_[m];
             if (!R.in_loop) continue;
@@ -1403,7 +1409,7 @@ int SolverGPU::iterate(int n, bool* conv) {
             gather(GATHER_START, MK_ADMM, true);
             mark(1);
             settle_timing();   // the previous iteration's events; this iteration's work is on its way
-            sync_read();
+            sync_gathered();
             for (int m = 0; m < nm; ++m) {
                 MeshRun& R = runs_[m];
                 R.in_loop = false;
@@ -1656,7 +1662,7 @@ double SolverGPU::global_grad(const double* xfree, double* grad) {
     if (xfree) set_state("xfree", xfree, 3LL * nf);
     grad_at_x(true, MK_ALL);
     gather(GATHER_START, MK_ALL, false);
-    sync_read();
+    sync_gathered();
     if (grad) {
         std::vector<double> g;
         get_state("grad", g);

@@ -95,6 +95,8 @@ private:
     void* dalloc(size_t bytes);
     template <typename X> X* dupload(const std::vector<X>& v);
     void sync_read();
+    void sync_gathered();
+    void synced();
     void mark(int slot);          // close the running profile slot at this point of the stream
     void profile_flush();         // turn recorded event pairs into milliseconds
     std::vector<std::pair<cudaEvent_t, int>> marks_;
