@@ -1559,7 +1559,13 @@ void SolverGPU::solve(double* out) {
 }
 
 // ---- components ------------------------------------------------------------------
-// Element-level steps over every mesh; the returned sums are over the batch.
+// Element-level steps over every mesh; the returned sums are over the batch.  Before
+// initialize, or after one that failed, the masks, the status word and the element
+// state they use are not there.
+void SolverGPU::need_initialized() const {
+    if (!initialized_) throw CudaError(WRAPD_E_STATE, "component call before initialize");
+}
+
 void SolverGPU::download_elem(const double* d, int comps, std::vector<double>& out) {
     const size_t n = (size_t)comps * ne;
     std::vector<double> soa(n);
@@ -1633,11 +1639,13 @@ void SolverGPU::set_state(const std::string& name, const double* in, int64_t n) 
 }
 
 void SolverGPU::update_defo_cache() {
+    need_initialized();
     grad_at_x(false, MK_ALL);
     sync_read();
 }
 
 double SolverGPU::polar_update(bool update_candidates) {
+    need_initialized();
     std::vector<bool> act(nm, true), f32(nm), net(nm, false);
     for (int m = 0; m < nm; ++m) {
         f32[m] = fp32() && !runs_[m].fp64_phase;
@@ -1659,6 +1667,7 @@ double SolverGPU::polar_update(bool update_candidates) {
 }
 
 double SolverGPU::global_grad(const double* xfree, double* grad) {
+    need_initialized();
     if (xfree) set_state("xfree", xfree, 3LL * nf);
     grad_at_x(true, MK_ALL);
     gather(GATHER_START, MK_ALL, false);
@@ -1674,6 +1683,7 @@ double SolverGPU::global_grad(const double* xfree, double* grad) {
 }
 
 void SolverGPU::potential_energy(double* pe, int* flips) {
+    need_initialized();
     grad_at_x(false, MK_ALL);
     sync_read();
     double p = 0.0;

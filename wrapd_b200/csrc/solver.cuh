@@ -106,6 +106,7 @@ private:
     void await_publish();
     void publish();
     void check_status();
+    void need_initialized() const;
     void raise_status();
     bool gamma_rule() const { return cfg.reweighting && cfg.rw_every <= 0; }
     void grad_at(const double* x, bool write_gel, int mask, int slot);
