@@ -54,7 +54,7 @@ struct MeshCtl {
     int k;         // live history entries (SplitLBFGS m_k)
     int it;        // two-loop length of the current inner iteration, min(M, k)
     int stage;     // history slot that receives the next s and y
-    int small;     // the two-loop runs in one CTA (3 x free vertices <= kTwoLoopMaxN)
+    int small;     // the two-loop runs in one cluster (3 x free vertices <= kTwoLoopMaxN)
     int v0, v1;    // the mesh's range in the n x 3 vectors, in doubles
 };
 // Where a launch hands a mesh's scalars to the host (publish_mesh).

@@ -963,15 +963,14 @@ static __global__ void __launch_bounds__(kTwoLoopGridThreads, REG ? 3 : 4) k_two
 
 // Meshes of at most kTwoLoopMaxN unknowns: a cluster of eight CTAs per mesh, which
 // stand for one CTA of 1024 threads (thread v of it is thread v % 128 of CTA v / 128)
-// with kTwoLoopPerThread entries of q each in registers.  A step's warp sums go to
+// with PT entries of q each in registers.  A step's warp sums go to
 // every CTA's shared memory, and after one cluster barrier every thread adds the
 // 32 of them in order, as block_reduce does for 1024 threads.  The history vectors of
 // the next step are loaded before the exchange.  (One CTA of 1024 threads, the form
 // before, reads all vectors through one SM and exchanges behind two barriers.)
 constexpr int kTwoLoopCluster = 8;
 constexpr int kTwoLoopThreads = 128;       // per CTA
-constexpr int kTwoLoopPerThread = 16;
-constexpr int kTwoLoopMaxN = kTwoLoopCluster * kTwoLoopThreads * kTwoLoopPerThread;
+constexpr int kTwoLoopMaxN = kTwoLoopCluster * kTwoLoopThreads * 16;   // PT 16, 8 or 4: see SolverGPU::initialize
 
 __device__ __forceinline__ double cluster_total(double v, double (*sm)[32], int buf, unsigned rank) {
     const int lane = threadIdx.x & 31, vw = rank * (kTwoLoopThreads / 32) + (threadIdx.x >> 5);
@@ -990,18 +989,19 @@ __device__ __forceinline__ double cluster_total(double v, double (*sm)[32], int 
     return r;
 }
 
-template <bool SECOND>
+// Cluster i serves mesh ids[i] (ids null: mesh i).
+template <bool SECOND, int PT>
 static __global__ void __cluster_dims__(kTwoLoopCluster, 1, 1) __launch_bounds__(kTwoLoopThreads)
-    k_two_loop_cluster(const int* on, TwoLoopArgs A) {
+    k_two_loop_cluster(const int* __restrict__ ids, const int* on, TwoLoopArgs A) {
     __shared__ double sm[2][32];   // by step parity: a step's barrier ends the reads of the step before the last
-    const int m = blockIdx.x / kTwoLoopCluster;
+    const int m = ids ? ids[blockIdx.x / kTwoLoopCluster] : blockIdx.x / kTwoLoopCluster;
     const unsigned rank = blockIdx.x % kTwoLoopCluster;
     const MeshCtl c = A.ctl[m];
-    if (!mesh_on(on, m) || !c.small) return;   // the whole cluster
+    if (!mesh_on(on, m)) return;   // the whole cluster
     const VecPools& P = A.P;
     const double* rho = A.rho + (size_t)m * kHistSlots;
     double* scal = A.scal + (size_t)m * A.stride;
-    constexpr int STEP = kTwoLoopCluster * kTwoLoopThreads, PT = kTwoLoopPerThread;
+    constexpr int STEP = kTwoLoopCluster * kTwoLoopThreads;
     const int i0 = c.v0 + (int)(rank * kTwoLoopThreads + threadIdx.x), end = c.v1;
     const bool lead = rank == 0 && threadIdx.x == 0;
     double qv[PT], av[PT], bv[PT];

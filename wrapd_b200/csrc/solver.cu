@@ -43,7 +43,7 @@ enum : int {
     MK_RW,           // reweights now
     MK_L32, MK_L32N, MK_L64, MK_L64N,   // local step: FP32 / FP64 arithmetic, without / with the prox network
     MK_ZERO,         // grad_old to be zeroed (history empty)
-    MK_SMALL,        // MK_LBFGS meshes whose two-loop runs in one CTA
+    MK_SMALL,        // MK_LBFGS meshes whose two-loop runs in one cluster
     MK_LARGE,        // the other MK_LBFGS meshes
     MK_COUNT
 };
@@ -545,6 +545,7 @@ void SolverGPU::initialize() {
         h_ctl_ = reinterpret_cast<MeshCtl*>(h + co);
         d_rho_ = reinterpret_cast<double*>(d + ro);
         h_rho_ = reinterpret_cast<double*>(h + ro);
+        for (auto& list : small_) list.clear();
         for (int m = 0; m < nm; ++m) {
             MeshCtl& c = runs_[m].ctl;
             c.v0 = 3 * runs_[m].f0;
@@ -557,7 +558,29 @@ void SolverGPU::initialize() {
             }
             set_mask(MK_ALL, m, true);
             set_mask(MK_ADMM, m, true);
+            const int n = c.v1 - c.v0;
+            if (c.small) small_[n <= kTwoLoopMaxN / 4 ? 2 : n <= kTwoLoopMaxN / 2 ? 1 : 0].push_back(m);
         }
+        // The clusters of 16 entries a thread are some 55 on the device at once, which
+        // their registers limit.  That many small meshes run side by side, in one launch;
+        // more would run in waves, so each takes the clusters of 16, 8 or 4 entries that
+        // it needs.  Us per inner iteration, first + second loop: one CTA a mesh (the form
+        // before the clusters, whose x step is a launch more), 16 entries for all, now:
+        //     40 meshes of    108 unknowns   10 +  11    11 +  12    11 +  12
+        //   1500 meshes of    108            90 +  84   232 + 265    86 + 103
+        //    600 meshes of  2,793            70 +  81   138 + 175    55 +  71
+        //    400 meshes of  7,533            57 +  67    85 + 124    58 +  88
+        //    300 meshes of 13,689           101 + 113    91 + 149    91 + 146
+        int per_sm = 0, dev = 0, sms = 0;
+        WRAPD_CUDA(cudaGetDevice(&dev));
+        WRAPD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        WRAPD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_two_loop_cluster<true, 16>, kTwoLoopThreads, 0));
+        if ((int)(small_[0].size() + small_[1].size() + small_[2].size()) <= per_sm * sms / kTwoLoopCluster)
+            for (int c : {1, 2}) {
+                small_[0].insert(small_[0].end(), small_[c].begin(), small_[c].end());
+                small_[c].clear();
+            }
+        for (int c = 0; c < 3; ++c) d_small_[c] = nm > 1 && !small_[c].empty() ? dupload(small_[c]) : nullptr;
         push_ctl();
     }
     lap("element state upload");
@@ -1170,12 +1193,19 @@ void SolverGPU::two_loop_grid(bool second, const TwoLoopArgs& args) {
 
 // One loop of the recursion of the meshes of MK_SMALL, a cluster each, on stream st.
 void SolverGPU::two_loop_cluster(bool second, const TwoLoopArgs& args, cudaStream_t st) {
-    if (second)
-        k_two_loop_cluster<true><<<nm * kTwoLoopCluster, kTwoLoopThreads, 0, st>>>(mask(MK_SMALL), args);
-    else
-        k_two_loop_cluster<false><<<nm * kTwoLoopCluster, kTwoLoopThreads, 0, st>>>(mask(MK_SMALL), args);
-    WRAPD_LAUNCH_CHECK();
-    kernel_launches++;
+    using Kernel = void (*)(const int*, const int*, TwoLoopArgs);
+    static const Kernel kernels[2][3] = {
+        {k_two_loop_cluster<false, 16>, k_two_loop_cluster<false, 8>, k_two_loop_cluster<false, 4>},
+        {k_two_loop_cluster<true, 16>, k_two_loop_cluster<true, 8>, k_two_loop_cluster<true, 4>}};
+    const int* on = h_masks_ + (size_t)MK_SMALL * nm;
+    for (int c = 0; c < 3; ++c) {
+        const std::vector<int>& list = small_[c];
+        if (std::none_of(list.begin(), list.end(), [&](int m) { return on[m] != 0; })) continue;
+        kernels[second][c]<<<(int)list.size() * kTwoLoopCluster, kTwoLoopThreads, 0, st>>>(d_small_[c], mask(MK_SMALL),
+                                                                                        args);
+        WRAPD_LAUNCH_CHECK();
+        kernel_launches++;
+    }
 }
 
 // One loop of a batch that has meshes of both kinds: the two launches touch

@@ -188,6 +188,8 @@ private:
     int coop_grid_ = 0;          // its CTAs (0: not used)
     bool coop_reg_ = false;      // its register form (one vector tile per CTA)
     void two_loop_grid(bool second, const struct TwoLoopArgs& args);
+    std::vector<int> small_[3];          // the meshes that take clusters of 16, 8 and 4 entries a thread
+    int* d_small_[3] = {};               // the same on the device (null: a single mesh)
     void two_loop_cluster(bool second, const TwoLoopArgs& args, cudaStream_t st);
     void two_loop_both(bool second, const TwoLoopArgs& args);
     // ---- the meshes of the batch: each its own ADMM and L-BFGS state ----
