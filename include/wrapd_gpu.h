@@ -243,6 +243,16 @@ WRAPD_API int wrapd_solve_A(wrapd_handle* h, const double* b, double* x);
  * usable; WRAPD_E_INPUT for a front outside [0, fronts) (wrapd_get_info). */
 WRAPD_API int wrapd_solve_A_holding(wrapd_handle* h, const double* b, double* x, int front);
 
+/* The bounded waits of the two-loop recursion (no reference counterpart):
+ * wrapd_iterate of one iteration in which tile `tile` of its vector tiles (2,048
+ * entries of the free positions each) does not hand its partial sums on, so that
+ * the waits for them run out after about a second.  Returns WRAPD_E_TIMEOUT when
+ * they did; the positions then hold nothing of use until the next
+ * wrapd_begin_solve, and the handle stays usable.  WRAPD_E_INPUT for a tile out
+ * of range; WRAPD_E_UNSUPPORTED where the system's recursion does not wait so;
+ * WRAPD_OK when the tile's mesh has too few unknowns for that form. */
+WRAPD_API int wrapd_iterate_holding(wrapd_handle* h, int tile);
+
 /* ---- per-element math over a batch, on the current device (handle-free) --
  * The same device functions the ADMM kernels inline.  fp32 = 1 runs them in
  * single precision (the element math of mixed mode). */

@@ -371,4 +371,8 @@ int wrapd_solve_A_holding(wrapd_handle* h, const double* b, double* x, int front
     return guarded(h, [&](wrapd::SolverGPU& s) { s.solve_A(b, x, front); });
 }
 
+int wrapd_iterate_holding(wrapd_handle* h, int tile) {
+    return guarded(h, [&](wrapd::SolverGPU& s) { s.iterate_holding(tile); });
+}
+
 }  // extern "C"

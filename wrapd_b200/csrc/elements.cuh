@@ -754,6 +754,7 @@ struct GridExchange {
     int count, t0, t1;
     int* status;
     bool lead;            // the mesh's first CTA
+    int hold;             // a tile whose sums are not handed on (-1: none): the test of the bounded waits
     // A tile's sum of the threads' v (block_reduce's order), to slot j.  `again`: the
     // second or a later tile of the step.
     __device__ __forceinline__ void put(int j, int tile, double v, bool again = false) {
@@ -765,7 +766,7 @@ struct GridExchange {
         if (threadIdx.x == 0) {
             double r = 0.0;
             for (int w = 0; w < kTwoLoopGridThreads / 32; ++w) r += sm[w];
-            st_relaxed(slots + (size_t)j * count + tile, r);
+            if (tile != hold) st_relaxed(slots + (size_t)j * count + tile, r);
         }
     }
     // The total of slot j over the mesh's tiles, in every thread; false when a wait gave up.
@@ -811,7 +812,8 @@ struct GridExchange {
 
 template <bool SECOND, bool REG>
 static __global__ void __launch_bounds__(kTwoLoopGridThreads, REG ? 3 : 4) k_two_loop_grid(Tiles T, const int* on, TwoLoopArgs A,
-                                                       double* slots, double* other, int nslots, int* status) {
+                                                       double* slots, double* other, int nslots, int* status,
+                                                       int hold) {
     const int count = T.count, G = gridDim.x;
     for (int s = threadIdx.x; s < nslots * ((count + G - 1) / G); s += kTwoLoopGridThreads) {
         const int t = blockIdx.x + (s / nslots) * G;
@@ -826,7 +828,7 @@ static __global__ void __launch_bounds__(kTwoLoopGridThreads, REG ? 3 : 4) k_two
     const int t0 = T.t ? T.tile0[tl.mesh] : 0;
     const bool first_cta = (int)blockIdx.x == t0;
     const size_t totals = (size_t)kHistSlots * count + (size_t)tl.mesh * kTotalSlots;
-    GridExchange X{slots, slots + totals, count, t0, T.t ? T.tile0[tl.mesh + 1] : count, status, first_cta};
+    GridExchange X{slots, slots + totals, count, t0, T.t ? T.tile0[tl.mesh + 1] : count, status, first_cta, hold};
     if (first_cta)
         for (int s = threadIdx.x; s < nslots * kTotalCopies; s += kTwoLoopGridThreads)
             st_relaxed(other + totals + s * kTotalPitch, unset_value());

@@ -894,11 +894,12 @@ void SolverGPU::profile_flush() {
     event_next_ = 0;
 }
 
-// The device status word carries a factorization's non-positive pivot and a
-// solve's dependency wait that gave up; it is read with every scalar block.
+// The device status word carries a factorization's non-positive pivot and a wait
+// of the triangular solve or of the two-loop recursion that gave up; it is read with
+// every scalar block.
 static void throw_status(int status) {
     if (status == WRAPD_E_TIMEOUT)
-        throw CudaError(status, "a dependency wait of the triangular solve gave up");
+        throw CudaError(status, "a bounded wait of the triangular solve or of the two-loop recursion gave up");
     throw CudaError(status, "factorization of D^T W D hit a non-positive pivot");
 }
 
@@ -1182,7 +1183,8 @@ void SolverGPU::two_loop_grid(bool second, const TwoLoopArgs& args) {
     double* other = d_slots_ + (second ? 0 : set);
     int nslots = cfg.lbfgs_m + 1;
     int* status = chol.d_status;
-    void* p[] = {&T, &on, &a, &mine, &other, &nslots, &status};
+    int hold = hold_tile_;
+    void* p[] = {&T, &on, &a, &mine, &other, &nslots, &status, &hold};
     const void* fn = coop_reg_ ? (second ? reinterpret_cast<const void*>(&k_two_loop_grid<true, true>)
                                          : reinterpret_cast<const void*>(&k_two_loop_grid<false, true>))
                                : (second ? reinterpret_cast<const void*>(&k_two_loop_grid<true, false>)
@@ -1546,6 +1548,21 @@ int SolverGPU::iterate(int n, bool* conv) {
     settle_timing();
     *conv = converged_;
     return done;
+}
+
+// One iteration in which a vector tile's sums are not handed on, so that the waits of
+// the cooperative two-loop recursion run out.
+void SolverGPU::iterate_holding(int tile) {
+    if (!solving_) throw CudaError(WRAPD_E_STATE, "iterate before begin_solve");
+    if (tile < 0 || tile >= tvec_.count) throw CudaError(WRAPD_E_INPUT, "vector tile out of range");
+    if (coop_grid_ == 0) throw CudaError(WRAPD_E_UNSUPPORTED, "this system's two-loop recursion has no such wait");
+    struct Hold {   // on every path
+        int& t;
+        ~Hold() { t = -1; }
+    } hold{hold_tile_};
+    hold_tile_ = tile;
+    bool conv = false;
+    iterate(1, &conv);
 }
 
 // Adds a finished iteration's phase times (CUDA events) to the runtime and its

@@ -65,6 +65,7 @@ public:
     // bounded-wait test: throws WRAPD_E_TIMEOUT)
     void solve_A(const double* b, double* x, int hold = -1);
     int n_fronts() const { return chol.nfronts; }
+    void iterate_holding(int tile);
 
     // The logs of a single mesh; of a batch, the sums over its meshes
     // (energies, flips, inner iterations), any reweight, and the x error of
@@ -185,6 +186,7 @@ private:
     double* d_slots_ = nullptr;  // the cooperative two-loop recursion's tile sums, first and second loop
     size_t slot_set() const;
     bool slots_stale_ = true;    // they are to be refilled before the next launch
+    int hold_tile_ = -1;         // see iterate_holding
     int coop_grid_ = 0;          // its CTAs (0: not used)
     bool coop_reg_ = false;      // its register form (one vector tile per CTA)
     void two_loop_grid(bool second, const struct TwoLoopArgs& args);

@@ -230,6 +230,11 @@ class Solver:
         self._h.check(self._h.lib.wrapd_solve_A_holding(self._h.h, capi.dptr(bb), capi.dptr(x), int(front)))
         return x
 
+    def iterate_holding(self, tile):
+        """wrapd_iterate_holding: an iteration in which one vector tile's sums are
+        not handed on; raises WrapdError (WRAPD_E_TIMEOUT) when the waits ran out."""
+        self._h.check(self._h.lib.wrapd_iterate_holding(self._h.h, int(tile)))
+
     def close(self):
         self._h.close()
 
