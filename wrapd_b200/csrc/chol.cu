@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_trsm(double* __restrict__ F, d
 
 // Panel steps with few CTAs (the upper levels: a few large fronts, where the
 // step is latency-bound) run as one launch: every CTA first factors the
-// front's NB x NB diagonal block itself (warp 0, registers) and keeps its
+// front's NB x NB diagonal block itself (cta_chol_inv) and keeps its
 // inverse Li in shared memory, so no separate diagonal launch precedes it.  Items per front: nP
 // panel-row tiles (P <- P Li^T below the diagonal block), then the inverse
 // row-block tiles Y[p, c0:c0+64] <- Li Y[p, c0:c0+64], c0 < p0; a front with
@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, WRAPD_GEMM_MINB) k_update(double
 }
 
 // W = L_rs Y (r x k) with Y lower triangular: tile (ti, tj) of 64 x 64 sums
-// t over [64 tj, k) in chunks of NB.
+// t over [64 tj, k) in chunks of KC.
 __global__ void __launch_bounds__(GEMM_THREADS) k_wgemm(const double* __restrict__ F, const double* __restrict__ Y,
                                                         double* __restrict__ W, const FrontDesc* __restrict__ desc,
                                                         WorkList wl) {
@@ -774,8 +774,15 @@ constexpr int SCH = 256;              // longest chunk of the streamed dimension
 constexpr int SCH_MIN = 64;
 constexpr int kSolveItems = 2 * 148;   // items wanted per level (see build and build_queues)
 constexpr int kBwdSub = 4;            // narrow backward bands per 64 columns
-constexpr size_t kBwdDeepBytes = (size_t)3 << 29;     // largest [Y; W] of the deep backward ring (see k_bwd_queue)
-constexpr size_t kGateBytes = (size_t)256 << 20;      // largest [Y; W] whose items poll their inputs directly (see k_fwd_queue)
+// Largest [Y; W] of the deep backward ring (see k_bwd_queue).  Us backward, deep and
+// not, over compact bars: 564 MB 161, 178; 705 MB 200, 206; 864 MB 261, 235; 1.2 GB 324, 296;
+// 2.1 GB 549, 472: they cross at 0.8 GB, so the line is higher than these want it.
+constexpr size_t kBwdDeepBytes = (size_t)3 << 29;
+// Largest [Y; W] whose items poll their inputs at once (see k_fwd_queue).  Us forward +
+// backward, at once and gated: compact bars of 126 MB 139, 145; 208 MB 192, 178; 255 MB 244,
+// 184; 363 MB 308, 227; thin bars (4 x 4, 3 x 3) of 218 MB 202, 216; 262 MB 236, 257; batches
+// of 50 to 370 MB within 4 % of each other.
+constexpr size_t kGateBytes = (size_t)256 << 20;
 __device__ __forceinline__ void st_unset3(double* p) {
     st_relaxed(p, unset_value());
     st_relaxed(p + 1, unset_value());
@@ -824,10 +831,13 @@ __device__ __forceinline__ bool add_chunks(double* P, int first, int nchunk, int
     return true;
 }
 
-// The CTA's item list position: thread 0 of warp `W` holds the ticket of the
-// next item (fetched once the current item's waits are over, so that a CTA
-// that waits does not sit on work another could take) and its warp copies that
-// item's record to shared memory while the others finish the current one.
+// The CTA's item list position: thread 0 of its last warp takes the ticket of the
+// next item and its warp copies that item's record to shared memory while the others
+// finish the current one.  Gated items (k_fwd_queue) take it after the gate's wait,
+// so that a CTA that waits does not sit on work another could take; the others before
+// they poll, which on a small system has CTAs to spare.  Either way a CTA's current
+// item comes before the one it holds, so the earliest unfinished item is always
+// some CTA's current one.
 struct ItemSlot {
     SolveWork it;
     int q;
@@ -1252,7 +1262,7 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
         const Front& F = S.fronts[f];
         FrontDesc& d = h_desc_[f];
         d.first = F.first; d.k = F.ncols; d.r = F.nrows(); d.ld = F.ld();
-        d.f_off = F.f_off; d.y_off = F.y_off; d.u_off = F.u_off; d.rel_off = F.rel_off;
+        d.f_off = F.f_off; d.y_off = F.y_off; d.u_off = F.u_off;
         d.rows_off = roff;
         rows.insert(rows.end(), F.rows.begin(), F.rows.end());
         roff += F.nrows();
@@ -1262,7 +1272,6 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
         d.child1 = d.nchild > 1 ? F.children[1] : -1;
         d.ldy = static_cast<int>(yw_ld(d.k, d.r));
         d.mesh = front_mesh.empty() ? 0 : front_mesh[f];
-        d.parent = F.parent;
     }
     if (S.u_pool / 3 > INT32_MAX) throw CudaError(WRAPD_E_INPUT, "solve update vectors exceed 32-bit row indexes");
     h_inv_.assign(ioff, -1);
@@ -1498,8 +1507,9 @@ void CholGPU::build(const Symbolic& S, const std::vector<int64_t>& A_pos, const 
 // The chosen candidate of every level, concatenated: forward leaves first,
 // backward root first, each item with the front's numbers it needs and the
 // entries its first poll looks at: the last of its inputs that each child
-// writes (forward), the nearest ancestor's (backward).  Every index the kernels
-// will use is checked against its buffer here.
+// writes (forward), the nearest ancestor's (backward).  Every index of an item is
+// checked against its buffer here; the entries of inv and rows that the kernels
+// look up are the symbolic analysis'.
 void CholGPU::build_queues(cudaStream_t st) {
     std::vector<SolveWork> qf, qb;
     auto work = [&](const SolveItem& g, int first) {

@@ -27,10 +27,9 @@ namespace wrapd {
 
 struct FrontDesc {
     int first, k, r, ld;
-    int64_t f_off, y_off, u_off, rows_off, rel_off, inv_off;
+    int64_t f_off, y_off, u_off, rows_off, inv_off;
     int nchild, child0, child1, ldy;   // ldy: leading dimension of the front's [Y; W] block
     int mesh;                          // the mesh of a batch the front belongs to (0: one mesh)
-    int parent;                        // -1 at a root
 };
 
 // A trailing-update job of the blocked factorization: C -= A B'^T over a K range

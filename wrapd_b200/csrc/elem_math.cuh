@@ -411,7 +411,7 @@ __device__ __forceinline__ T NH<T>::hess_lmax(const T* x) const {
 // min_x psi(x) + (wov/2)|x - x0|^2 by LBFGS<3, M=8> with cubic-interpolating
 // Armijo backtracking, restating deps/mcloptlib/include/MCL/LBFGS.hpp:52-152,
 // Backtracking.hpp:268-332 and Prox::converged (src/TetElements.hpp:40-42).
-// The history is kept in registers (fully unrolled, predicated loops); the
+// The history is kept in shared memory (ProxHistory); the
 // line search is capped at 4096 trials instead of 100000 (the step shrinks by
 // at least 2x per trial, so it underflows to zero long before).
 template <typename T>

@@ -620,7 +620,7 @@ static __global__ void __launch_bounds__(256) k_lbfgs_first(Tiles T, const int* 
     const Tile tl = tile_at(T, blockIdx.x);
     if (!mesh_on(on, tl.mesh)) return;
     const MeshCtl c = ctl[tl.mesh];
-    if (j >= c.it || (j == -1 && false)) return;
+    if (j >= c.it) return;
     double* sc = scal + (size_t)tl.mesh * stride;
     const bool first = j == c.it - 1;                  // q = g (also j = -1 with it = 0)
     const double* g = g_cur(P, c);
@@ -714,7 +714,10 @@ __device__ __forceinline__ void x_step(const TwoLoopArgs& a, double* s, int i, d
 // of the next step loaded before the exchange.  Otherwise one mesh, CTA b taking tiles
 // b, b + G, ... with q in memory.
 constexpr int kTwoLoopGridThreads = 256;
-constexpr int kDirectTiles = 64;   // (203 tiles: 26 + 38 us polled by all, 15 + 21 through the first CTA)
+// Us per inner iteration, first + second loop, polled by all and through the first
+// CTA: 9 tiles 10.5 + 12.6, 12.4 + 16.4; 41 to 75 tiles the same within 0.5; 106 tiles 16.8 + 23.2,
+// 13.5 + 21.0; 203 tiles 31.9 + 36.0, 16.3 + 23.2.
+constexpr int kDirectTiles = 64;
 constexpr int kTwoLoopPT = kVecTile / kTwoLoopGridThreads;
 static_assert(kVecTile % kTwoLoopGridThreads == 0, "whole entries per thread");
 

@@ -17,7 +17,7 @@ namespace wrapd {
 
 namespace {
 
-// Slots of the device scalar block (k_publish hands them to the host).
+// Slots of the device scalar block (publish_mesh hands them to the host).
 enum : int {
     S_GRAD = 0,      // value, pe, flips
     S_GATHER = 4,    // |grad - gold|^2, <s, y>, |x - x_soln|^2
@@ -26,10 +26,8 @@ enum : int {
     S_INIT = 14,     // polar potential energy after initialize_dual_vars
     S_DIR = 16,      // L-BFGS decrement
     S_XERR = 18,     // |x - x_soln|^2
-    S_DUMMY = 19,
     S_ALPHA = 20,    // alpha_i, up to 32 entries (these two: on the device only)
     S_C = 52,        // alpha_i - beta_i, up to 32 entries
-    S_ONE = 84,      // constant 1 (a device-side coefficient)
     S_LSN = 85,      // line search: <q, q>, <grad, grad>
     S_LSM = 87,      // line search: max |grad|
     S_LSV = 88,      // line search: AL value, pe, flips at the trial point
@@ -63,7 +61,7 @@ int blocks_for(int64_t n, int threads) { return std::max(1, ceil_div(n, threads)
 int vec_blocks(int64_t n) { return std::max(1, std::min(2 * kNumSMs, ceil_div(n, 256))); }
 
 // The slots of a mesh that the host reads, [0, kHostLow) and [kHostHigh, S_COUNT)
-// (elements.cuh), are all but S_ALPHA, S_C and S_ONE.
+// (elements.cuh), are all but S_ALPHA and S_C.
 static_assert(S_LSM == S_LSN + 2, "k_ls_norms' third value");
 static_assert(S_RATIO == S_LOCAL + 5, "the local step's sixth value");
 static_assert(kHostLow == S_ALPHA && kHostHigh == S_LSN && kHostSlots == kHostLow + S_COUNT - kHostHigh, "published slots");
@@ -524,10 +522,6 @@ void SolverGPU::initialize() {
     WRAPD_CUDA(cudaMallocHost(&h_words_, (size_t)nm * (kHostSlots + 1) * sizeof(*h_words_)));
     h_scal_.assign((size_t)nm * kScalStride, 0.0);
     publishing_.assign(nm, 0);
-    {
-        static const double one = 1.0;
-        WRAPD_CUDA(cudaMemcpyAsync(d_scal_ + S_ONE, &one, sizeof(double), cudaMemcpyHostToDevice, st_));
-    }
     // the per-mesh control block: masks, MeshCtl, rho
     {
         const size_t mb = (size_t)MK_COUNT * nm * sizeof(int), cb = (size_t)nm * sizeof(MeshCtl),
@@ -1006,7 +1000,7 @@ void SolverGPU::x_error_launch(int mk) {
     kernel_launches++;
 }
 
-// The local step's tile (elements per CTA, 64, 128 or 256) timed on this
+// The local step's tile (elements per CTA, 64, 128, 256 or 512) timed on this
 // system's first local step: every candidate runs the step the solve will run
 // (its precision and prox), from the same saved state, which is restored
 // afterwards; the fastest is kept.  Called once, from the first begin_solve.
