@@ -213,7 +213,7 @@ private:
     // 512 elements (16 warps, one CTA per SM): the FP64 local step takes 0.577
     // ms on the 786k bar (0.587 at 256, 0.71 at 128, 0.96 at 64, 1.67 at 32)
     // and 2.60 ms on the 3.9M bar (2.79 at 256, 3.65 at 128), all before the shorter
-    // FP64 arithmetic of svd3_fast and the prox: 0.49 and 2.23 ms at 512 with it
+    // FP64 arithmetic of svd3_fast and the prox: 0.50 and 2.25 ms at 512 with it
     int local_per_ = 512;
     bool local_tuned_ = false;
     void autotune_local();
