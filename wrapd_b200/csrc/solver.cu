@@ -1213,7 +1213,12 @@ void SolverGPU::two_loop_both(bool second, const TwoLoopArgs& args) {
     WRAPD_CUDA(cudaEventRecord(ev_fork_, st_));
     two_loop_grid(second, args);
     WRAPD_CUDA(cudaStreamWaitEvent(side_, ev_fork_, 0));
-    two_loop_cluster(second, args, side_);   // (last: nothing of it is under way if the other launch fails)
+    try {
+        two_loop_cluster(second, args, side_);   // (last: nothing of it is under way if the other launch fails)
+    } catch (...) {
+        cudaStreamSynchronize(side_);   // one of its launches may be
+        throw;
+    }
     WRAPD_CUDA(cudaEventRecord(ev_join_, side_));
     WRAPD_CUDA(cudaStreamWaitEvent(st_, ev_join_, 0));
 }
